@@ -495,14 +495,14 @@ int hk_attn_bwd_prep(const void* o, const void* d_o, float* delta, int B, int N,
   int rc = scope.enter(device, &st);
   if (rc != HK_OK) return rc;
   const long long rows = static_cast<long long>(B) * N * H;
-  const int rows_per_block = 8 * (32 / (D / 8));  // 8 warps, D/8 lanes per row
-  const long long blocks = (rows + rows_per_block - 1) / rows_per_block;
-  if (blocks > 0x7fffffffll) return HK_EINVAL;
+  if (rows > 0x7fffffffll) return HK_EINVAL;  // rows are indexed with int
+  const int rows_per_block = hk::row_pass_rows(D / 8);
+  const unsigned blocks = unsigned((rows + rows_per_block - 1) / rows_per_block);
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   const auto* po = static_cast<const __nv_bfloat16*>(o);
   const auto* pd = static_cast<const __nv_bfloat16*>(d_o);
-  if (D == 128) hk::attn_bwd_prep_kernel<128><<<unsigned(blocks), 256, 0, stream>>>(po, pd, delta, B, N, H);
-  else hk::attn_bwd_prep_kernel<64><<<unsigned(blocks), 256, 0, stream>>>(po, pd, delta, B, N, H);
+  auto* fn = D == 128 ? hk::attn_bwd_prep_kernel<128> : hk::attn_bwd_prep_kernel<64>;
+  fn<<<blocks, 256, 0, stream>>>(po, pd, delta, int(rows), N, H, hk::FastDiv(H), hk::FastDiv(N));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   HK_CUDA(cudaGetLastError());
   return HK_OK;
@@ -594,11 +594,14 @@ int hk_attn_dq_shuffle(const void* dq_bhnd, void* dq_bnhd, int B, int N, int H, 
   int rc = scope.enter(device, &st);
   if (rc != HK_OK) return rc;
   const int vec = D / 8;
-  const long long total = static_cast<long long>(B) * N * H * vec;
-  const long long blocks = (total + 255) / 256;
+  const long long rows = static_cast<long long>(B) * N * H, total = rows * vec;
+  const long long blocks = (total + 256 * hk::kRowPassUnroll - 1) / (256 * hk::kRowPassUnroll);
   if (blocks > 0x7fffffffll) return HK_EINVAL;
-  hk::attn_dq_shuffle_kernel<<<unsigned(blocks), 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
-      static_cast<const uint4*>(dq_bhnd), static_cast<uint4*>(dq_bnhd), B, N, H, vec);
+  if ((vec == 8 || vec == 16) && rows > 0x7fffffffll) return HK_EINVAL;  // these index rows with int
+  auto* fn = vec == 16 ? hk::attn_dq_shuffle_kernel<16>
+                       : (vec == 8 ? hk::attn_dq_shuffle_kernel<8> : hk::attn_dq_shuffle_kernel<0>);
+  fn<<<unsigned(blocks), 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+      static_cast<const uint4*>(dq_bhnd), static_cast<uint4*>(dq_bnhd), total, N, H, vec, hk::FastDiv(H), hk::FastDiv(N));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   HK_CUDA(cudaGetLastError());
   return HK_OK;
