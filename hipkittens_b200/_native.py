@@ -30,6 +30,8 @@ EXPORTED_SYMBOLS = (
     "hk_attn_bwd",
     "hk_attn_bwd_varlen",
     "hk_attn_bwd_cross",
+    "hk_attn_bwd_strided",
+    "hk_key_padding_lens",
     "hk_attn_dq_shuffle",
     "hk_rotary",
     "hk_rotary_bnhd",
@@ -96,6 +98,10 @@ def capi() -> ctypes.CDLL:
     lib.hk_attn_bwd_varlen.restype = ci
     lib.hk_attn_bwd_cross.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp, ci, cf, ci, ci, vp]
     lib.hk_attn_bwd_cross.restype = ci
+    lib.hk_attn_bwd_strided.argtypes = [vp] * 10 + [ci] * 6 + [ll3] * 6 + [vp, ci, cf, ci, vp]
+    lib.hk_attn_bwd_strided.restype = ci
+    lib.hk_key_padding_lens.argtypes = [vp, vp, vp, ci, ci, ci, vp]
+    lib.hk_key_padding_lens.restype = ci
     lib.hk_attn_dq_shuffle.argtypes = [vp, vp, ci, ci, ci, ci, ci, vp]
     lib.hk_attn_dq_shuffle.restype = ci
     lib.hk_rotary.argtypes = [vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp]
@@ -314,6 +320,64 @@ def attn_bwd(
                                    s.cuda_stream)
     _check(rc, "hk_attn_bwd")
     return dq, dk, dv
+
+
+def attn_bwd_strided(
+    q: torch.Tensor,
+    k: torch.Tensor,
+    v: torch.Tensor,
+    o: torch.Tensor,
+    d_o: torch.Tensor,
+    lse: torch.Tensor,
+    dq: torch.Tensor,
+    dk: torch.Tensor,
+    dv: torch.Tensor,
+    causal: bool = False,
+    softmax_scale: Optional[float] = None,
+    kv_lens: Optional[torch.Tensor] = None,
+) -> None:
+    """The backward in one call: delta = rowsum(O * dO), then dQ, dK, dV written into the given tensors. q, k, v, dq,
+    dk and dv may be strided views with a contiguous last dimension (slices of a packed projection and of its
+    gradient); o and d_o [B,N,H,D] are contiguous. Asynchronous on torch's current stream."""
+    b, n, h, d = q.shape
+    nk, hkv = k.shape[1], k.shape[2]
+    for name, t, shape in (("q", q, (b, n, h, d)), ("k", k, (b, nk, hkv, d)), ("v", v, (b, nk, hkv, d)),
+                           ("dq", dq, (b, n, h, d)), ("dk", dk, (b, nk, hkv, d)), ("dv", dv, (b, nk, hkv, d)),
+                           ("o", o, (b, n, h, d)), ("d_o", d_o, (b, n, h, d))):
+        if t.dtype != torch.bfloat16 or t.shape != shape or t.device != q.device or not t.is_cuda:
+            raise RuntimeError(f"{name} must be a bf16 tensor of shape {shape} on q's CUDA device")
+        if d > 1 and t.stride(3) != 1:
+            raise RuntimeError(f"{name}: the last dimension must be contiguous")
+    if not o.is_contiguous() or not d_o.is_contiguous():
+        raise RuntimeError("Tensor must be contiguous")
+    if lse.shape != (b, h, 1, n) or lse.dtype != torch.float32 or not lse.is_contiguous() or lse.device != q.device:
+        raise RuntimeError("lse must be a contiguous fp32 tensor [B, H, 1, N] on q's device")
+    if kv_lens is not None and (kv_lens.dtype != torch.int32 or kv_lens.shape != (b,) or kv_lens.device != q.device):
+        raise RuntimeError("kv_lens must be an int32 tensor [B] on q's device")
+    s = torch.cuda.current_stream(q.device)
+    delta = torch.empty_like(lse)
+
+    def arr(t):  # a dimension of size 1 has no stride that matters: give it one the library takes
+        return (ctypes.c_longlong * 3)(*(st if n_i > 1 else d for st, n_i in zip(t.stride()[:3], t.shape[:3])))
+
+    rc = capi().hk_attn_bwd_strided(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(),
+                                    lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                    b, n, nk, h, hkv, d, arr(q), arr(k), arr(v), arr(dq), arr(dk), arr(dv),
+                                    kv_lens.data_ptr() if kv_lens is not None else None, int(bool(causal)),
+                                    float(softmax_scale or 0.0), q.device.index, s.cuda_stream)
+    _check(rc, "hk_attn_bwd_strided")
+
+
+def key_padding_lens(mask: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Key lengths int32 [B] of a CUDA bool mask [B, N] (True = keep), and an int32 scalar tensor that is non-zero if a
+    row does not keep a prefix of at least one key. Asynchronous on torch's current stream."""
+    b, n = mask.shape
+    mask = mask.contiguous()
+    buf = torch.zeros(b + 1, dtype=torch.int32, device=mask.device)
+    s = torch.cuda.current_stream(mask.device)
+    _check(capi().hk_key_padding_lens(mask.data_ptr(), buf.data_ptr(), buf.data_ptr() + 4 * b, b, n, mask.device.index,
+                                      s.cuda_stream), "hk_key_padding_lens")
+    return buf[:b], buf[b]
 
 
 def dq_shuffle(dq_bhnd: torch.Tensor, dq_bnhd: Optional[torch.Tensor] = None,

@@ -1,14 +1,17 @@
 """Host-side mirror of the reference's attention call site (forward and backward).
 
 ``HipAttnFunction`` / ``HipSelfAttention`` / ``HipCrossAttention`` follow
-``training/llama/llama/models/attentions/hipkittens.py:17-61,122-202``: inputs and outputs are BNHD,
-q/k/v are cast to bf16 and made contiguous, O [B,N,H,D] bf16 and L [B,H,1,N] fp32 are allocated by the
-caller side and filled by the blocking ``tk_kernel_fwd.dispatch_fwd(q, k, v, O, L)``; O is returned in the
-input dtype and (q, k, v, O, L) are saved for the backward pass, which runs the reference's three calls
-(hipkittens.py:64-119): ``dispatch_prep(O, dO, delta)``, ``dispatch_bwd_combined(q, k, v, dO, dQ_in, dK, dV,
-L, delta)`` and ``dispatch_dq_shuffle(dQ_in, dQ)``.
+``training/llama/llama/models/attentions/hipkittens.py:17-61,122-202``: inputs and outputs are BNHD, O [B,N,H,D] bf16
+and L [B,H,1,N] fp32 are allocated here, O is returned in the input dtype and (q, k, v, O, L) are saved for the backward
+pass. Like the reference's ``tk_kernel_fwd.dispatch_fwd`` and its three backward calls (hipkittens.py:64-119), forward
+and backward each return when the device is done and raise if a kernel reported a failure; they synchronise once for
+that, not after each kernel.
 
-Differences: dQ_in is not zero-filled (nothing is accumulated into it); a right-padded ``key_padding_mask``
+Differences: bf16 tensors are read through strided TMA descriptors and gradients written through strides, so there are
+no ``.contiguous()`` copies of q, k and v (hipkittens.py:37-39) in either direction, and the modules' packed
+qkv / kv gradient is written in place instead of being stacked from its parts afterwards; dQ is written in its final
+layout, without the zero fill and the shuffle pass (``dispatch_prep`` / ``dispatch_bwd_combined`` /
+``dispatch_dq_shuffle`` stay available in the compiled modules); a right-padded ``key_padding_mask``
 (True = keep, as in ``base.py:88-103``) is honoured through per-batch key lengths, also together with ``causal``
 and with more keys than queries (``base.py:104-116``), where the reference's modules accept the argument and ignore
 it (hipkittens.py:147-162); and causality and the softmax scale are honoured here (they are baked into the reference's compiled module, and its modules
@@ -20,30 +23,7 @@ import torch
 import torch.nn as nn
 from torch.autograd import Function
 
-from ._native import (
-    attn_bwd,
-    attn_bwd_prep,
-    attn_fwd,
-    device_status,
-    load_tk_kernel_bkwd,
-    load_tk_kernel_bkwd_prep,
-    load_tk_kernel_fwd,
-)
-
-_fwd_modules = {}
-_bkwd_modules = {}
-
-
-def _tk_kernel_bkwd(causal: bool):
-    if causal not in _bkwd_modules:
-        _bkwd_modules[causal] = (load_tk_kernel_bkwd(causal), load_tk_kernel_bkwd_prep(causal))
-    return _bkwd_modules[causal]
-
-
-def _tk_kernel_fwd(causal: bool):
-    if causal not in _fwd_modules:
-        _fwd_modules[causal] = load_tk_kernel_fwd(causal)
-    return _fwd_modules[causal]
+from ._native import attn_bwd_strided, attn_fwd, device_status, key_padding_lens
 
 
 def _tma_viewable(t: torch.Tensor) -> bool:
@@ -52,97 +32,114 @@ def _tma_viewable(t: torch.Tensor) -> bool:
             and all(st > 0 and st % 8 == 0 for st in t.stride()[:3]))
 
 
+def _check_qkv(q, k, v):
+    B, N, H, D = q.shape
+    HKV, NK = k.shape[2], k.shape[1]
+    assert k.shape == (B, NK, HKV, D), f"K shape mismatch: expected ({B}, {NK}, {HKV}, {D}), got {k.shape}"
+    assert v.shape == (B, NK, HKV, D), f"V shape mismatch: expected ({B}, {NK}, {HKV}, {D}), got {v.shape}"
+    assert q.is_cuda and k.is_cuda and v.is_cuda, "All tensors must be on CUDA device"
+    assert q.device == k.device == v.device, "All tensors must be on same device"
+    assert H % HKV == 0, f"H ({H}) must be divisible by HKV ({HKV}) for GQA"
+
+
+def _blocking_status(dev, what):
+    status = device_status(dev.index)  # blocks on the device like the reference's dispatch_* calls do
+    if status != 0:
+        raise RuntimeError(f"attention {what} failed on the device (status {status})")
+
+
+def _forward(q, k, v, causal, softmax_scale, kv_lens):
+    O, L = attn_fwd(q, k, v, causal=causal, softmax_scale=softmax_scale, kv_lens=kv_lens)
+    _blocking_status(q.device, "forward")
+    return O, L
+
+
+def _backward(ctx, q, k, v, O, L, dO_bnhd, dQ, dK, dV):
+    assert dO_bnhd.shape == O.shape, f"dO shape mismatch: expected {tuple(O.shape)}, got {dO_bnhd.shape}"
+    assert dO_bnhd.is_cuda and dO_bnhd.device == O.device, "dO must be on correct CUDA device"
+    dO = dO_bnhd.to(torch.bfloat16).contiguous()
+    attn_bwd_strided(q, k, v, O, dO, L, dQ, dK, dV, causal=ctx.causal, softmax_scale=ctx.softmax_scale,
+                     kv_lens=ctx.kv_lens)
+    _blocking_status(O.device, "backward")
+
+
 class HipAttnFunction(Function):
     @staticmethod
     def forward(ctx, q_bnhd: torch.Tensor, k_bnhd: torch.Tensor, v_bnhd: torch.Tensor, causal: bool = True,
                 softmax_scale=None, kv_lens=None):
-        B, N, H, D = q_bnhd.shape
-        HKV, NK = k_bnhd.shape[2], k_bnhd.shape[1]
-        dev = q_bnhd.device
-        out_dtype = q_bnhd.dtype
-        assert k_bnhd.shape == (B, NK, HKV, D), f"K shape mismatch: expected ({B}, {NK}, {HKV}, {D}), got {k_bnhd.shape}"
-        assert v_bnhd.shape == (B, NK, HKV, D), f"V shape mismatch: expected ({B}, {NK}, {HKV}, {D}), got {v_bnhd.shape}"
-        assert q_bnhd.is_cuda and k_bnhd.is_cuda and v_bnhd.is_cuda, "All tensors must be on CUDA device"
-        assert q_bnhd.device == k_bnhd.device == v_bnhd.device, "All tensors must be on same device"
-        assert H % HKV == 0, f"H ({H}) must be divisible by HKV ({HKV}) for GQA"
-
-        O = torch.empty((B, N, H, D), dtype=torch.bfloat16, device=dev)
-        L = torch.empty((B, H, 1, N), dtype=torch.float32, device=dev)
-        ctx.general = kv_lens is not None or NK != N  # cases the reference's compiled modules have no entry for
-        if ctx.general or (all(_tma_viewable(t) for t in (q_bnhd, k_bnhd, v_bnhd)) and not all(
-                t.is_contiguous() for t in (q_bnhd, k_bnhd, v_bnhd))):
-            # bf16 views of a packed projection (what qkv.unbind(2) gives): the kernel reads them through
-            # strided TMA descriptors, so the reference's three .contiguous() copies (hipkittens.py:37-39) go
-            # (key lengths go the same way: the reference's dispatch_fwd has no argument for them)
-            if all(_tma_viewable(t) for t in (q_bnhd, k_bnhd, v_bnhd)):
-                q, k, v = q_bnhd, k_bnhd, v_bnhd
-            else:
-                q, k, v = (t.to(torch.bfloat16).contiguous() for t in (q_bnhd, k_bnhd, v_bnhd))
-            attn_fwd(q, k, v, causal=bool(causal), softmax_scale=softmax_scale, out=O, lse=L, kv_lens=kv_lens)
-            status = device_status(dev.index)  # blocks on the device like dispatch_fwd does
-            if status != 0:
-                raise RuntimeError(f"attention forward failed on the device (status {status})")
+        _check_qkv(q_bnhd, k_bnhd, v_bnhd)
+        if all(_tma_viewable(t) for t in (q_bnhd, k_bnhd, v_bnhd)):
+            q, k, v = q_bnhd, k_bnhd, v_bnhd
         else:
-            q = q_bnhd.to(torch.bfloat16).contiguous()
-            k = k_bnhd.to(torch.bfloat16).contiguous()
-            v = v_bnhd.to(torch.bfloat16).contiguous()
-            _tk_kernel_fwd(bool(causal)).dispatch_fwd(q, k, v, O, L, softmax_scale=softmax_scale)
-
+            q, k, v = (t.to(torch.bfloat16).contiguous() for t in (q_bnhd, k_bnhd, v_bnhd))
+        O, L = _forward(q, k, v, bool(causal), softmax_scale, kv_lens)
         ctx.save_for_backward(q, k, v, O, L)
         ctx.causal = bool(causal)
         ctx.softmax_scale = softmax_scale
         ctx.kv_lens = kv_lens
-        return O.to(out_dtype)
+        return O.to(q_bnhd.dtype)
 
     @staticmethod
     def backward(ctx, dO_bnhd: torch.Tensor):
         q, k, v, O, L = ctx.saved_tensors
-        B, N, H, D = O.shape
-        HKV = k.shape[2]
-        dev = dO_bnhd.device
-        assert dO_bnhd.shape == (B, N, H, D), f"dO shape mismatch: expected ({B}, {N}, {H}, {D}), got {dO_bnhd.shape}"
-        assert dO_bnhd.is_cuda and dO_bnhd.device == O.device, "dO must be on correct CUDA device"
-
-        # the strided forward path saves views; the backward kernels read contiguous tensors
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        dO = dO_bnhd.to(torch.bfloat16).contiguous()
-
-        dQ_in = torch.empty((B, H, N, D), dtype=torch.bfloat16, device=dev)  # BHND (pre-shuffle)
-        dQ = torch.empty((B, N, H, D), dtype=torch.bfloat16, device=dev)
-        dK = torch.empty(k.shape, dtype=torch.bfloat16, device=dev)
-        dV = torch.empty(v.shape, dtype=torch.bfloat16, device=dev)
-        delta = torch.empty((B, H, 1, N), dtype=torch.float32, device=dev)
-
-        if ctx.general:
-            # padded batch, or more keys than queries: the C ABI's general entry (no counterpart among the reference's
-            # three calls); dQ is written in its final layout, so no shuffle pass
-            attn_bwd_prep(O, dO, delta)
-            attn_bwd(q, k, v, dO, L, delta, causal=ctx.causal, softmax_scale=ctx.softmax_scale, dq=dQ, dk=dK, dv=dV,
-                     kv_lens=ctx.kv_lens)
-            status = device_status(dev.index)
-            if status != 0:
-                raise RuntimeError(f"attention backward failed on the device (status {status})")
-            return dQ.to(dO_bnhd.dtype), dK.to(dO_bnhd.dtype), dV.to(dO_bnhd.dtype), None, None, None
-
-        tk_kernel_bkwd, tk_kernel_bkwd_prep = _tk_kernel_bkwd(ctx.causal)
-        tk_kernel_bkwd_prep.dispatch_prep(O, dO, delta)
-        tk_kernel_bkwd.dispatch_bwd_combined(q, k, v, dO, dQ_in, dK, dV, L, delta, causal=ctx.causal,
-                                             softmax_scale=ctx.softmax_scale)
-        tk_kernel_bkwd_prep.dispatch_dq_shuffle(dQ_in, dQ)
-
+        dQ, dK, dV = (torch.empty(t.shape, dtype=torch.bfloat16, device=t.device) for t in (q, k, v))
+        _backward(ctx, q, k, v, O, L, dO_bnhd, dQ, dK, dV)
         return dQ.to(dO_bnhd.dtype), dK.to(dO_bnhd.dtype), dV.to(dO_bnhd.dtype), None, None, None
 
 
-def _lens_from_key_padding_mask(mask: torch.Tensor, seqlen: int):
+class _PackedAttnFunction(Function):
+    """``HipAttnFunction`` on the modules' packed bf16 projections: `packed` [B,S,2,H_KV,D] with a `q` of its own, or
+    [B,S,3,H,D] with q = None. q, k and v are read as strided views and the packed gradient is written in place (as
+    ``unbind`` outputs the three gradients would be stacked by a copy of them all)."""
+
+    @staticmethod
+    def forward(ctx, q, packed, causal, softmax_scale, kv_lens):
+        qkv = packed.unbind(dim=2) if q is None else (q, *packed.unbind(dim=2))
+        O, L = _forward(*qkv, causal, softmax_scale, kv_lens)
+        ctx.save_for_backward(*([packed] if q is None else [q, packed]), O, L)
+        ctx.causal = causal
+        ctx.softmax_scale = softmax_scale
+        ctx.kv_lens = kv_lens
+        return O
+
+    @staticmethod
+    def backward(ctx, dO_bnhd):
+        *q, packed, O, L = ctx.saved_tensors
+        d_packed = torch.empty(packed.shape, dtype=torch.bfloat16, device=packed.device)
+        d_q = [torch.empty(t.shape, dtype=torch.bfloat16, device=t.device) for t in q]
+        _backward(ctx, *q, *packed.unbind(dim=2), O, L, dO_bnhd, *d_q, *d_packed.unbind(dim=2))
+        return d_q[0] if q else None, d_packed, None, None, None
+
+
+def _attend(q, packed, causal, softmax_scale, key_padding_mask):
+    """Attention of q (None: the first of the packed tensors) over a packed projection [B, S, 2 or 3, H, D]."""
+    views = packed.unbind(dim=2) if q is None else (q, *packed.unbind(dim=2))
+    _check_qkv(*views)
+    kv_lens = bad = None
+    if key_padding_mask is not None:
+        kv_lens, bad = _lens_from_key_padding_mask(key_padding_mask, packed)
+    if all(_tma_viewable(t) for t in views):
+        out = _PackedAttnFunction.apply(q, packed, bool(causal), softmax_scale, kv_lens)
+    else:
+        out = HipAttnFunction.apply(*views, causal, softmax_scale, kv_lens)
+    # read here, behind the forward's own synchronisation: whatever the mask, the lengths are clamped by the kernels
+    if bad is not None and int(bad) != 0:
+        raise ValueError(_BAD_MASK)
+    return out.to(views[0].dtype).contiguous()
+
+
+_BAD_MASK = "only right-padded key_padding_mask (a kept prefix of at least one key per row) is supported"
+
+
+def _lens_from_key_padding_mask(mask: torch.Tensor, packed: torch.Tensor):
     """(B, S) bool, True = keep (base.py:88-89) -> int32 key lengths, for masks that keep a prefix of each row
-    (right padding, what padded batches have). Anything else cannot be expressed as lengths and is refused."""
-    if mask.dim() != 2 or mask.shape[1] != seqlen or mask.dtype != torch.bool:
+    (right padding, what padded batches have), and a flag on the device: non-zero if a row is anything else, which
+    cannot be expressed as lengths and is refused."""
+    if mask.dim() != 2 or mask.shape[1] != packed.shape[1] or mask.dtype != torch.bool:
         raise ValueError("key_padding_mask must be a bool tensor (batch, seqlen), True = keep")
-    lens = mask.sum(dim=1).to(torch.int32)
-    prefix = torch.arange(seqlen, device=mask.device).unsqueeze(0) < lens.unsqueeze(1)
-    if not bool((mask == prefix).all()) or bool((lens < 1).any()):
-        raise ValueError("only right-padded key_padding_mask (a kept prefix of at least one key per row) is supported")
-    return lens.contiguous()
+    if mask.device != packed.device:
+        raise RuntimeError("key_padding_mask must be on the device of q, k and v")
+    return key_padding_lens(mask)
 
 
 class HipSelfAttention(nn.Module):
@@ -161,12 +158,7 @@ class HipSelfAttention(nn.Module):
         assert qkv.dtype in [torch.float16, torch.bfloat16]
         assert qkv.is_cuda
         causal = self.causal if causal is None else causal
-        kv_lens = None
-        if key_padding_mask is not None:
-            kv_lens = _lens_from_key_padding_mask(key_padding_mask, qkv.shape[1])
-        q, k, v = qkv.unbind(dim=2)
-        out_bnhd = HipAttnFunction.apply(q, k, v, causal, self.softmax_scale, kv_lens)
-        return out_bnhd.to(q.dtype).contiguous()
+        return _attend(None, qkv, causal, self.softmax_scale, key_padding_mask)
 
 
 class HipCrossAttention(nn.Module):
@@ -185,9 +177,4 @@ class HipCrossAttention(nn.Module):
         batch_size = q.shape[0]
         causal = self.causal if causal is None else causal
         assert kv.shape[0] == batch_size and kv.shape[4] == q.shape[3]
-        kv_lens = None
-        if key_padding_mask is not None:
-            kv_lens = _lens_from_key_padding_mask(key_padding_mask, kv.shape[1])
-        k, v = kv.unbind(dim=2)
-        out_bnhd = HipAttnFunction.apply(q, k, v, causal, self.softmax_scale, kv_lens)
-        return out_bnhd.to(q.dtype).contiguous()
+        return _attend(q, kv, causal, self.softmax_scale, key_padding_mask)

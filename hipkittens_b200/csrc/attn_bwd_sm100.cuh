@@ -59,9 +59,11 @@ struct BwdParams {
   const float* lse;     // [B,H,1,N] from the forward pass (natural log)
   const float* delta;   // [B,H,1,N] rowsum(dO * O)
   __nv_bfloat16* dq;    // written through the three strides below
-  __nv_bfloat16* dk;    // [B,NK,H_KV,D]
-  __nv_bfloat16* dv;    // [B,NK,H_KV,D]
+  __nv_bfloat16* dk;    // [B,NK,H_KV,D], through strides of their own: the gradient of a packed projection is
+  __nv_bfloat16* dv;    // written in place, without the copy that would stack dK and dV afterwards
   long long dq_stride_b, dq_stride_n, dq_stride_h;  // elements; [B,N,H,D] or [B,H,N,D]
+  long long dk_stride_b, dk_stride_n, dk_stride_h;
+  long long dv_stride_b, dv_stride_n, dv_stride_h;
   int B, N, H, H_KV;    // N = query rows per batch element
   int NK;               // keys per batch element (N for self-attention)
   int n_items;
@@ -88,6 +90,13 @@ struct BwdParams {
   long long* trace;     // [4 roles][4096] clock stamps of CTA 0 (debug builds only)
 #endif
 };
+
+__device__ __forceinline__ __nv_bfloat16* dk_row(const BwdParams& p, int b, int key, int kvh) {
+  return p.dk + b * p.dk_stride_b + key * p.dk_stride_n + kvh * p.dk_stride_h;
+}
+__device__ __forceinline__ __nv_bfloat16* dv_row(const BwdParams& p, int b, int key, int kvh) {
+  return p.dv + b * p.dv_stride_b + key * p.dv_stride_n + kvh * p.dv_stride_h;
+}
 
 template <int D>
 struct BwdSmem {
@@ -482,12 +491,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         // nobody sees this key block (padding, or causal with every query before it): its gradients are zero and no
         // product was issued for it
         if (w.j * kBlockN + row < p.NK) {
-          const size_t off =
-              ((static_cast<size_t>(w.b) * p.NK + w.j * kBlockN + row) * p.H_KV + w.kvh) * D + part * (D / kBwdParts);
+          __nv_bfloat16* const dk = dk_row(p, w.b, w.j * kBlockN + row, w.kvh) + part * (D / kBwdParts);
+          __nv_bfloat16* const dv = dv_row(p, w.b, w.j * kBlockN + row, w.kvh) + part * (D / kBwdParts);
 #pragma unroll
           for (int v = 0; v < D / kBwdParts / 8; ++v) {
-            reinterpret_cast<uint4*>(p.dk + off)[v] = make_uint4(0, 0, 0, 0);
-            reinterpret_cast<uint4*>(p.dv + off)[v] = make_uint4(0, 0, 0, 0);
+            reinterpret_cast<uint4*>(dk)[v] = make_uint4(0, 0, 0, 0);
+            reinterpret_cast<uint4*>(dv)[v] = make_uint4(0, 0, 0, 0);
           }
         }
         continue;
@@ -621,10 +630,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       if (!ok) break;
       ++acc_cnt;
       tc_fence_after();
-      const size_t off = ((static_cast<size_t>(w.b) * p.NK + w.j * kBlockN + row) * p.H_KV + w.kvh) * D + part * (D / kBwdParts);
       const bool row_exists = w.j * kBlockN + row < p.NK;  // keys of a partial last block beyond NK are computed, not stored
-      bwd_store_part_row<D>(tmem + lane_addr + cDK + part * (D / kBwdParts), p.dk + off, p.scale, row_exists);
-      bwd_store_part_row<D>(tmem + lane_addr + cDV + part * (D / kBwdParts), p.dv + off, 1.0f, row_exists);
+      const int key = w.j * kBlockN + row;
+      bwd_store_part_row<D>(tmem + lane_addr + cDK + part * (D / kBwdParts),
+                            dk_row(p, w.b, key, w.kvh) + part * (D / kBwdParts), p.scale, row_exists);
+      bwd_store_part_row<D>(tmem + lane_addr + cDV + part * (D / kBwdParts),
+                            dv_row(p, w.b, key, w.kvh) + part * (D / kBwdParts), 1.0f, row_exists);
       tc_fence_before();  // orders these reads before the next item's first dV product (published through P_FULL)
     }
   } else {

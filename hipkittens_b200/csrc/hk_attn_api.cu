@@ -18,6 +18,7 @@
 #define HK_BWD_PARTS 2
 #include "attn_bwd_sm100.cuh"
 #include "attn_fwd_sm100.cuh"
+#include "key_padding_sm100.cuh"
 #include "paged_decode_sm100.cuh"
 #include "paged_kv_append_sm100.cuh"
 #include "rotary_sm100.cuh"
@@ -60,7 +61,8 @@ struct DeviceState {
   bool ready = false;     // set once init_device succeeded; a failed attempt is retried by the next call
   int sm_count = 0;
   int cc_major = 0;
-  int* status = nullptr;  // device word
+  int* status = nullptr;       // the status word, device address (kernels write it only when something went wrong)
+  int* status_host = nullptr;  // ... and host address: mapped memory, so that reading it needs no copy
 };
 DeviceState g_dev[kMaxDevices];
 
@@ -150,15 +152,20 @@ int init_device(int device) {
   if ((rc = prepare_bwd_kernels<128, true>()) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<64, false>()) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<64, true>()) != HK_OK) return rc;
-  // the one allocation this library makes: the status word (last, so that a failure above leaves nothing behind)
-  int* word = nullptr;
-  HK_CUDA(cudaMalloc(&word, sizeof(int)));
-  cudaError_t e = cudaMemset(word, 0, sizeof(int));
+  // the one allocation this library makes: the status word (last, so that a failure above leaves nothing behind). It
+  // lies in mapped host memory: a blocking call reads it after its synchronisation, and a 4-byte copy from device
+  // memory to a pageable variable took 18 us of every one of them.
+  void* word = nullptr;
+  HK_CUDA(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+  *static_cast<volatile int*>(word) = 0;
+  void* dev_word = nullptr;
+  cudaError_t e = cudaHostGetDevicePointer(&dev_word, word, 0);
   if (e != cudaSuccess) {
-    cudaFree(word);
-    return cuda_fail(e, "cudaMemset(status word)");
+    cudaFreeHost(word);
+    return cuda_fail(e, "cudaHostGetDevicePointer(status word)");
   }
-  st.status = word;
+  st.status_host = static_cast<int*>(word);
+  st.status = static_cast<int*>(dev_word);
   return HK_OK;
 }
 
@@ -245,9 +252,18 @@ int make_bnhd_map(CUtensorMap* map, const void* base, int B, int N, int heads, i
   cuuint64_t strides[3] = {cuuint64_t(st[2]) * 2, cuuint64_t(st[1]) * 2, cuuint64_t(st[0]) * 2};
   cuuint32_t box[4] = {64, 1, cuuint32_t(box_rows), 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // a thread that has made no runtime call yet (autograd's) has no current context: let the runtime bind the
+    // device's own and try again
+    HK_CUDA(cudaFree(nullptr));
+    r = encode();
+  }
   if (r != CUDA_SUCCESS) {
     snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled failed with CUresult %d", int(r));
     return HK_ECUDA;
@@ -484,6 +500,20 @@ int hk_attn_fwd_paged(const void* q, const void* k_pages, const void* v_pages, c
                     block_table, max_pages_per_seq, num_pages, causal, softmax_scale, device, cuda_stream);
 }
 
+static int prep_launch(const void* o, const void* d_o, float* delta, int B, int N, int H, int D, cudaStream_t stream) {
+  const long long rows = static_cast<long long>(B) * N * H;
+  if (rows > 0x7fffffffll) return HK_EINVAL;  // rows are indexed with int
+  const int rows_per_block = hk::row_pass_rows(D / 8);
+  const unsigned blocks = unsigned((rows + rows_per_block - 1) / rows_per_block);
+  const auto* po = static_cast<const __nv_bfloat16*>(o);
+  const auto* pd = static_cast<const __nv_bfloat16*>(d_o);
+  auto* fn = D == 128 ? hk::attn_bwd_prep_kernel<128> : hk::attn_bwd_prep_kernel<64>;
+  fn<<<blocks, 256, 0, stream>>>(po, pd, delta, int(rows), N, H, hk::FastDiv(H), hk::FastDiv(N));
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  HK_CUDA(cudaGetLastError());
+  return HK_OK;
+}
+
 int hk_attn_bwd_prep(const void* o, const void* d_o, float* delta, int B, int N, int H, int D, int device,
                      void* cuda_stream) {
   if (!o || !d_o || !delta) return HK_EINVAL;
@@ -494,18 +524,7 @@ int hk_attn_bwd_prep(const void* o, const void* d_o, float* delta, int B, int N,
   DeviceScope scope;
   int rc = scope.enter(device, &st);
   if (rc != HK_OK) return rc;
-  const long long rows = static_cast<long long>(B) * N * H;
-  if (rows > 0x7fffffffll) return HK_EINVAL;  // rows are indexed with int
-  const int rows_per_block = hk::row_pass_rows(D / 8);
-  const unsigned blocks = unsigned((rows + rows_per_block - 1) / rows_per_block);
-  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-  const auto* po = static_cast<const __nv_bfloat16*>(o);
-  const auto* pd = static_cast<const __nv_bfloat16*>(d_o);
-  auto* fn = D == 128 ? hk::attn_bwd_prep_kernel<128> : hk::attn_bwd_prep_kernel<64>;
-  fn<<<blocks, 256, 0, stream>>>(po, pd, delta, int(rows), N, H, hk::FastDiv(H), hk::FastDiv(N));
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  HK_CUDA(cudaGetLastError());
-  return HK_OK;
+  return prep_launch(o, d_o, delta, B, N, H, D, static_cast<cudaStream_t>(cuda_stream));
 }
 
 int hk_attn_bwd(const void* q, const void* k, const void* v, const void* d_o, const float* lse, const float* delta,
@@ -523,16 +542,24 @@ int hk_attn_bwd_varlen(const void* q, const void* k, const void* v, const void* 
                            dq_layout, device, cuda_stream);
 }
 
-int hk_attn_bwd_cross(const void* q, const void* k, const void* v, const void* d_o, const float* lse,
-                      const float* delta, void* dq, void* dk, void* dv, int B, int N, int NK, int H, int H_KV, int D,
-                      const int32_t* kv_lens, int causal, float softmax_scale, int dq_layout, int device,
+// Element strides of the batch, sequence and head dimensions of the tensors of one backward call.
+struct BwdStrides {
+  const long long *q, *k, *v, *dq, *dk, *dv;
+};
+
+// Shared tail of the backward entries. o != null: delta is computed here first.
+static int bwd_launch(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse,
+                      float* delta, void* dq, void* dk, void* dv, int B, int N, int NK, int H, int H_KV, int D,
+                      const BwdStrides& s, const int32_t* kv_lens, int causal, float softmax_scale, int device,
                       void* cuda_stream) {
   if (!q || !k || !v || !d_o || !lse || !delta || !dq || !dk || !dv) return HK_EINVAL;
   if (B <= 0 || N <= 0 || NK <= 0 || H <= 0 || H_KV <= 0) return HK_EINVAL;
   if (D != 64 && D != 128) return HK_EUNSUPPORTED;
   if (H % H_KV != 0) return HK_EINVAL;
-  if (dq_layout != HK_DQ_BNHD && dq_layout != HK_DQ_BHND) return HK_EINVAL;
-  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(d_o) || !aligned16(dq) || !aligned16(dk) ||
+  for (const long long* s3 : {s.q, s.k, s.v, s.dq, s.dk, s.dv})
+    for (int i = 0; i < 3; ++i)
+      if (s3[i] <= 0 || s3[i] % 8 != 0 || s3[i] >= (1ll << 39)) return HK_EINVAL;
+  if ((o && !aligned16(o)) || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(d_o) || !aligned16(dq) || !aligned16(dk) ||
       !aligned16(dv) || (reinterpret_cast<uintptr_t>(lse) & 3) || (reinterpret_cast<uintptr_t>(delta) & 3))
     return HK_EINVAL;
   DeviceState* st = nullptr;
@@ -540,13 +567,14 @@ int hk_attn_bwd_cross(const void* q, const void* k, const void* v, const void* d
   int rc = scope.enter(device, &st);
   if (rc != HK_OK) return rc;
 
-  const long long qs[3] = {(long long)N * H * D, (long long)H * D, D};
-  const long long ks[3] = {(long long)NK * H_KV * D, (long long)H_KV * D, D};
+  const long long dos[3] = {(long long)N * H * D, (long long)H * D, D};
   CUtensorMap tq, tk, tv, tdo;
-  if ((rc = make_bnhd_map(&tq, q, B, N, H, D, qs)) != HK_OK) return rc;
-  if ((rc = make_bnhd_map(&tk, k, B, NK, H_KV, D, ks)) != HK_OK) return rc;
-  if ((rc = make_bnhd_map(&tv, v, B, NK, H_KV, D, ks)) != HK_OK) return rc;
-  if ((rc = make_bnhd_map(&tdo, d_o, B, N, H, D, qs)) != HK_OK) return rc;
+  if ((rc = make_bnhd_map(&tq, q, B, N, H, D, s.q)) != HK_OK) return rc;
+  if ((rc = make_bnhd_map(&tk, k, B, NK, H_KV, D, s.k)) != HK_OK) return rc;
+  if ((rc = make_bnhd_map(&tv, v, B, NK, H_KV, D, s.v)) != HK_OK) return rc;
+  if ((rc = make_bnhd_map(&tdo, d_o, B, N, H, D, dos)) != HK_OK) return rc;
+  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+  if (o && (rc = prep_launch(o, d_o, delta, B, N, H, D, stream)) != HK_OK) return rc;
 
   hk::BwdParams p;
   p.lse = lse;
@@ -554,9 +582,9 @@ int hk_attn_bwd_cross(const void* q, const void* k, const void* v, const void* d
   p.dq = static_cast<__nv_bfloat16*>(dq);
   p.dk = static_cast<__nv_bfloat16*>(dk);
   p.dv = static_cast<__nv_bfloat16*>(dv);
-  p.dq_stride_b = (long long)N * H * D;
-  p.dq_stride_n = dq_layout == HK_DQ_BNHD ? (long long)H * D : D;
-  p.dq_stride_h = dq_layout == HK_DQ_BNHD ? D : (long long)N * D;
+  p.dq_stride_b = s.dq[0], p.dq_stride_n = s.dq[1], p.dq_stride_h = s.dq[2];
+  p.dk_stride_b = s.dk[0], p.dk_stride_n = s.dk[1], p.dk_stride_h = s.dk[2];
+  p.dv_stride_b = s.dv[0], p.dv_stride_n = s.dv[1], p.dv_stride_h = s.dv[2];
   p.B = B;
   p.N = N;
   p.NK = NK;
@@ -577,11 +605,50 @@ int hk_attn_bwd_cross(const void* q, const void* k, const void* v, const void* d
 #ifdef HK_TRACE
   p.trace = g_trace_buf;
 #endif
-  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   if (D == 128) return causal ? launch_bwd<128, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, st->sm_count, stream)
                               : launch_bwd<128, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, st->sm_count, stream);
   return causal ? launch_bwd<64, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, st->sm_count, stream)
                 : launch_bwd<64, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, st->sm_count, stream);
+}
+
+int hk_attn_bwd_cross(const void* q, const void* k, const void* v, const void* d_o, const float* lse,
+                      const float* delta, void* dq, void* dk, void* dv, int B, int N, int NK, int H, int H_KV, int D,
+                      const int32_t* kv_lens, int causal, float softmax_scale, int dq_layout, int device,
+                      void* cuda_stream) {
+  if (dq_layout != HK_DQ_BNHD && dq_layout != HK_DQ_BHND) return HK_EINVAL;
+  if (N <= 0 || NK <= 0 || H <= 0 || H_KV <= 0) return HK_EINVAL;
+  if (D != 64 && D != 128) return HK_EUNSUPPORTED;
+  const long long qs[3] = {(long long)N * H * D, (long long)H * D, D};
+  const long long ks[3] = {(long long)NK * H_KV * D, (long long)H_KV * D, D};
+  const long long dqs[3] = {(long long)N * H * D, D, (long long)N * D};  // [B, H, N, D]
+  const BwdStrides s{qs, ks, ks, dq_layout == HK_DQ_BNHD ? qs : dqs, ks, ks};
+  return bwd_launch(q, k, v, nullptr, d_o, lse, const_cast<float*>(delta), dq, dk, dv, B, N, NK, H, H_KV, D, s, kv_lens,
+                    causal, softmax_scale, device, cuda_stream);
+}
+
+int hk_attn_bwd_strided(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse,
+                        float* delta, void* dq, void* dk, void* dv, int B, int N, int NK, int H, int H_KV, int D,
+                        const long long* q_strides, const long long* k_strides, const long long* v_strides,
+                        const long long* dq_strides, const long long* dk_strides, const long long* dv_strides,
+                        const int32_t* kv_lens, int causal, float softmax_scale, int device, void* cuda_stream) {
+  if (!q_strides || !k_strides || !v_strides || !dq_strides || !dk_strides || !dv_strides) return HK_EINVAL;
+  const BwdStrides s{q_strides, k_strides, v_strides, dq_strides, dk_strides, dv_strides};
+  return bwd_launch(q, k, v, o, d_o, lse, delta, dq, dk, dv, B, N, NK, H, H_KV, D, s, kv_lens, causal, softmax_scale,
+                    device, cuda_stream);
+}
+
+int hk_key_padding_lens(const unsigned char* mask, int32_t* lens, int32_t* bad, int B, int N, int device,
+                        void* cuda_stream) {
+  if (!mask || !lens || !bad || B <= 0 || N <= 0) return HK_EINVAL;
+  if ((reinterpret_cast<uintptr_t>(lens) & 3) || (reinterpret_cast<uintptr_t>(bad) & 3)) return HK_EINVAL;
+  DeviceState* st = nullptr;
+  DeviceScope scope;
+  int rc = scope.enter(device, &st);
+  if (rc != HK_OK) return rc;
+  hk::key_padding_lens_kernel<<<B, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(mask, lens, bad, N);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  HK_CUDA(cudaGetLastError());
+  return HK_OK;
 }
 
 int hk_attn_dq_shuffle(const void* dq_bhnd, void* dq_bnhd, int B, int N, int H, int D, int device,
@@ -783,9 +850,9 @@ int hk_last_device_status(int device) {
   int rc = scope.enter(device, &st);
   if (rc != HK_OK) return rc;
   HK_CUDA(cudaDeviceSynchronize());
-  int word = 0;
-  HK_CUDA(cudaMemcpy(&word, st->status, sizeof(int), cudaMemcpyDeviceToHost));
-  if (word != 0) HK_CUDA(cudaMemset(st->status, 0, sizeof(int)));
+  volatile int* const host = st->status_host;
+  const int word = *host;
+  if (word != 0) *host = 0;
   return status_to_code(word);
 }
 

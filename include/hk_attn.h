@@ -164,6 +164,23 @@ int hk_attn_bwd_cross(const void* q, const void* k, const void* v, const void* d
                       const int32_t* kv_lens, int causal, float softmax_scale, int dq_layout, int device,
                       void* cuda_stream);
 
+/* hk_attn_bwd_cross on strided tensors: q, k, v are read and dq, dk, dv written through element strides of the batch,
+ * sequence and head dimensions (positive multiples of 8; the last dimension is contiguous), so that the views of a
+ * packed projection (qkv.unbind(2), the reference's call site, hipkittens.py:37-39) are read without copies and
+ * the gradient of the packed tensor is written in place. d_o and o are contiguous [B,Nq,H,D].
+ *   o : the forward's output, or NULL. Not NULL: delta is computed first (hk_attn_bwd_prep) and written to `delta`;
+ *       NULL: `delta` is an input, as in hk_attn_bwd_cross. */
+int hk_attn_bwd_strided(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse,
+                        float* delta, void* dq, void* dk, void* dv, int B, int Nq, int Nk, int H, int H_KV, int D,
+                        const long long* q_strides, const long long* k_strides, const long long* v_strides,
+                        const long long* dq_strides, const long long* dk_strides, const long long* dv_strides,
+                        const int32_t* kv_lens, int causal, float softmax_scale, int device, void* cuda_stream);
+
+/* Key lengths of a right-padded batch: mask is DEVICE bool (one byte) [B, N] contiguous, True = keep (base.py:88-103);
+ * lens[b] = kept keys of row b. *bad, zero on entry, becomes 1 if a row does not keep a prefix of at least one key. */
+int hk_key_padding_lens(const unsigned char* mask, int32_t* lens, int32_t* bad, int B, int N, int device,
+                        void* cuda_stream);
+
 /* dq_bnhd[b,n,h,:] = dq_bhnd[b,h,n,:]. Replaces dispatch_dq_shuffle (attn_bkwd_prep.cpp:199-223,236-239); only
  * needed after hk_attn_bwd with HK_DQ_BHND. D a multiple of 8; the two buffers must not alias. */
 int hk_attn_dq_shuffle(const void* dq_bhnd, void* dq_bnhd, int B, int N, int H, int D, int device,

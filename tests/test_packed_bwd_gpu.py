@@ -1,0 +1,68 @@
+"""The modules' packed path: q, k, v read as views of a packed projection in both directions, its gradient written in
+place, key lengths taken from the mask on the device."""
+import pytest
+import torch
+
+from hipkittens_b200 import _native
+from hipkittens_b200.attention import HipAttnFunction, HipCrossAttention, HipSelfAttention
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*shape, seed):
+    return torch.randn(shape, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).cuda()
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("b,n,nk,h,hkv,d", [(1, 1, 1, 1, 1, 64), (2, 129, 129, 4, 2, 128), (3, 200, 333, 6, 2, 64),
+                                            (1, 256, 256, 8, 8, 128), (2, 300, 130, 2, 1, 64)])
+def test_packed_gradient_is_the_gradient_of_the_parts(b, n, nk, h, hkv, d, causal):
+    """Same kernels on the same values: O and every gradient are bit-identical to the contiguous call's."""
+    q, kv, d_o = _rand(b, n, h, d, seed=1), _rand(b, nk, 2, hkv, d, seed=2), _rand(b, n, h, d, seed=3)
+    qp, kvp = q.clone().requires_grad_(), kv.clone().requires_grad_()
+    out = HipCrossAttention(causal=causal)(qp, kvp)
+    out.backward(d_o)
+    parts = [t.clone(memory_format=torch.contiguous_format).requires_grad_()
+             for t in (q, kv[:, :, 0], kv[:, :, 1])]
+    ref = HipAttnFunction.apply(*parts, causal)
+    ref.backward(d_o)
+    assert torch.equal(out, ref) and torch.equal(qp.grad, parts[0].grad)
+    assert kvp.grad.is_contiguous()
+    assert torch.equal(kvp.grad[:, :, 0], parts[1].grad) and torch.equal(kvp.grad[:, :, 1], parts[2].grad)
+    if n == nk and h == hkv:
+        qkv = torch.stack([q, kv[:, :, 0], kv[:, :, 1]], dim=2).detach().requires_grad_()
+        HipSelfAttention(causal=causal)(qkv).backward(d_o)
+        for i in range(3):
+            assert torch.equal(qkv.grad[:, :, i], parts[i].grad)
+
+
+def test_float16_projection_takes_the_converting_path():
+    qkv = _rand(2, 160, 3, 2, 64, seed=4).half().requires_grad_()
+    out = HipSelfAttention()(qkv)
+    d_o = _rand(2, 160, 2, 64, seed=5).half()
+    out.backward(d_o)
+    ref = qkv.detach().to(torch.bfloat16).requires_grad_()
+    HipSelfAttention()(ref).backward(d_o.to(torch.bfloat16))
+    assert out.dtype == torch.float16 and qkv.grad.dtype == torch.float16
+    assert torch.equal(qkv.grad, ref.grad.half())
+
+
+@pytest.mark.parametrize("b,n", [(1, 1), (3, 255), (2, 256), (5, 1000)])
+def test_key_padding_lens(b, n):
+    gen = torch.Generator().manual_seed(n)
+    lens = torch.randint(1, n + 1, (b,), generator=gen)
+    mask = torch.arange(n)[None] < lens[:, None]
+    got, bad = _native.key_padding_lens(mask.cuda())
+    assert got.cpu().tolist() == lens.tolist() and int(bad) == 0
+    wide = torch.zeros(b, 2 * n, dtype=torch.bool)  # a mask that is a strided view
+    wide[:, ::2] = mask
+    got, bad = _native.key_padding_lens(wide.cuda()[:, ::2])
+    assert got.cpu().tolist() == lens.tolist() and int(bad) == 0
+    empty = mask.clone()
+    empty[b - 1] = False
+    assert int(_native.key_padding_lens(empty.cuda())[1]) != 0
+    if n > 2:
+        hole = mask.clone()
+        hole[0] = True
+        hole[0, n // 2] = False
+        assert int(_native.key_padding_lens(hole.cuda())[1]) != 0
