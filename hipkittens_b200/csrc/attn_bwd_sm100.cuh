@@ -80,7 +80,7 @@ struct BwdParams {
   FastDiv fd_inner;     // dQ kernel: query tiles (non-causal order) or G (causal order)
   FastDiv fd_group;     // causal: items of a full group
   FastDiv fd_in_grp, fd_in_grp_last;  // causal: items per key block / query tile in a full group, in the last group
-  int n_pairs;          // causal dK/dV kernel: pairs of key blocks (j, NBK - 1 - j) over all units
+  int n_pairs;          // causal dK/dV kernel: pairs of key blocks (j, NBK - 1 - j) over all units; 0: single blocks
   FastDiv fd_pairs;     // pairs per unit, (NBK + 1) / 2
   float scale;
   float scale_log2;
@@ -350,9 +350,12 @@ struct DkdvItem {
 // N = 8192, and a unit has fewer blocks than the GPU has SMs, so no dealing of single blocks to CTAs balances. The
 // blocks are therefore dealt in pairs (j, NBK - 1 - j) of the same unit, which all cost the same: a CTA's round 2r
 // is the first block of its r-th pair and round 2r + 1 the second (none for the middle block of an odd count).
+// When there are no more blocks than SMs every block gets a CTA of its own instead (n_pairs = 0): the longest block
+// alone is then the kernel's time, not the longest plus the shortest (B2 N384 H8/2 D128, 12 blocks: 34.6 us for the
+// kernel in pairs, 25.1 us singly).
 template <bool CAUSAL>
 __device__ __forceinline__ int dkdv_item_for_round(const BwdParams& p, int round, int cta, int n_cta) {
-  if (!CAUSAL) return item_for_round(p, round, cta, n_cta);
+  if (!CAUSAL || p.n_pairs == 0) return item_for_round(p, round, cta, n_cta);
   const int pair = (round >> 1) * n_cta + cta;
   if (pair >= p.n_pairs) return -1;
   int unit, jp;

@@ -325,7 +325,12 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   p.n_items = B * H_KV * nbk;
   int grid = p.n_items < sm_count ? p.n_items : sm_count;
   set_bwd_decode(p, nbk, 1, 1, grid, CAUSAL);
-  if (CAUSAL) {
+  p.n_pairs = 0;
+  if (CAUSAL && p.n_items <= sm_count) {
+    p.group_items = p.n_items;
+    p.rounds_per_group = p.total_rounds = 1;
+    p.fd_rounds = hk::FastDiv(1);
+  } else if (CAUSAL) {
     // key blocks are dealt in pairs (j, nbk - 1 - j) of equal cost, two rounds per pair
     const int per_unit = (nbk + 1) / 2;
     p.n_pairs = B * H_KV * per_unit;

@@ -47,6 +47,31 @@ def test_float16_projection_takes_the_converting_path():
     assert torch.equal(qkv.grad, ref.grad.half())
 
 
+@pytest.mark.parametrize("b,nk,hkv", [(1, 128 * 148, 1), (1, 128 * 148 + 1, 1), (4, 128 * 37, 1), (2, 128 * 37, 2),
+                                      (3, 128 * 50, 1)])
+def test_causal_key_blocks_around_the_number_of_sms(b, nk, hkv):
+    """One CTA per key block up to the number of SMs, pairs of blocks beyond: every block is served exactly once, so a
+    batch element's dK and dV are bit-identical to those of the call that holds it alone."""
+    n = 200
+    q, kv, d_o = _rand(b, n, 2 * hkv, 64, seed=6), _rand(b, nk, 2, hkv, 64, seed=7), _rand(b, n, 2 * hkv, 64, seed=8)
+
+    def grads(sl):
+        qd, kvd = q[sl].clone().requires_grad_(), kv[sl].clone().requires_grad_()
+        HipCrossAttention(causal=True)(qd, kvd).backward(d_o[sl])
+        return kvd.grad
+
+    got = grads(slice(0, b))
+    assert bool(torch.isfinite(got).all()) and float(got.float().abs().max()) > 0
+    if b > 1:
+        for i in range(b):
+            assert torch.equal(got[i:i + 1], grads(slice(i, i + 1)))
+    else:  # a second batch element changes the dealing, not the gradients
+        two = torch.cat([kv, kv]).requires_grad_()
+        q2 = torch.cat([q, q]).requires_grad_()
+        HipCrossAttention(causal=True)(q2, two).backward(torch.cat([d_o, d_o]))
+        assert torch.equal(two.grad[:1], got) and torch.equal(two.grad[1:], got)
+
+
 @pytest.mark.parametrize("b,n", [(1, 1), (3, 255), (2, 256), (5, 1000)])
 def test_key_padding_lens(b, n):
     gen = torch.Generator().manual_seed(n)
