@@ -13,6 +13,8 @@ into directories that mirror the reference's:
     kernels/attn/gqa{,_causal}_backwards/tk_kernel_bkwd_prep  dispatch_prep, dispatch_dq_shuffle
     kernels/rotary/tk_kernel                       dispatch_rotary
 
+and ``lib/_torch_front``, the native half of the tensor front ends in ``_native.py``.
+
 Run as ``python -m hipkittens_b200._build``. nvcc cross-compiles without a GPU.
 """
 from __future__ import annotations
@@ -136,10 +138,32 @@ def build_shims(force: bool = False):
     return out
 
 
+def build_torch_front(force: bool = False) -> str:
+    """``lib/_torch_front``: the tensor front ends in native code, the one piece that links against libtorch."""
+    import torch
+
+    target = shim_path("lib", "_torch_front")
+    src = os.path.join(CSRC, "torch_front.cpp")
+    if not force and _newer(target, [src, os.path.join(INCLUDE, "hk_attn.h"), LIB_PATH]):
+        return target
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(nvcc_path())) or "/usr/local/cuda"
+    _run([
+        "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+        "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+        "-I", os.path.join(cuda, "include"), "-I", sysconfig.get_paths()["include"],
+        src, "-o", target,
+        "-L", LIB_DIR, "-lhk_attn", "-Wl,-rpath,$ORIGIN",
+        "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+    ])
+    return target
+
+
 def build_all(force: bool = False):
     lib = build_lib(force)
     shims = build_shims(force)
-    return [lib, *shims]
+    return [lib, *shims, build_torch_front(force)]
 
 
 if __name__ == "__main__":

@@ -146,6 +146,27 @@ def _check(rc: int, what: str) -> None:
         raise HkError(rc, what, detail)
 
 
+_front_module = None
+
+
+def _front():
+    """The native front ends (csrc/torch_front.cpp): each returns None when the arguments are not plain CUDA tensors that
+    the call accepts as they are, and the checks below, in Python, have the word."""
+    global _front_module
+    if _front_module is None:
+        capi()  # the front ends link against the library: this names it if it is missing
+        _front_module = _load_ext("lib", "_torch_front")
+    return _front_module
+
+
+def _done(r, what: str):
+    """Result of a native front end: an int is the library's return code, anything else the outputs."""
+    if type(r) is int:
+        _check(r, what)
+        return None
+    return r
+
+
 def kernel_launch_count() -> int:
     return int(capi().hk_kernel_launch_count())
 
@@ -193,6 +214,10 @@ def attn_fwd(
     r + (kv_len_b - N): the mask is aligned to the last query and the last kept key as in base.py:104-116; a row
     that sees no key gets O = 0 and L = -inf.
     """
+    if stream is None:
+        r = _front().attn_fwd(q, k, v, bool(causal), softmax_scale, out, lse, kv_lens)
+        if r is not None:
+            return _done(r, "hk_attn_fwd")
     strided = not (q.is_contiguous() and k.is_contiguous() and v.is_contiguous())
     for name, t in (("q", q), ("k", k), ("v", v)):
         if strided:
@@ -339,6 +364,9 @@ def attn_bwd_strided(
     """The backward in one call: delta = rowsum(O * dO), then dQ, dK, dV written into the given tensors. q, k, v, dq,
     dk and dv may be strided views with a contiguous last dimension (slices of a packed projection and of its
     gradient); o and d_o [B,N,H,D] are contiguous. Asynchronous on torch's current stream."""
+    r = _front().attn_bwd_strided(q, k, v, o, d_o, lse, dq, dk, dv, bool(causal), softmax_scale, kv_lens)
+    if r is not None:
+        return _done(r, "hk_attn_bwd_strided")
     b, n, h, d = q.shape
     nk, hkv = k.shape[1], k.shape[2]
     for name, t, shape in (("q", q, (b, n, h, d)), ("k", k, (b, nk, hkv, d)), ("v", v, (b, nk, hkv, d)),
@@ -429,6 +457,10 @@ def rotary_bnhd(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out: Opti
                 pos_offset: int = 0, stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
     """Rotary embedding of x [B,N,H,D] bf16 (the attention entries' layout) with cos, sin [>= N + pos_offset, R/2]
     bf16; row n of the sequence uses table row n + pos_offset. `out` may be `x` itself."""
+    if stream is None:
+        r = _front().rotary_bnhd(x, cos, sin, out, pos_offset)
+        if r is not None:
+            return _done(r, "hk_rotary_bnhd")
     for name, t in (("x", x), ("cos", cos), ("sin", sin)):
         if not isinstance(t, torch.Tensor) or not t.is_contiguous() or t.device.type != "cuda" or t.dtype != torch.bfloat16:
             raise RuntimeError(f"{name} must be a contiguous bf16 CUDA tensor")
@@ -465,6 +497,10 @@ def paged_decode(
     """Paged-KV decode: q [S,1,H,D] bf16, pages [P,16,H_KV,D] bf16, block_table [S,max_pages] int32,
     ctx_lens [S] int32 -> O [S,1,H,D] bf16, L [S,H,1,1] fp32. `workspace` is a uint8 CUDA tensor of at
     least ``paged_decode_workspace_bytes(...)`` bytes (allocated here when omitted)."""
+    if stream is None:
+        r = _front().paged_decode(q, k_pages, v_pages, block_table, ctx_lens, softmax_scale, out, lse, workspace)
+        if r is not None:
+            return _done(r, "hk_attn_paged_decode")
     for name, t in (("q", q), ("k_pages", k_pages), ("v_pages", v_pages)):
         _require_cuda_bf16(name, t, 4)
         if t.dtype != torch.bfloat16:
@@ -517,6 +553,10 @@ def attn_fwd_paged(
     """Chunked prefill against the paged KV cache: q [S,T,H,D] bf16 (the last T tokens of each context when `causal`),
     pages [P,16,H_KV,D] bf16, block_table [S,max_pages] int32, ctx_lens [S] int32 -> O [S,T,H,D] bf16,
     L [S,H,1,T] fp32. The chunk's keys must already be in the cache (`paged_kv_append` first)."""
+    if stream is None:
+        r = _front().attn_fwd_paged(q, k_pages, v_pages, block_table, ctx_lens, bool(causal), softmax_scale, out, lse)
+        if r is not None:
+            return _done(r, "hk_attn_fwd_paged")
     for name, t in (("q", q), ("k_pages", k_pages), ("v_pages", v_pages)):
         _require_cuda_bf16(name, t, 4)
         if t.dtype != torch.bfloat16:
@@ -561,6 +601,10 @@ def paged_kv_append(
 ) -> None:
     """Write k_new/v_new [S,T,H_KV,D] into the page pools at positions start_pos[s] .. start_pos[s]+T-1 of each
     sequence (the paged form of the reference's `_update_kv_cache`, training/llama/llama/models/mha.py:16-42)."""
+    if stream is None:
+        r = _front().paged_kv_append(k_new, v_new, k_pages, v_pages, block_table, start_pos)
+        if r is not None:
+            return _done(r, "hk_paged_kv_append")
     for name, t in (("k_new", k_new), ("v_new", v_new), ("k_pages", k_pages), ("v_pages", v_pages)):
         _require_cuda_bf16(name, t, 4)
         if t.dtype != torch.bfloat16:
@@ -598,6 +642,10 @@ def paged_kv_append_rotary(
     """`paged_kv_append` with the rotary embedding of K applied on the way: token t of sequence s is rotated with row
     start_pos[s] + t of cos / sin [rows, R/2] bf16 (V is copied). The pages end up bit-identical to `rotary_bnhd`
     followed by `paged_kv_append` (the reference's order, mha.py:217-220 then 16-42)."""
+    if stream is None:
+        r = _front().paged_kv_append(k_new, v_new, k_pages, v_pages, block_table, start_pos, cos, sin)
+        if r is not None:
+            return _done(r, "hk_paged_kv_append_rotary")
     for name, t in (("k_new", k_new), ("v_new", v_new), ("k_pages", k_pages), ("v_pages", v_pages)):
         _require_cuda_bf16(name, t, 4)
         if t.dtype != torch.bfloat16:

@@ -32,6 +32,12 @@ def _tma_viewable(t: torch.Tensor) -> bool:
             and all(st > 0 and st % 8 == 0 for st in t.stride()[:3]))
 
 
+def _packed_viewable(t: torch.Tensor) -> bool:
+    """The same for the q, k, v slices of a packed projection [B, S, 2 or 3, H, D]."""
+    return (t.dtype == torch.bfloat16 and t.dim() == 5 and t.stride(4) == 1
+            and all(t.stride(i) > 0 and t.stride(i) % 8 == 0 for i in (0, 1, 3)))
+
+
 def _check_qkv(q, k, v):
     B, N, H, D = q.shape
     HKV, NK = k.shape[2], k.shape[1]
@@ -95,6 +101,7 @@ class _PackedAttnFunction(Function):
     @staticmethod
     def forward(ctx, q, packed, causal, softmax_scale, kv_lens):
         qkv = packed.unbind(dim=2) if q is None else (q, *packed.unbind(dim=2))
+        _check_qkv(*qkv)
         O, L = _forward(*qkv, causal, softmax_scale, kv_lens)
         ctx.save_for_backward(*([packed] if q is None else [q, packed]), O, L)
         ctx.causal = causal
@@ -113,19 +120,18 @@ class _PackedAttnFunction(Function):
 
 def _attend(q, packed, causal, softmax_scale, key_padding_mask):
     """Attention of q (None: the first of the packed tensors) over a packed projection [B, S, 2 or 3, H, D]."""
-    views = packed.unbind(dim=2) if q is None else (q, *packed.unbind(dim=2))
-    _check_qkv(*views)
     kv_lens = bad = None
     if key_padding_mask is not None:
         kv_lens, bad = _lens_from_key_padding_mask(key_padding_mask, packed)
-    if all(_tma_viewable(t) for t in views):
+    if _packed_viewable(packed) and (q is None or _tma_viewable(q)):
         out = _PackedAttnFunction.apply(q, packed, bool(causal), softmax_scale, kv_lens)
     else:
+        views = packed.unbind(dim=2) if q is None else (q, *packed.unbind(dim=2))
         out = HipAttnFunction.apply(*views, causal, softmax_scale, kv_lens)
     # read here, behind the forward's own synchronisation: whatever the mask, the lengths are clamped by the kernels
     if bad is not None and int(bad) != 0:
         raise ValueError(_BAD_MASK)
-    return out.to(views[0].dtype).contiguous()
+    return out.to((packed if q is None else q).dtype).contiguous()
 
 
 _BAD_MASK = "only right-padded key_padding_mask (a kept prefix of at least one key per row) is supported"
@@ -137,6 +143,7 @@ def _lens_from_key_padding_mask(mask: torch.Tensor, packed: torch.Tensor):
     cannot be expressed as lengths and is refused."""
     if mask.dim() != 2 or mask.shape[1] != packed.shape[1] or mask.dtype != torch.bool:
         raise ValueError("key_padding_mask must be a bool tensor (batch, seqlen), True = keep")
+    assert packed.is_cuda, "All tensors must be on CUDA device"
     if mask.device != packed.device:
         raise RuntimeError("key_padding_mask must be on the device of q, k and v")
     return key_padding_lens(mask)
