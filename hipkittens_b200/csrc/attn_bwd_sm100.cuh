@@ -81,7 +81,7 @@ struct BwdParams {
   FastDiv fd_group;     // causal: items of a full group
   FastDiv fd_in_grp, fd_in_grp_last;  // causal: items per key block / query tile in a full group, in the last group
   int n_pairs;          // causal dK/dV kernel: pairs of key blocks (j, NBK - 1 - j) over all units; 0: single blocks
-  FastDiv fd_pairs;     // pairs per unit, (NBK + 1) / 2
+  FastDiv fd_pairs;     // pairs per unit, (NBK + 1) / 2; single blocks: units
   float scale;
   float scale_log2;
   const int* kv_lens;   // optional device [B]: batch b attends to keys [0, kv_lens[b]) only; null = NK
@@ -350,12 +350,19 @@ struct DkdvItem {
 // N = 8192, and a unit has fewer blocks than the GPU has SMs, so no dealing of single blocks to CTAs balances. The
 // blocks are therefore dealt in pairs (j, NBK - 1 - j) of the same unit, which all cost the same: a CTA's round 2r
 // is the first block of its r-th pair and round 2r + 1 the second (none for the middle block of an odd count).
-// When there are no more blocks than SMs every block gets a CTA of its own instead (n_pairs = 0): the longest block
-// alone is then the kernel's time, not the longest plus the shortest (B2 N384 H8/2 D128, 12 blocks: 34.6 us for the
-// kernel in pairs, 25.1 us singly).
+// When the pairs would leave the last round badly filled (deal_dkdv), single blocks are dealt instead (n_pairs = 0),
+// the longest of all units first, in snake order. B2 N384 H8/2 D128, 12 blocks: 34.6 us in pairs, 25.1 us singly;
+// B4 N4096 H32/8 D128, 512 pairs = 3.46 rounds: 920 us in pairs, 859 us singly.
 template <bool CAUSAL>
 __device__ __forceinline__ int dkdv_item_for_round(const BwdParams& p, int round, int cta, int n_cta) {
-  if (!CAUSAL || p.n_pairs == 0) return item_for_round(p, round, cta, n_cta);
+  if (!CAUSAL) return item_for_round(p, round, cta, n_cta);
+  if (p.n_pairs == 0) {
+    const int k = round * n_cta + ((round & 1) ? n_cta - 1 - cta : cta);
+    if (k >= p.n_items) return -1;
+    int j, u;
+    p.fd_pairs.divmod(k, j, u);
+    return u * static_cast<int>(p.fd_unit.d) + j;
+  }
   const int pair = (round >> 1) * n_cta + cta;
   if (pair >= p.n_pairs) return -1;
   int unit, jp;

@@ -315,6 +315,33 @@ void set_bwd_decode(hk::BwdParams& p, int per_unit, int per_pos, int inner, int 
   p.fd_in_grp_last = hk::FastDiv((units - p.last_group * p.group_units) * per_pos);
 }
 
+// Deals the key blocks to CTAs (dkdv_item_for_round); returns the grid.
+template <bool CAUSAL>
+int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count) {
+  const int units = p.B * p.H_KV;
+  p.n_items = units * nbk;
+  int grid = p.n_items < sm_count ? p.n_items : sm_count;
+  set_bwd_decode(p, nbk, 1, 1, grid, false);
+  p.n_pairs = 0;
+  if (CAUSAL) {
+    // Pairs of blocks (j, nbk - 1 - j) all cost the same and keep few units in flight at a time (a unit's Q and dO are
+    // what its blocks share in L2); they are dealt when they fill their rounds to 95 %. Otherwise single blocks, the
+    // longest first, which even out to a few per cent whatever their number.
+    const int per_unit = (nbk + 1) / 2;
+    const long long pairs = 1ll * units * per_unit, rounds = (pairs + sm_count - 1) / sm_count;
+    if (pairs * 100 >= rounds * sm_count * 95) {
+      p.n_pairs = static_cast<int>(pairs);
+      p.fd_pairs = hk::FastDiv(per_unit);
+      grid = pairs < sm_count ? static_cast<int>(pairs) : sm_count;
+      p.total_rounds = 2 * static_cast<int>(rounds);
+    } else {
+      p.fd_pairs = hk::FastDiv(units);
+      p.total_rounds = (p.n_items + grid - 1) / grid;
+    }
+  }
+  return grid;
+}
+
 template <int D, bool CAUSAL>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                hk::BwdParams p, int B, int N, int NK, int H, int H_KV, int sm_count, cudaStream_t stream) {
@@ -322,22 +349,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   const int nbk = (NK + hk::kBlockN - 1) / hk::kBlockN;  // key blocks
   if (static_cast<long long>(B) * H * nbq > 0x3fffffffll || static_cast<long long>(B) * H_KV * nbk > 0x3fffffffll)
     return HK_EINVAL;  // work items are indexed with int
-  p.n_items = B * H_KV * nbk;
-  int grid = p.n_items < sm_count ? p.n_items : sm_count;
-  set_bwd_decode(p, nbk, 1, 1, grid, CAUSAL);
-  p.n_pairs = 0;
-  if (CAUSAL && p.n_items <= sm_count) {
-    p.group_items = p.n_items;
-    p.rounds_per_group = p.total_rounds = 1;
-    p.fd_rounds = hk::FastDiv(1);
-  } else if (CAUSAL) {
-    // key blocks are dealt in pairs (j, nbk - 1 - j) of equal cost, two rounds per pair
-    const int per_unit = (nbk + 1) / 2;
-    p.n_pairs = B * H_KV * per_unit;
-    p.fd_pairs = hk::FastDiv(per_unit);
-    grid = p.n_pairs < sm_count ? p.n_pairs : sm_count;
-    p.total_rounds = 2 * ((p.n_pairs + grid - 1) / grid);
-  }
+  int grid = deal_dkdv<CAUSAL>(p, nbk, sm_count);
 #ifdef HK_TRACE
   long long* const trace_buf = p.trace;
   p.trace = g_trace_bwd_kernel == 0 ? trace_buf : nullptr;
