@@ -136,6 +136,8 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
   const int sub = lane % kLanesPerRow;
   const int row0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * (kRowsPerWarp * kRowPassUnroll) + lane / kLanesPerRow;
   uint4 a[kRowPassUnroll], b[kRowPassUnroll];
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
 #pragma unroll
   for (int u = 0; u < kRowPassUnroll; ++u) {
     const int row = row0 + u * kRowsPerWarp;
@@ -181,6 +183,8 @@ __global__ void __launch_bounds__(256) attn_dq_shuffle_kernel(const uint4* __res
   const int vec = VEC ? VEC : vec_any;
   const long long idx0 = static_cast<long long>(blockIdx.x) * (256 * kRowPassUnroll) + threadIdx.x;
   uint4 val[kRowPassUnroll];
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
 #pragma unroll
   for (int u = 0; u < kRowPassUnroll; ++u) {
     const long long idx = idx0 + u * 256;  // enumerates the destination [B,N,H,vec]
@@ -418,7 +422,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int warp = tid >> 5;
   const int lane = tid & 31;
 
-  if ((smem_u32(bwd_smem) & 1023u) != 0) {  // uniform over the CTA; nothing has been allocated yet
+  if ((smem_u32(bwd_smem) & 1023u) != 0) {
+    grid_dep_wait();  // uniform over the CTA; nothing has been allocated yet
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusSmemAlign);
     return;
   }
@@ -457,6 +462,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   volatile uint32_t* abortp = abort_word;
+  grid_dep_wait();
+  grid_dep_launch();
   const int G = p.G;
   // TMEM columns: X [0,128) takes the two score-shaped products in turn, S^T(n) then dP^T(n), each free again as soon
   // as the element-wise warps hold it in registers; Y [128,256) holds the two bf16 operands, P^T in [128,192) and dS^T
@@ -965,6 +972,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   const int lane = tid & 31;
 
   if ((smem_u32(bwd_smem) & 1023u) != 0) {
+    grid_dep_wait();
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusSmemAlign);
     return;
   }
@@ -998,6 +1006,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   volatile uint32_t* abortp = abort_word;
+  grid_dep_wait();
+  grid_dep_launch();
   // TMEM columns: S [0,128)  dP [128,256)  dQ [256,256+D)  dS (bf16, 64 packed columns) [384,448).
   // Nothing aliases: S and dP are free for the next tile as soon as they are in registers.
   constexpr uint32_t cS = 0, cDP = 128, cDQ = 256, cDS = 384;

@@ -355,6 +355,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_after();
   const uint32_t tmem = tmem_base_slot;
   volatile uint32_t* abortp = &abort_flag;
+  grid_dep_wait();
+  grid_dep_launch();
 
   if (warp < 8) {
     // ------------------------------------------------------------------ softmax warpgroups

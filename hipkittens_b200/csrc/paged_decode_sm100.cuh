@@ -114,6 +114,8 @@ template <int G>
 __global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(const DecodeParams p) {
   using namespace dec;
   extern __shared__ __align__(128) uint8_t dsmem[];
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   const int split = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z;
   // A length beyond what the block-table row can address is clamped to the row's capacity and reported; nothing
   // past the row is read.
@@ -306,16 +308,13 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(c
       }
     }
   }
-  // programmatic dependent launch: this CTA's results are written, the combine grid may be set up
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // grid = (H, S), block = 128 threads (one per output column). Merges the per-chunk partials of
 // sequences that span more than one chunk.
 __global__ void __launch_bounds__(kDecodeD) paged_decode_combine_kernel(const DecodeParams p) {
-  // launched with programmatic stream serialization: wait here until the split grid has completed and its
-  // partials are visible (a no-op under an ordinary launch)
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();  // the split grid has completed and its partials are visible
   const int head = blockIdx.x, seq = blockIdx.y;
   const int ctx = min(p.ctx_lens[seq], p.max_pages * kPageTokens);  // clamped as in the split kernel, which reports it
   const int d = threadIdx.x;
@@ -360,6 +359,24 @@ __global__ void __launch_bounds__(kDecodeD) paged_decode_combine_kernel(const De
   if (d == 0) p.lse[size_t(seq) * p.H + head] = s_M * p.scale + __logf(s_L);
 }
 
+// Launch with programmatic stream serialization (see ptx::grid_dep_wait, which every kernel launched so executes), or, with
+// `early` false, an ordinary launch.
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                             cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 inline int prepare_decode_kernels(char* err, size_t err_len) {
   cudaError_t e;
 #define HK_PREP(G)                                                                                      \
@@ -380,29 +397,17 @@ inline cudaError_t launch_paged_decode(DecodeParams p, int sm_count, cudaStream_
   if (splits > kMaxCombineSplits) return cudaErrorInvalidValue;
   const dim3 grid(splits, p.H_KV, p.S);
   const int G = p.H / p.H_KV;
+  cudaError_t e;
   switch (G) {
 #define HK_CASE(g) \
-  case g: paged_decode_split_kernel<g><<<grid, kDecodeThreads, kDecodeSmemBytes, stream>>>(p); break;
+  case g: e = launch_dependent(true, paged_decode_split_kernel<g>, grid, kDecodeThreads, kDecodeSmemBytes, stream, p); break;
     HK_CASE(1) HK_CASE(2) HK_CASE(3) HK_CASE(4) HK_CASE(5) HK_CASE(6) HK_CASE(7) HK_CASE(8)
 #undef HK_CASE
     default: return cudaErrorInvalidValue;
   }
   *launched += 1;
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  // The combine grid is launched with programmatic stream serialization, so that its launch overlaps the tail
-  // of the split grid; it blocks in griddepcontrol.wait until the split grid is complete.
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.H, p.S);
-  cfg.blockDim = dim3(kDecodeD);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, paged_decode_combine_kernel, p);
+  e = launch_dependent(true, paged_decode_combine_kernel, dim3(p.H, p.S), kDecodeD, 0, stream, p);
   *launched += 1;
   return e;
 }

@@ -34,6 +34,8 @@ struct AppendParams {
 constexpr int kAppendUnroll = 4;
 
 __global__ void __launch_bounds__(128) paged_kv_append_kernel(const AppendParams p) {
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   const long long total = static_cast<long long>(p.S) * p.T;
   for (long long base = static_cast<long long>(blockIdx.x) * kAppendUnroll; base < total;
        base += static_cast<long long>(gridDim.x) * kAppendUnroll) {
@@ -90,6 +92,8 @@ struct AppendRotaryParams {
 
 __global__ void __launch_bounds__(128) paged_kv_append_rotary_kernel(const AppendRotaryParams q) {
   const AppendParams& p = q.a;
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   const long long total = static_cast<long long>(p.S) * p.T;
   const int half = q.R / 2;
   const int pair_units = q.R / 16;                      // 8 rotated pairs each

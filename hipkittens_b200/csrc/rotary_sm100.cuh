@@ -21,6 +21,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sm100_ptx.cuh"
+
 namespace hk {
 
 struct RotaryParams {
@@ -54,6 +56,8 @@ __device__ __forceinline__ uint32_t rot_hi(uint32_t x1, uint32_t x2, uint32_t c,
 // Work unit = 8 rotated pairs (or 8 pass-through elements) of one row: `units_per_row` = R/16 pair units followed by
 // (D - R)/8 copy units. grid = ceil(rows * units_per_row / 256), block = 256.
 __global__ void __launch_bounds__(256) rotary_kernel(const RotaryParams p) {
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   const int pair_units = p.R / 16;
   const int units_per_row = pair_units + (p.D - p.R) / 8;
   const long long gid = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;

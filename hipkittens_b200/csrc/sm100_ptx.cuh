@@ -36,6 +36,18 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// ---------------------------------------------------------------- dependent launch
+// Kernels are launched with programmatic stream serialization: their CTAs may start while the kernel before them in the
+// stream is finishing, and run their prologue (barriers, TMEM, descriptor prefetch) under its tail. grid_dep_wait() is
+// every thread's first step before it touches global memory: it returns when the kernels before have completed and their
+// writes are visible. It also makes completion transitive (a kernel only completes after the one before it), so no
+// CTA may leave without it. grid_dep_launch() lets the next kernel do the same, once every CTA of this one has got there.
+// What it is worth (us per pass in a loop, before -> after): B1 N256 D64 forward
+// 8.3 -> 7.0, rotary twice and attention of a 1511-token prompt 43.2 -> 38.3, one-token append and decode 16.4 -> 12.2;
+// nothing beyond 0.3 ms, where attention kernels are launched the ordinary way (see launch_dependent).
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -1,0 +1,75 @@
+"""Kernels are launched so that they may start under the tail of the one before them. A chain of calls that hand their
+buffers on and overwrite them must give what the same calls give with a synchronisation after each."""
+import pytest
+import torch
+
+import hipkittens_b200 as hk
+from hipkittens_b200 import _native
+
+pytestmark = pytest.mark.gpu
+
+
+def _chain(n, d, steps, sync):
+    gen = torch.Generator("cuda").manual_seed(11)
+
+    def rand(*shape):
+        return torch.randn(shape, device="cuda", generator=gen).to(torch.bfloat16)
+
+    def call(fn, *args, **kwargs):
+        r = fn(*args, **kwargs)
+        if sync:
+            torch.cuda.synchronize()
+        return r
+
+    q, k, v, d_o = rand(2, n, 4, d), rand(2, n, 2, d), rand(2, n, 2, d), rand(2, n, 4, d)
+    angle = torch.rand(n, d // 2, device="cuda", generator=gen)
+    cos, sin = angle.cos().to(torch.bfloat16), angle.sin().to(torch.bfloat16)
+    kr, outs = torch.empty_like(k), [torch.empty_like(q), torch.empty_like(q)]
+    lse = torch.empty(2, 4, 1, n, device="cuda")
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    pools = [torch.zeros(2 * n, 16, 2, 128, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    table = torch.arange(2 * n, device="cuda", dtype=torch.int32).reshape(2, n)
+    tokens, q1 = rand(2, 1, 2, 128), rand(2, 1, 8, 128)
+    seen = []
+    for i in range(steps):
+        # every call reads what the one before it wrote, and overwrites what earlier ones read
+        out, vi = outs[i % 2], v if i == 0 else outs[(i + 1) % 2][:, :, :2]
+        call(hk.rotary_bnhd, k if i == 0 else kr, cos, sin, out=kr)
+        call(hk.attn_fwd, q, kr, vi, causal=True, out=out, lse=lse)
+        call(_native.attn_bwd_strided, q, kr, vi, out, d_o, lse, dq, dk, dv, causal=True)
+        if d == 128:
+            start = torch.full((2,), i, dtype=torch.int32, device="cuda")
+            call(hk.paged_kv_append, tokens, tokens, *pools, table, start)
+            o1, _ = call(hk.paged_decode, q1, *pools, table, start + 1)
+            tokens = o1[:, :, :2].contiguous()
+            seen.append(o1)
+    return [*outs, lse, dq, dk, dv, kr, *pools, *seen]
+
+
+@pytest.mark.parametrize("n,d", [(64, 64), (200, 128), (1000, 128)])
+def test_back_to_back_calls_equal_synchronised_ones(n, d):
+    for a, b in zip(_chain(n, d, 12, False), _chain(n, d, 12, True)):
+        assert torch.equal(a, b)
+
+
+def test_captured_chain_replays():
+    """The dependent launches survive capture into a CUDA graph."""
+    q, kv = torch.randn(2, 1, 300, 4, 64, device="cuda").to(torch.bfloat16)
+    cos, sin = (torch.randn(300, 32, device="cuda").to(torch.bfloat16) for _ in range(2))
+    rot, out, lse = torch.empty_like(q), torch.empty_like(q), torch.empty(1, 4, 1, 300, device="cuda")
+
+    def calls():
+        hk.rotary_bnhd(q, cos, sin, out=rot)
+        hk.attn_fwd(rot, kv, kv, causal=True, out=out, lse=lse)
+
+    calls()
+    torch.cuda.synchronize()
+    expected = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        calls()
+    out.zero_()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, expected)
