@@ -31,6 +31,7 @@ thread_local char g_cuda_err[256] = "";
 std::atomic<unsigned long long> g_launches{0};
 
 int cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here, and not once more by the caller's next check
   snprintf(g_cuda_err, sizeof(g_cuda_err), "%s: %s", what, cudaGetErrorString(e));
   return HK_ECUDA;
 }
