@@ -20,11 +20,12 @@ namespace {
 
 using at::Tensor;
 
-// A plain strided CUDA tensor, or null (also for None: `none` tells).
+// A plain strided CUDA tensor, or null. The wrappers of torch.func's transforms are of the exact class too, but have no
+// storage, and so no pointer to read.
 const Tensor* plain(PyObject* o) {
   if (!THPVariable_CheckExact(o)) return nullptr;
   const Tensor& t = THPVariable_Unpack(o);
-  return t.defined() && t.is_cuda() && t.layout() == at::kStrided ? &t : nullptr;
+  return t.defined() && t.is_cuda() && t.layout() == at::kStrided && t.has_storage() ? &t : nullptr;
 }
 bool is(const Tensor* t, at::ScalarType type, int64_t dim) { return t && t->scalar_type() == type && t->dim() == dim; }
 bool dense(const Tensor* t, at::ScalarType type, int64_t dim) { return is(t, type, dim) && t->is_contiguous(); }
@@ -37,7 +38,7 @@ bool same_device(const Tensor& ref, std::initializer_list<const Tensor*> ts) {
 bool output(PyObject* o, const Tensor& ref, at::IntArrayRef shape, at::ScalarType type, Tensor& out) {
   if (o == Py_None) {
     out = at::empty(shape, ref.options().dtype(type).requires_grad(false));
-    return true;
+    return out.has_storage();  // under a transform a new tensor is a wrapper as well
   }
   const Tensor* t = plain(o);
   if (!dense(t, type, int64_t(shape.size())) || t->sizes() != shape || t->device() != ref.device()) return false;
@@ -61,8 +62,15 @@ bool number(PyObject* o, float& v) {
   return true;
 }
 
+// The device pointer of a tensor. data_ptr() can throw and must not race with a resize_ or set_ of another thread, so it
+// is read while the interpreter lock is held.
+template <typename T = void>
+T* ptr(const Tensor& t) { return static_cast<T*>(t.data_ptr()); }
+
+// The library call without the interpreter lock, as ctypes makes it. `call` must not throw: it holds pointers and numbers
+// that were read before, and touches no tensor.
 template <typename Call>
-int unlocked(Call&& call) {  // the library call without the interpreter lock, as ctypes makes it
+int unlocked(const Call& call) {
   int rc;
   Py_BEGIN_ALLOW_THREADS rc = call();
   Py_END_ALLOW_THREADS return rc;
@@ -107,14 +115,15 @@ PyObject* attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     Py_RETURN_NONE;
   void* st = stream_of(*q);
   const int causal = a[3] == Py_True, dev = q->device().index();
+  const void *qp = ptr(*q), *kp = ptr(*k), *vp = ptr(*v);
+  void* outp = ptr(out);
+  float* lsep = ptr<float>(lse);
+  const int32_t* lensp = lens ? ptr<int32_t>(*lens) : nullptr;
   const int rc = unlocked([&] {
     if (lens || nk != n || strided)
-      return hk_attn_fwd_cross(q->data_ptr(), k->data_ptr(), v->data_ptr(), out.data_ptr(),
-                               static_cast<float*>(lse.data_ptr()), i32(b), i32(n), i32(nk), i32(h), i32(hkv), i32(d),
-                               qs, ks, vs, lens ? static_cast<const int32_t*>(lens->data_ptr()) : nullptr, causal, scale,
-                               dev, st);
-    return hk_attn_fwd(q->data_ptr(), k->data_ptr(), v->data_ptr(), out.data_ptr(), static_cast<float*>(lse.data_ptr()),
-                       i32(b), i32(n), i32(h), i32(hkv), i32(d), causal, scale, dev, st);
+      return hk_attn_fwd_cross(qp, kp, vp, outp, lsep, i32(b), i32(n), i32(nk), i32(h), i32(hkv), i32(d), qs, ks, vs, lensp,
+                               causal, scale, dev, st);
+    return hk_attn_fwd(qp, kp, vp, outp, lsep, i32(b), i32(n), i32(h), i32(hkv), i32(d), causal, scale, dev, st);
   });
   return result(rc, out, lse);
   END_HANDLE_TH_ERRORS
@@ -148,15 +157,18 @@ PyObject* attn_bwd_strided(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!is(lens, at::kInt, 1) || lens->size(0) != b || lens->device() != q->device()) Py_RETURN_NONE;
   }
   const Tensor delta = at::empty({b, h, 1, n}, lse->options().requires_grad(false));
+  if (!delta.has_storage()) Py_RETURN_NONE;
   void* stream = stream_of(*q);
-  const int causal = a[9] == Py_True;
+  const int causal = a[9] == Py_True, dev = q->device().index();
+  const void *qp = ptr(*q), *kp = ptr(*k), *vp = ptr(*v), *op = ptr(*o), *dop = ptr(*d_o);
+  const float* lsep = ptr<float>(*lse);
+  float* deltap = ptr<float>(delta);
+  void *dqp = ptr(*dq), *dkp = ptr(*dk), *dvp = ptr(*dv);
+  const int32_t* lensp = lens ? ptr<int32_t>(*lens) : nullptr;
   const int rc = unlocked([&] {
-    return hk_attn_bwd_strided(q->data_ptr(), k->data_ptr(), v->data_ptr(), o->data_ptr(), d_o->data_ptr(),
-                               static_cast<const float*>(lse->data_ptr()), static_cast<float*>(delta.data_ptr()),
-                               dq->data_ptr(), dk->data_ptr(), dv->data_ptr(), i32(b), i32(n), i32(nk), i32(h), i32(hkv),
-                               i32(d), st[0], st[1], st[2], st[3], st[4], st[5],
-                               lens ? static_cast<const int32_t*>(lens->data_ptr()) : nullptr, causal, scale,
-                               q->device().index(), stream);
+    return hk_attn_bwd_strided(qp, kp, vp, op, dop, lsep, deltap, dqp, dkp, dvp, i32(b), i32(n), i32(nk), i32(h),
+                               i32(hkv), i32(d), st[0], st[1], st[2], st[3], st[4], st[5], lensp, causal, scale, dev,
+                               stream);
   });
   return PyLong_FromLong(rc);
   END_HANDLE_TH_ERRORS
@@ -178,11 +190,11 @@ PyObject* rotary_bnhd(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   Tensor out;
   if (!output(a[3], *x, x->sizes(), at::kBFloat16, out)) Py_RETURN_NONE;
   void* st = stream_of(*x);
-  const int rc = unlocked([&] {
-    return hk_rotary_bnhd(x->data_ptr(), out.data_ptr(), sin->data_ptr(), cos->data_ptr(), i32(x->size(0)),
-                          i32(x->size(1)), i32(x->size(2)), i32(x->size(3)), i32(2 * cos->size(1)), i32(pos),
-                          x->device().index(), st);
-  });
+  const int b = i32(x->size(0)), n = i32(x->size(1)), h = i32(x->size(2)), d = i32(x->size(3)), r = i32(2 * cos->size(1));
+  const int dev = x->device().index();
+  const void *xp = ptr(*x), *sinp = ptr(*sin), *cosp = ptr(*cos);
+  void* outp = ptr(out);
+  const int rc = unlocked([&] { return hk_rotary_bnhd(xp, outp, sinp, cosp, b, n, h, d, r, i32(pos), dev, st); });
   if (rc != HK_OK) return PyLong_FromLong(rc);
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
@@ -192,6 +204,15 @@ PyObject* rotary_bnhd(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 struct Paged {
   const Tensor *q, *kp, *vp, *table, *lens;
   int64_t s, t, h, d, pool, page, hkv, max_pages;
+  void *q_ptr, *k_pages, *v_pages;
+  const int32_t *table_ptr, *lens_ptr;
+  int device;
+  // What the library call needs of the tensors, read before the interpreter lock is given up.
+  void read() {
+    q_ptr = ptr(*q), k_pages = ptr(*kp), v_pages = ptr(*vp);
+    table_ptr = ptr<int32_t>(*table), lens_ptr = ptr<int32_t>(*lens);
+    device = q->device().index();
+  }
   bool take(PyObject* const* a) {
     q = plain(a[0]), kp = plain(a[1]), vp = plain(a[2]), table = plain(a[3]), lens = plain(a[4]);
     if (!dense(q, at::kBFloat16, 4) || !dense(kp, at::kBFloat16, 4) || !dense(vp, at::kBFloat16, 4) ||
@@ -217,19 +238,21 @@ PyObject* paged_decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     Py_RETURN_NONE;
   if (a[8] == Py_None) {
     ws = at::empty({int64_t(need < 256 ? 256 : need)}, p.q->options().dtype(at::kByte).requires_grad(false));
+    if (!ws.has_storage()) Py_RETURN_NONE;
   } else {
     const Tensor* t = plain(a[8]);
     if (!dense(t, at::kByte, 1) || t->device() != p.q->device()) Py_RETURN_NONE;
     ws = *t;
   }
   void* st = stream_of(*p.q);
+  p.read();
+  void *outp = ptr(out), *wsp = ptr(ws);
+  float* lsep = ptr<float>(lse);
+  const size_t ws_bytes = size_t(ws.numel());
   const int rc = unlocked([&] {
-    return hk_attn_paged_decode(p.q->data_ptr(), p.kp->data_ptr(), p.vp->data_ptr(),
-                                static_cast<const int32_t*>(p.table->data_ptr()),
-                                static_cast<const int32_t*>(p.lens->data_ptr()), out.data_ptr(),
-                                static_cast<float*>(lse.data_ptr()), i32(p.s), i32(p.h), i32(p.hkv), i32(p.d), i32(p.page),
-                                i32(p.max_pages), i32(p.pool), scale, ws.data_ptr(), size_t(ws.numel()),
-                                p.q->device().index(), st);
+    return hk_attn_paged_decode(p.q_ptr, p.k_pages, p.v_pages, p.table_ptr, p.lens_ptr, outp, lsep, i32(p.s), i32(p.h),
+                                i32(p.hkv), i32(p.d), i32(p.page), i32(p.max_pages), i32(p.pool), scale, wsp, ws_bytes,
+                                p.device, st);
   });
   return result(rc, out, lse);
   END_HANDLE_TH_ERRORS
@@ -246,12 +269,14 @@ PyObject* attn_fwd_paged(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
       !output(a[8], *p.q, {p.s, p.h, 1, p.t}, at::kFloat, lse))
     Py_RETURN_NONE;
   void* st = stream_of(*p.q);
+  p.read();
+  const int causal = a[5] == Py_True;
+  void* outp = ptr(out);
+  float* lsep = ptr<float>(lse);
   const int rc = unlocked([&] {
-    return hk_attn_fwd_paged(p.q->data_ptr(), p.kp->data_ptr(), p.vp->data_ptr(),
-                             static_cast<const int32_t*>(p.table->data_ptr()),
-                             static_cast<const int32_t*>(p.lens->data_ptr()), out.data_ptr(),
-                             static_cast<float*>(lse.data_ptr()), i32(p.s), i32(p.t), i32(p.h), i32(p.hkv), i32(p.d),
-                             i32(p.page), i32(p.max_pages), i32(p.pool), a[5] == Py_True, scale, p.q->device().index(), st);
+    return hk_attn_fwd_paged(p.q_ptr, p.k_pages, p.v_pages, p.table_ptr, p.lens_ptr, outp, lsep, i32(p.s), i32(p.t),
+                             i32(p.h), i32(p.hkv), i32(p.d), i32(p.page), i32(p.max_pages), i32(p.pool), causal, scale,
+                             p.device, st);
   });
   return result(rc, out, lse);
   END_HANDLE_TH_ERRORS
@@ -275,17 +300,16 @@ PyObject* paged_kv_append(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
       Py_RETURN_NONE;
   }
   void* st = stream_of(*p.q);
-  const auto* table = static_cast<const int32_t*>(p.table->data_ptr());
-  const auto* start = static_cast<const int32_t*>(p.lens->data_ptr());
-  const int dev = p.q->device().index();
+  p.read();
+  const void *vp = ptr(*v_new), *cosp = cos ? ptr(*cos) : nullptr, *sinp = cos ? ptr(*sin) : nullptr;
+  const int rows = cos ? i32(cos->size(0)) : 0, rotary_dim = cos ? i32(2 * cos->size(1)) : 0;
   const int rc = unlocked([&] {
-    if (cos)
-      return hk_paged_kv_append_rotary(p.q->data_ptr(), v_new->data_ptr(), p.kp->data_ptr(), p.vp->data_ptr(), table,
-                                       start, sin->data_ptr(), cos->data_ptr(), i32(p.s), i32(p.t), i32(p.h), i32(p.d),
-                                       i32(2 * cos->size(1)), i32(cos->size(0)), i32(p.page), i32(p.max_pages),
-                                       i32(p.pool), dev, st);
-    return hk_paged_kv_append(p.q->data_ptr(), v_new->data_ptr(), p.kp->data_ptr(), p.vp->data_ptr(), table, start,
-                              i32(p.s), i32(p.t), i32(p.h), i32(p.d), i32(p.page), i32(p.max_pages), i32(p.pool), dev, st);
+    if (n_args == 8)
+      return hk_paged_kv_append_rotary(p.q_ptr, vp, p.k_pages, p.v_pages, p.table_ptr, p.lens_ptr, sinp, cosp, i32(p.s),
+                                       i32(p.t), i32(p.h), i32(p.d), rotary_dim, rows, i32(p.page), i32(p.max_pages),
+                                       i32(p.pool), p.device, st);
+    return hk_paged_kv_append(p.q_ptr, vp, p.k_pages, p.v_pages, p.table_ptr, p.lens_ptr, i32(p.s), i32(p.t), i32(p.h),
+                              i32(p.d), i32(p.page), i32(p.max_pages), i32(p.pool), p.device, st);
   });
   return PyLong_FromLong(rc);
   END_HANDLE_TH_ERRORS
