@@ -193,6 +193,19 @@ def _require_same_device(ref: torch.Tensor, **tensors) -> None:
                                f"{t.device if isinstance(t, torch.Tensor) else type(t).__name__})")
 
 
+def _dense_lens(kv_lens: Optional[torch.Tensor], b: int, device: torch.device, stream) -> Optional[torch.Tensor]:
+    """Key lengths as the kernels index them, one int32 after the other: a view with other strides (every second length, one
+    length expanded to all) is copied on the stream that reads it."""
+    if kv_lens is None:
+        return None
+    if kv_lens.dtype != torch.int32 or kv_lens.shape != (b,) or kv_lens.device != device:
+        raise RuntimeError("kv_lens must be an int32 tensor [B] on q's device")
+    if not kv_lens.is_contiguous():
+        with torch.cuda.stream(stream):
+            kv_lens = kv_lens.contiguous()
+    return kv_lens
+
+
 def attn_fwd(
     q: torch.Tensor,
     k: torch.Tensor,
@@ -246,8 +259,7 @@ def attn_fwd(
     _require_same_device(q, k=k, v=v, out=out, lse=lse)
     s = stream if stream is not None else torch.cuda.current_stream(q.device)
     if kv_lens is not None or nk != n:
-        if kv_lens is not None and (kv_lens.dtype != torch.int32 or kv_lens.shape != (b,) or kv_lens.device != q.device):
-            raise RuntimeError("kv_lens must be an int32 tensor [B] on q's device")
+        kv_lens = _dense_lens(kv_lens, b, q.device, s)
         arr = lambda t: (ctypes.c_longlong * 3)(*t.stride()[:3])  # noqa: E731
         rc = capi().hk_attn_fwd_cross(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
                                       b, n, nk, h, hkv, d, arr(q), arr(k), arr(v),
@@ -336,8 +348,7 @@ def attn_bwd(
             raise RuntimeError(f"{name} must be a contiguous bf16 tensor of shape {tuple(shp)}")
     _require_same_device(q, k=k, v=v, d_o=d_o, dq=dq, dk=dk, dv=dv)
     s = stream if stream is not None else torch.cuda.current_stream(q.device)
-    if kv_lens is not None and (kv_lens.dtype != torch.int32 or kv_lens.shape != (b,) or kv_lens.device != q.device):
-        raise RuntimeError("kv_lens must be an int32 tensor [B] on q's device")
+    kv_lens = _dense_lens(kv_lens, b, q.device, s)
     rc = capi().hk_attn_bwd_cross(q.data_ptr(), k.data_ptr(), v.data_ptr(), d_o.data_ptr(), lse.data_ptr(),
                                   delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), b, n, nk, h, hkv, d,
                                   kv_lens.data_ptr() if kv_lens is not None else None,
@@ -380,9 +391,8 @@ def attn_bwd_strided(
         raise RuntimeError("Tensor must be contiguous")
     if lse.shape != (b, h, 1, n) or lse.dtype != torch.float32 or not lse.is_contiguous() or lse.device != q.device:
         raise RuntimeError("lse must be a contiguous fp32 tensor [B, H, 1, N] on q's device")
-    if kv_lens is not None and (kv_lens.dtype != torch.int32 or kv_lens.shape != (b,) or kv_lens.device != q.device):
-        raise RuntimeError("kv_lens must be an int32 tensor [B] on q's device")
     s = torch.cuda.current_stream(q.device)
+    kv_lens = _dense_lens(kv_lens, b, q.device, s)
     delta = torch.empty_like(lse)
 
     def arr(t):  # a dimension of size 1 has no stride that matters: give it one the library takes

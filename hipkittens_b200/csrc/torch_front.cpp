@@ -108,7 +108,7 @@ PyObject* attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const Tensor* lens = nullptr;
   if (a[7] != Py_None) {
     lens = plain(a[7]);
-    if (!is(lens, at::kInt, 1) || lens->size(0) != b || lens->device() != q->device()) Py_RETURN_NONE;
+    if (!dense(lens, at::kInt, 1) || lens->size(0) != b || lens->device() != q->device()) Py_RETURN_NONE;
   }
   Tensor out, lse;
   if (!output(a[5], *q, q->sizes(), at::kBFloat16, out) || !output(a[6], *q, {b, h, 1, n}, at::kFloat, lse))
@@ -154,7 +154,7 @@ PyObject* attn_bwd_strided(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const Tensor* lens = nullptr;
   if (a[11] != Py_None) {
     lens = plain(a[11]);
-    if (!is(lens, at::kInt, 1) || lens->size(0) != b || lens->device() != q->device()) Py_RETURN_NONE;
+    if (!dense(lens, at::kInt, 1) || lens->size(0) != b || lens->device() != q->device()) Py_RETURN_NONE;
   }
   const Tensor delta = at::empty({b, h, 1, n}, lse->options().requires_grad(false));
   if (!delta.has_storage()) Py_RETURN_NONE;
