@@ -126,9 +126,9 @@ constexpr int kRowPassUnroll = 4;
 __host__ __device__ constexpr int row_pass_rows(int lanes_per_row) { return 8 * (32 / lanes_per_row) * kRowPassUnroll; }
 
 template <int D>
-__global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o,
-                                                            const __nv_bfloat16* __restrict__ d_o,
-                                                            float* __restrict__ delta, int rows, int N, int H,
+__global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* o,
+                                                            const __nv_bfloat16* d_o,
+                                                            float* delta, int rows, int N, int H,
                                                             FastDiv fd_h, FastDiv fd_n) {
   constexpr int kLanesPerRow = D / 8;               // 16 or 8
   constexpr int kRowsPerWarp = 32 / kLanesPerRow;   // 2 or 4
@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
     const int row = row0 + u * kRowsPerWarp;
     a[u] = b[u] = make_uint4(0, 0, 0, 0);
     if (row < rows) {
-      a[u] = __ldg(reinterpret_cast<const uint4*>(o + static_cast<size_t>(row) * D) + sub);
-      b[u] = __ldg(reinterpret_cast<const uint4*>(d_o + static_cast<size_t>(row) * D) + sub);
+      a[u] = reinterpret_cast<const uint4*>(o + static_cast<size_t>(row) * D)[sub];
+      b[u] = reinterpret_cast<const uint4*>(d_o + static_cast<size_t>(row) * D)[sub];
     }
   }
 #pragma unroll
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
 // 164 us now). VEC: units per row (16 or 8; 0 = any, `vec` says how many).
 // grid = ceil(rows * vec / (256 * kRowPassUnroll)), block = 256.
 template <int VEC>
-__global__ void __launch_bounds__(256) attn_dq_shuffle_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst,
+__global__ void __launch_bounds__(256) attn_dq_shuffle_kernel(const uint4* src, uint4* dst,
                                                               long long total, int N, int H, int vec_any, FastDiv fd_h,
                                                               FastDiv fd_n) {
   const int vec = VEC ? VEC : vec_any;
@@ -194,10 +194,10 @@ __global__ void __launch_bounds__(256) attn_dq_shuffle_kernel(const uint4* __res
         int bn, h, b, n;
         fd_h.divmod(row, bn, h);
         fd_n.divmod(bn, b, n);
-        val[u] = __ldg(src + ((static_cast<size_t>(b) * H + h) * N + n) * VEC + v);
+        val[u] = src[((static_cast<size_t>(b) * H + h) * N + n) * VEC + v];
       } else {
         const long long row = idx / vec, bn = row / H, h = row - bn * H, b = bn / N, n = bn - b * N;
-        val[u] = __ldg(src + ((b * H + h) * N + n) * vec + (idx - row * vec));
+        val[u] = src[((b * H + h) * N + n) * vec + (idx - row * vec)];
       }
     }
   }
@@ -856,8 +856,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           const int pos = i * kBlockM + t * 32 + lane;
           const bool in = pos < p.N;
           // stored ready for use: -L * log2(e) is the addend of the exponent, -delta the addend of dP
-          lv[t] = in ? __ldg(p.lse + base + pos) * -1.4426950408889634f : 0.f;
-          dv_[t] = in ? -__ldg(p.delta + base + pos) : 0.f;
+          lv[t] = in ? p.lse[base + pos] * -1.4426950408889634f : 0.f;
+          dv_[t] = in ? -p.delta[base + pos] : 0.f;
         }
       };
       for (int round = 0; ok; ++round) {

@@ -795,8 +795,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             // repeat its last page, so that every row of the tile holds cache contents (those keys are masked; their
             // V rows meet p = 0). An id outside the pool is reported and replaced, never dereferenced.
             const int total_pages = (kv_len + 15) >> 4;
-            int id = __ldg(p.block_table + static_cast<size_t>(b) * p.max_pages +
-                           min(tile * (kBlockN / 16) + lane, total_pages - 1));
+            int id = p.block_table[static_cast<size_t>(b) * p.max_pages +
+                                   min(tile * (kBlockN / 16) + lane, total_pages - 1)];
             if (id < 0 || id >= p.num_pages) {
               atomicCAS(p.status, kStatusOk, kStatusFwdBadPage);
               id = 0;

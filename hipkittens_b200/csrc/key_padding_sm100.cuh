@@ -10,8 +10,7 @@ namespace hk {
 // grid = B, block = 256. lens[b] = number of kept keys of row b; *bad (zero on entry) is raised by a row that does not
 // keep a prefix, or keeps nothing. One launch in place of the sum / compare / reduce chain of nine that tensor
 // operations need for it; a row is N bytes, so this is launch latency (about 3 us) and nothing else.
-__global__ void __launch_bounds__(256) key_padding_lens_kernel(const unsigned char* __restrict__ mask,
-                                                               int32_t* __restrict__ lens, int32_t* __restrict__ bad,
+__global__ void __launch_bounds__(256) key_padding_lens_kernel(const unsigned char* mask, int32_t* lens, int32_t* bad,
                                                                int N) {
   const unsigned char* row = mask + static_cast<size_t>(blockIdx.x) * N;
   int kept = 0, end = 0;  // kept keys, and one past the last of them

@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kDecodeD) paged_decode_combine_kernel(const De
   __syncthreads();
   float acc = 0.f;
 #pragma unroll 4
-  for (int i = 0; i < n_splits; ++i) acc += s_w[i] * __ldg(ws_o + (slot0 + i) * kDecodeD + d);
+  for (int i = 0; i < n_splits; ++i) acc += s_w[i] * ws_o[(slot0 + i) * kDecodeD + d];
   p.o[(size_t(seq) * p.H + head) * kDecodeD + d] = __float2bfloat16(acc / s_L);
   if (d == 0) p.lse[size_t(seq) * p.H + head] = s_M * p.scale + __logf(s_L);
 }

@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(128) paged_kv_append_rotary_kernel(const Appen
       if (u < pair_units) {
         const uint4 x1 = *reinterpret_cast<const uint4*>(xr + u * 8);
         const uint4 x2 = *reinterpret_cast<const uint4*>(xr + half + u * 8);
-        const uint4 c = __ldg(reinterpret_cast<const uint4*>(q.cos + static_cast<size_t>(pos) * half + u * 8));
-        const uint4 sn = __ldg(reinterpret_cast<const uint4*>(q.sin + static_cast<size_t>(pos) * half + u * 8));
+        const uint4 c = *reinterpret_cast<const uint4*>(q.cos + static_cast<size_t>(pos) * half + u * 8);
+        const uint4 sn = *reinterpret_cast<const uint4*>(q.sin + static_cast<size_t>(pos) * half + u * 8);
         uint4 lo, hi;
         lo.x = rot_lo(x1.x, x2.x, c.x, sn.x);
         lo.y = rot_lo(x1.y, x2.y, c.y, sn.y);

@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(256) rotary_kernel(const RotaryParams p) {
     const int half = p.R / 2;
     const uint4 x1 = *reinterpret_cast<const uint4*>(xr + u * 8);
     const uint4 x2 = *reinterpret_cast<const uint4*>(xr + half + u * 8);
-    const uint4 c = __ldg(reinterpret_cast<const uint4*>(p.cos + static_cast<size_t>(n) * half + u * 8));
-    const uint4 s = __ldg(reinterpret_cast<const uint4*>(p.sin + static_cast<size_t>(n) * half + u * 8));
+    const uint4 c = *reinterpret_cast<const uint4*>(p.cos + static_cast<size_t>(n) * half + u * 8);
+    const uint4 s = *reinterpret_cast<const uint4*>(p.sin + static_cast<size_t>(n) * half + u * 8);
     uint4 lo, hi;
     lo.x = rot_lo(x1.x, x2.x, c.x, s.x);
     lo.y = rot_lo(x1.y, x2.y, c.y, s.y);
