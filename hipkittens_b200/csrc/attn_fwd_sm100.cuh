@@ -272,7 +272,17 @@ inline void set_item_decode(FwdParams& p) {
 #define HK_STAMP2(role, ev) do {} while (0)
 #endif
 
+// Whether the long launches of an instantiation run code with the two griddepcontrol instructions in it. They need neither
+// (a launch of the ordinary way starts after the kernels before it and is waited for as a whole), and their presence
+// alone changes the schedule that the compiler finds for everything behind them. At a full clock (1965 MHz, us with
+// -> without): B16 N4096 H16 D64 1317.0 -> 1309.4, B4 N8192 H64/8 D128 causal 3414 -> 3407, B8 N4096 H32/8 D64 causal
+// 0.3 % less; but B16 N2048 H64/8 D128 1718.6 -> 1722.4, which therefore keeps them. A run-time branch around them is
+// no way out: it costs D128 0.5 %.
 template <int D, bool CAUSAL>
+constexpr bool kLongFwdDependent = D == 128 && !CAUSAL;
+
+// DEP: may be launched as a dependent (launch_dependent with `early`); false: only the ordinary way.
+template <int D, bool CAUSAL, bool DEP>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
@@ -355,8 +365,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_after();
   const uint32_t tmem = tmem_base_slot;
   volatile uint32_t* abortp = &abort_flag;
-  grid_dep_wait();
-  grid_dep_launch();
+  if constexpr (DEP) {
+    grid_dep_wait();
+    grid_dep_launch();
+  }
 
   if (warp < 8) {
     // ------------------------------------------------------------------ softmax warpgroups

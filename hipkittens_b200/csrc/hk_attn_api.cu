@@ -67,9 +67,9 @@ struct DeviceState {
 };
 DeviceState g_dev[kMaxDevices];
 
-template <int D, bool CAUSAL>
+template <int D, bool CAUSAL, bool DEP>
 int prepare_fwd_kernel() {
-  auto* fn = hk::attn_fwd_kernel<D, CAUSAL>;
+  auto* fn = hk::attn_fwd_kernel<D, CAUSAL, DEP>;
   HK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, hk::FwdSmem<D, CAUSAL>::kDynBytes));
   cudaFuncAttributes attr;
   HK_CUDA(cudaFuncGetAttributes(&attr, fn));
@@ -77,11 +77,18 @@ int prepare_fwd_kernel() {
   // that only adds up if it was compiled to exactly kFwdRegsAtLaunch registers per thread at launch.
   // Refuse to launch otherwise: a register pool that is too small would block the re-allocation forever.
   if (attr.numRegs != hk::kFwdRegsAtLaunch) {
-    snprintf(g_cuda_err, sizeof(g_cuda_err), "attn_fwd_kernel<%d,%d> compiled to %d registers, expected %d", D,
-             int(CAUSAL), attr.numRegs, hk::kFwdRegsAtLaunch);
+    snprintf(g_cuda_err, sizeof(g_cuda_err), "attn_fwd_kernel<%d,%d,%d> compiled to %d registers, expected %d", D,
+             int(CAUSAL), int(DEP), attr.numRegs, hk::kFwdRegsAtLaunch);
     return HK_EUNSUPPORTED;
   }
   return HK_OK;
+}
+
+template <int D, bool CAUSAL>
+int prepare_fwd_kernels() {
+  const int rc = prepare_fwd_kernel<D, CAUSAL, true>();
+  if (rc != HK_OK) return rc;
+  return prepare_fwd_kernel<D, CAUSAL, hk::kLongFwdDependent<D, CAUSAL>>();
 }
 
 // The layout that serves an instantiation, with its kernels and launch constants.
@@ -144,10 +151,10 @@ int init_device(int device) {
     return HK_EUNSUPPORTED;
   }
   int rc;
-  if ((rc = prepare_fwd_kernel<128, false>()) != HK_OK) return rc;
-  if ((rc = prepare_fwd_kernel<128, true>()) != HK_OK) return rc;
-  if ((rc = prepare_fwd_kernel<64, false>()) != HK_OK) return rc;
-  if ((rc = prepare_fwd_kernel<64, true>()) != HK_OK) return rc;
+  if ((rc = prepare_fwd_kernels<128, false>()) != HK_OK) return rc;
+  if ((rc = prepare_fwd_kernels<128, true>()) != HK_OK) return rc;
+  if ((rc = prepare_fwd_kernels<64, false>()) != HK_OK) return rc;
+  if ((rc = prepare_fwd_kernels<64, true>()) != HK_OK) return rc;
   if ((rc = hk::prepare_decode_kernels(g_cuda_err, sizeof(g_cuda_err))) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<128, false>()) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<128, true>()) != HK_OK) return rc;
@@ -296,8 +303,9 @@ template <int D, bool CAUSAL>
 int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
                const hk::FwdParams& p, int grid, cudaStream_t stream) {
   const int nk_tiles = (p.NK + hk::kBlockN - 1) / hk::kBlockN;
-  HK_CUDA(hk::launch_dependent(short_kernel(1ll * p.n_items * nk_tiles, grid), hk::attn_fwd_kernel<D, CAUSAL>, grid,
-                               hk::kFwdThreads, hk::FwdSmem<D, CAUSAL>::kDynBytes, stream, tq, tk, tv, to, p));
+  const bool early = short_kernel(1ll * p.n_items * nk_tiles, grid);
+  auto* fn = early ? hk::attn_fwd_kernel<D, CAUSAL, true> : hk::attn_fwd_kernel<D, CAUSAL, hk::kLongFwdDependent<D, CAUSAL>>;
+  HK_CUDA(hk::launch_dependent(early, fn, grid, hk::kFwdThreads, hk::FwdSmem<D, CAUSAL>::kDynBytes, stream, tq, tk, tv, to, p));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return HK_OK;
 }

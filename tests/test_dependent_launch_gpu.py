@@ -52,6 +52,35 @@ def test_back_to_back_calls_equal_synchronised_ones(n, d):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("d", [64, 128])
+def test_long_forward_between_dependent_launches(d, causal):
+    """A forward of more than 100 tiles per CTA is launched the ordinary way (most of them as code without the
+    instructions of dependent launches): it still comes after what is before it, and before what follows."""
+    n, h, hkv = 4096, 32, 8
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert (h // 2) * (n // 128) ** 2 > 100 * sms
+    gen = torch.Generator("cuda").manual_seed(12)
+    q, k, v, d_o = (torch.randn(1, n, x, d, device="cuda", generator=gen).to(torch.bfloat16) for x in (h, hkv, hkv, h))
+    angle = torch.rand(n, d // 2, device="cuda", generator=gen)
+    cos, sin = angle.cos().to(torch.bfloat16), angle.sin().to(torch.bfloat16)
+
+    def chain(sync):
+        x, seen = q.clone(), []
+        for _ in range(4):
+            for step in (lambda: hk.rotary_bnhd(x, cos, sin, out=x),
+                         lambda: seen.extend(hk.attn_fwd(x, k, v, causal=causal)),
+                         lambda: seen.append(hk.attn_bwd_prep(seen[-2], d_o)),
+                         lambda: hk.rotary_bnhd(seen[-3], cos, sin, out=x)):
+                step()
+                if sync:
+                    torch.cuda.synchronize()
+        return seen
+
+    for a, b in zip(chain(False), chain(True)):
+        assert torch.equal(a, b)
+
+
 def test_captured_chain_replays():
     """The dependent launches survive capture into a CUDA graph."""
     q, kv = torch.randn(2, 1, 300, 4, 64, device="cuda").to(torch.bfloat16)
