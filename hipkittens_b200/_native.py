@@ -43,6 +43,7 @@ EXPORTED_SYMBOLS = (
     "hk_last_device_status",
     "hk_selftest_bounded_wait",
     "hk_selftest_fastdiv",
+    "hk_selftest_dkdv_in_pairs",
     "hk_kernel_launch_count",
     "hk_strerror",
     "hk_last_cuda_error",
@@ -126,6 +127,8 @@ def capi() -> ctypes.CDLL:
     lib.hk_selftest_bounded_wait.restype = ci
     lib.hk_selftest_fastdiv.argtypes = []
     lib.hk_selftest_fastdiv.restype = ci
+    lib.hk_selftest_dkdv_in_pairs.argtypes = [ci] * 7
+    lib.hk_selftest_dkdv_in_pairs.restype = ci
     lib.hk_kernel_launch_count.argtypes = []
     lib.hk_kernel_launch_count.restype = ctypes.c_ulonglong
     lib.hk_strerror.argtypes = [ci]

@@ -351,12 +351,10 @@ struct DkdvItem {
 // time read the same Q / dO tiles from L2; an item index is unit * key blocks + key block.
 //
 // Causal: key block j meets G * (NBQ - j) query tiles, 64 times more for the first block than for the last at
-// N = 8192, and a unit has fewer blocks than the GPU has SMs, so no dealing of single blocks to CTAs balances. The
-// blocks are therefore dealt in pairs (j, NBK - 1 - j) of the same unit, which all cost the same: a CTA's round 2r
-// is the first block of its r-th pair and round 2r + 1 the second (none for the middle block of an odd count).
-// When the pairs would leave the last round badly filled (deal_dkdv), single blocks are dealt instead (n_pairs = 0),
-// the longest of all units first, in snake order. B2 N384 H8/2 D128, 12 blocks: 34.6 us in pairs, 25.1 us singly;
-// B4 N4096 H32/8 D128, 512 pairs = 3.46 rounds: 920 us in pairs, 859 us singly.
+// N = 8192. The blocks are dealt in one of two ways (deal_in_pairs says which, why and what it measured): in pairs
+// (j, NBK - 1 - j) of the same unit, which all cost the same - a CTA's round 2r is the first block of its r-th pair and
+// round 2r + 1 the second (none for the middle block of an odd count) -, or singly (n_pairs = 0), the longest of all
+// units first, in snake order.
 template <bool CAUSAL>
 __device__ __forceinline__ int dkdv_item_for_round(const BwdParams& p, int round, int cta, int n_cta) {
   if (!CAUSAL) return item_for_round(p, round, cta, n_cta);

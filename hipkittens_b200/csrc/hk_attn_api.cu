@@ -331,8 +331,33 @@ void set_bwd_decode(hk::BwdParams& p, int per_unit, int per_pos, int inner, int 
   p.fd_in_grp_last = hk::FastDiv((units - p.last_group * p.group_units) * per_pos);
 }
 
+// Whether the causal dK/dV kernel takes its key blocks in pairs (j, nbk - 1 - j), which all cost the same, or singly, the
+// longest of all units first, which leaves no round badly filled whatever their number.
+// Pairs lose the idle part of their last round, and about half of what the missing partner of a middle block (odd counts)
+// leaves idle; the other half is made up by CTAs that drift apart. Single blocks run through many units at a time, so a unit's Q and dO,
+// which its blocks share, come from HBM once the units in flight hold more than L2 keeps. The line is where the two
+// losses meet, fitted to 581 measured shapes (D 64 and 128, 4 to 314 units, 2 to 68 blocks, groups of 1 to 8,
+// pairs 0.61 to 1.00 full): in dK/dV and dQ together a shape takes 0.1 % longer than with the better dealing on average,
+// 2.7 % at worst; always pairs would be 25 % off at worst, always single blocks 10 %. At most 5 % idle stay in
+// pairs, where single blocks gain 2.6 % at best.
+// us, pairs / single: 12 blocks (B2 N384 H8/2 D128) 34.6 / 25.1 and B4 N4096 H32/8 D128 (pairs 0.865 full, 256 MB of Q and
+// dO) 920 / 859, dK/dV alone; with dQ, D128 H16/4: B48 N2048 (0.943 full, 768 MB) 2467 / 2680, B24 N2048 (0.865, 384 MB)
+// 1280 / 1310, B24 N512 (0.649, 96 MB) 152 / 130.
+bool deal_in_pairs(int units, int G, int N, int nbk, int D, int sm_count) {
+  const long long pairs = 1ll * units * ((nbk + 1) / 2), rounds = (pairs + sm_count - 1) / sm_count;
+  const double slots = double(rounds * sm_count);
+  const double idle = 1.0 - 0.5 * (double(pairs) + 0.5 * units * nbk) / slots;
+  constexpr double kKept = 70.0 * (1 << 20);                              // what of the 126 MB of L2 serves Q and dO
+  const int in_flight = units < sm_count ? units : sm_count;
+  const double bytes = 4.0 * in_flight * G * N * D;                       // their Q and dO
+  const double missed = bytes > kKept ? 1.0 - kKept / bytes : 0.0;        // share of the reads that go to HBM
+  const double unshared = std::sqrt(double(in_flight) / double(sm_count));  // few units: their blocks run side by side
+  const double lost = (D == 128 ? 0.22 : 0.13) * missed * unshared;       // a D = 64 tile has half the bytes
+  return idle <= (lost > 0.05 ? lost : 0.05);
+}
+
 // Deals the key blocks to CTAs (dkdv_item_for_round); returns the grid.
-template <bool CAUSAL>
+template <int D, bool CAUSAL>
 int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count) {
   const int units = p.B * p.H_KV;
   p.n_items = units * nbk;
@@ -340,16 +365,12 @@ int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count) {
   set_bwd_decode(p, nbk, 1, 1, grid, false);
   p.n_pairs = 0;
   if (CAUSAL) {
-    // Pairs of blocks (j, nbk - 1 - j) all cost the same and keep few units in flight at a time (a unit's Q and dO are
-    // what its blocks share in L2); they are dealt when they fill their rounds to 95 %. Otherwise single blocks, the
-    // longest first, which even out to a few per cent whatever their number.
-    const int per_unit = (nbk + 1) / 2;
-    const long long pairs = 1ll * units * per_unit, rounds = (pairs + sm_count - 1) / sm_count;
-    if (pairs * 100 >= rounds * sm_count * 95) {
-      p.n_pairs = static_cast<int>(pairs);
+    if (deal_in_pairs(units, p.H / p.H_KV, p.N, nbk, D, sm_count)) {
+      const int per_unit = (nbk + 1) / 2;
+      p.n_pairs = units * per_unit;
       p.fd_pairs = hk::FastDiv(per_unit);
-      grid = pairs < sm_count ? static_cast<int>(pairs) : sm_count;
-      p.total_rounds = 2 * static_cast<int>(rounds);
+      grid = p.n_pairs < sm_count ? p.n_pairs : sm_count;
+      p.total_rounds = 2 * ((p.n_pairs + grid - 1) / grid);
     } else {
       p.fd_pairs = hk::FastDiv(units);
       p.total_rounds = (p.n_items + grid - 1) / grid;
@@ -365,7 +386,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   const int nbk = (NK + hk::kBlockN - 1) / hk::kBlockN;  // key blocks
   if (static_cast<long long>(B) * H * nbq > 0x3fffffffll || static_cast<long long>(B) * H_KV * nbk > 0x3fffffffll)
     return HK_EINVAL;  // work items are indexed with int
-  int grid = deal_dkdv<CAUSAL>(p, nbk, sm_count);
+  int grid = deal_dkdv<D, CAUSAL>(p, nbk, sm_count);
 #ifdef HK_TRACE
   long long* const trace_buf = p.trace;
   p.trace = g_trace_bwd_kernel == 0 ? trace_buf : nullptr;
@@ -884,6 +905,14 @@ int hk_last_device_status(int device) {
   const int word = *host;
   if (word != 0) *host = 0;
   return status_to_code(word);
+}
+
+int hk_selftest_dkdv_in_pairs(int B, int Nq, int Nk, int H, int H_KV, int D, int sm_count) {
+  if (B <= 0 || Nq <= 0 || Nk <= 0 || H <= 0 || H_KV <= 0 || H % H_KV != 0 || sm_count <= 0) return HK_EINVAL;
+  if (D != 64 && D != 128) return HK_EUNSUPPORTED;
+  const int nbk = (Nk + hk::kBlockN - 1) / hk::kBlockN;
+  if (static_cast<long long>(B) * H_KV * nbk > 0x3fffffffll) return HK_EINVAL;
+  return deal_in_pairs(B * H_KV, H / H_KV, Nq, nbk, D, sm_count) ? 1 : 0;
 }
 
 int hk_selftest_fastdiv(void) {

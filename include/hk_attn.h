@@ -279,6 +279,10 @@ int hk_selftest_bounded_wait(int device, unsigned limit_us);
  * decodes its block index with plain divisions (kernels/attn/gqa/kernel.cpp:104-118). */
 int hk_selftest_fastdiv(void);
 
+/* Host-only self-test: how the causal backward deals the key blocks of such a call to a GPU of sm_count SMs: 1 = in pairs
+ * of equal cost, 0 = singly, the longest first; a negative HK_E* code for what hk_attn_bwd_cross would refuse. */
+int hk_selftest_dkdv_in_pairs(int B, int Nq, int Nk, int H, int H_KV, int D, int sm_count);
+
 /* Number of kernels this library has launched in the calling process (all devices). */
 unsigned long long hk_kernel_launch_count(void);
 
