@@ -64,6 +64,8 @@ def _backward(ctx, q, k, v, O, L, dO_bnhd, dQ, dK, dV):
     assert dO_bnhd.shape == O.shape, f"dO shape mismatch: expected {tuple(O.shape)}, got {dO_bnhd.shape}"
     assert dO_bnhd.is_cuda and dO_bnhd.device == O.device, "dO must be on correct CUDA device"
     dO = dO_bnhd.to(torch.bfloat16).contiguous()
+    # saved-tensor hooks may give a tensor back in another layout than it was saved in
+    q, k, v = (t if _tma_viewable(t) else t.contiguous() for t in (q, k, v))
     attn_bwd_strided(q, k, v, O, dO, L, dQ, dK, dV, causal=ctx.causal, softmax_scale=ctx.softmax_scale,
                      kv_lens=ctx.kv_lens)
     _blocking_status(O.device, "backward")

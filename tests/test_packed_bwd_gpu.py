@@ -36,6 +36,58 @@ def test_packed_gradient_is_the_gradient_of_the_parts(b, n, nk, h, hkv, d, causa
             assert torch.equal(qkv.grad[:, :, i], parts[i].grad)
 
 
+@pytest.mark.parametrize("order", [(0, 1, 2, 3, 4), (4, 3, 2, 1, 0), (1, 0, 3, 4, 2)])
+def test_saved_tensor_hooks_may_change_the_layout(order):
+    """What a hook gives back for the projection, or for q, k and v, is the same numbers in a layout of its own choice."""
+    def unpack(t):
+        if t.dtype != torch.bfloat16 or t.dim() != 5:
+            return t  # O and L
+        return t.permute(order).contiguous().permute([order.index(i) for i in range(5)])
+
+    qkv, d_o = _rand(2, 160, 3, 2, 64, seed=9), _rand(2, 160, 2, 64, seed=10)
+    grads = []
+    for hook in (lambda t: t, unpack):
+        x = qkv.clone().requires_grad_()
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, hook):
+            HipSelfAttention(causal=True)(x).backward(d_o)
+        grads.append(x.grad)
+    assert torch.equal(*grads)
+
+
+@pytest.mark.parametrize("order", [(3, 2, 1, 0), (1, 0, 3, 2)])
+def test_saved_tensor_hooks_may_change_the_layout_of_parts(order):
+    q, k, v, d_o = (_rand(2, 160, h, 64, seed=s) for s, h in ((11, 6), (12, 2), (13, 2), (14, 6)))
+    saved = []
+
+    def unpack(t):
+        if t.dtype != torch.bfloat16 or t.data_ptr() == saved[3]:
+            return t  # L and O
+        return t.permute(order).contiguous().permute([order.index(i) for i in range(4)])
+
+    def pack(t):
+        saved.append(t.data_ptr())
+        return t
+
+    grads = []
+    for hook in (lambda t: t, unpack):
+        saved.clear()
+        leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+        with torch.autograd.graph.saved_tensors_hooks(pack, hook):
+            HipAttnFunction.apply(*leaves, True).backward(d_o)
+        grads.append([t.grad for t in leaves])
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
+
+
+def test_offloaded_saved_tensors():
+    qkv, d_o = _rand(2, 160, 3, 2, 64, seed=15), _rand(2, 160, 2, 64, seed=16)
+    a, b = qkv.clone().requires_grad_(), qkv.clone().requires_grad_()
+    HipSelfAttention()(a).backward(d_o)
+    with torch.autograd.graph.save_on_cpu():
+        HipSelfAttention()(b).backward(d_o)
+    assert torch.equal(a.grad, b.grad)
+
+
 def test_float16_projection_takes_the_converting_path():
     qkv = _rand(2, 160, 3, 2, 64, seed=4).half().requires_grad_()
     out = HipSelfAttention()(qkv)
