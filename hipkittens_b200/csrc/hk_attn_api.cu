@@ -268,8 +268,11 @@ int make_bnhd_map(CUtensorMap* map, const void* base, int B, int N, int heads, i
   CUresult r = encode();
   if (r == CUDA_ERROR_INVALID_CONTEXT) {
     // a thread that has made no runtime call yet (autograd's) has no current context: let the runtime bind the
-    // device's own and try again
-    HK_CUDA(cudaFree(nullptr));
+    // device's own and try again. cudaSetDevice does that and, unlike cudaFree(nullptr), leaves a graph alone that
+    // some thread is capturing at the time.
+    int device = 0;
+    HK_CUDA(cudaGetDevice(&device));
+    HK_CUDA(cudaSetDevice(device));
     r = encode();
   }
   if (r != CUDA_SUCCESS) {

@@ -102,3 +102,26 @@ def test_captured_chain_replays():
         graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, expected)
+
+
+def test_a_new_thread_launches_into_a_capture():
+    """A thread without a CUDA context of its own may be the one that launches, also while a stream is being captured."""
+    import threading
+
+    q = torch.randn(1, 300, 4, 64, device="cuda").to(torch.bfloat16)
+    out, lse = torch.empty_like(q), torch.empty(1, 4, 1, 300, device="cuda")
+    expected, _ = hk.attn_fwd(q, q, q)
+    torch.cuda.synchronize()
+    codes = []
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):  # "global": calls that could disturb the capture are refused in every thread
+        stream = torch.cuda.current_stream().cuda_stream
+        t = threading.Thread(target=lambda: codes.append(_native.capi().hk_attn_fwd(
+            q.data_ptr(), q.data_ptr(), q.data_ptr(), out.data_ptr(), lse.data_ptr(), 1, 300, 4, 4, 64, 0, 0.0, 0, stream)))
+        t.start()
+        t.join()
+    assert codes == [0]
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, expected)
