@@ -672,9 +672,11 @@ int hk_attn_bwd_cross(const void* q, const void* k, const void* v, const void* d
                       const float* delta, void* dq, void* dk, void* dv, int B, int N, int NK, int H, int H_KV, int D,
                       const int32_t* kv_lens, int causal, float softmax_scale, int dq_layout, int device,
                       void* cuda_stream) {
-  if (dq_layout != HK_DQ_BNHD && dq_layout != HK_DQ_BHND) return HK_EINVAL;
-  if (N <= 0 || NK <= 0 || H <= 0 || H_KV <= 0) return HK_EINVAL;
+  // in the order in which a call that is wrong in several ways is answered
+  if (!q || !k || !v || !d_o || !lse || !delta || !dq || !dk || !dv) return HK_EINVAL;
+  if (B <= 0 || N <= 0 || NK <= 0 || H <= 0 || H_KV <= 0) return HK_EINVAL;
   if (D != 64 && D != 128) return HK_EUNSUPPORTED;
+  if (dq_layout != HK_DQ_BNHD && dq_layout != HK_DQ_BHND) return HK_EINVAL;
   const long long qs[3] = {(long long)N * H * D, (long long)H * D, D};
   const long long ks[3] = {(long long)NK * H_KV * D, (long long)H_KV * D, D};
   const long long dqs[3] = {(long long)N * H * D, D, (long long)N * D};  // [B, H, N, D]

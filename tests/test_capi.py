@@ -128,3 +128,14 @@ def test_bwd_rejects_bad_arguments_before_cuda(native_built):
     assert lib.hk_attn_bwd_prep(64, 64, 64, 1, 0, 2, 128, 0, None) == _native.HK_EINVAL
     assert lib.hk_attn_dq_shuffle(64, 64, 1, 128, 2, 128, 0, None) == _native.HK_EINVAL  # aliasing buffers
     assert lib.hk_attn_dq_shuffle(64, 128, 1, 128, 2, 100, 0, None) == _native.HK_EINVAL  # D not a multiple of 8
+
+
+def test_bwd_answers_calls_that_are_wrong_twice_in_one_order(native_built):
+    """Pointers and sizes first, then the head dimension, then the layout."""
+    lib = hk.capi()
+
+    def bwd(q=64, B=1, H=2, HKV=1, D=128, layout=0):
+        return lib.hk_attn_bwd(q, 64, 64, 64, 64, 64, 64, 64, 64, B, 128, H, HKV, D, 0, 0.0, layout, 0, None)
+
+    assert bwd(q=None, D=96) == bwd(B=0, D=96) == bwd(layout=2) == _native.HK_EINVAL
+    assert bwd(D=96, layout=2) == bwd(D=96, H=3, HKV=2) == _native.HK_EUNSUPPORTED
