@@ -138,19 +138,29 @@ def build_shims(force: bool = False):
     return out
 
 
+def built_for_this_torch(path: str) -> bool:
+    """Whether the built ``_torch_front`` was compiled against the torch that is installed: its tensors are read through
+    torch's C++ classes, which another version may lay out differently."""
+    import torch
+
+    with open(path, "rb") as f:
+        return f"built for torch {torch.__version__}\0".encode() in f.read()
+
+
 def build_torch_front(force: bool = False) -> str:
     """``lib/_torch_front``: the tensor front ends in native code, the one piece that links against libtorch."""
     import torch
 
     target = shim_path("lib", "_torch_front")
     src = os.path.join(CSRC, "torch_front.cpp")
-    if not force and _newer(target, [src, os.path.join(INCLUDE, "hk_attn.h"), LIB_PATH]):
+    if (not force and _newer(target, [src, os.path.join(INCLUDE, "hk_attn.h"), LIB_PATH])
+            and built_for_this_torch(target)):
         return target
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(nvcc_path())) or "/usr/local/cuda"
     _run([
         "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DHK_TORCH_VERSION="{torch.__version__}"',
         "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
         "-I", os.path.join(cuda, "include"), "-I", sysconfig.get_paths()["include"],
         src, "-o", target,

@@ -158,6 +158,12 @@ def _front():
     global _front_module
     if _front_module is None:
         capi()  # the front ends link against the library: this names it if it is missing
+        from . import _build
+
+        path = _build.shim_path("lib", "_torch_front")
+        if os.path.exists(path) and not _build.built_for_this_torch(path):
+            raise ImportError(f"{path} was built for another version of torch than {torch.__version__}: "
+                              "rebuild it with `python -m hipkittens_b200._build`")
         _front_module = _load_ext("lib", "_torch_front")
     return _front_module
 

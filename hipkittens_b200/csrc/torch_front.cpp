@@ -324,4 +324,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_torch_front", "Native tensor fron
 
 }  // namespace
 
+// Looked for in the built file, before it is loaded, by whoever wants to know which torch it was compiled against.
+extern "C" __attribute__((used, visibility("default"))) const char hk_torch_front_built_for[] =
+    "built for torch " HK_TORCH_VERSION;
+
 PyMODINIT_FUNC PyInit__torch_front(void) { return PyModule_Create(&module); }
