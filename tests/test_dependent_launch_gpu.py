@@ -52,6 +52,109 @@ def test_back_to_back_calls_equal_synchronised_ones(n, d):
         assert torch.equal(a, b)
 
 
+def test_decode_steps_over_several_chunks():
+    """Contexts that are cut into 2 to 9 chunks, so that the combine kernel merges partials of the split kernel before it
+    while the append of the next step stands behind it; the workspace is one and the same."""
+    gen = torch.Generator("cuda").manual_seed(13)
+    b, h, hkv, pages = 3, 16, 2, 290
+    start0 = torch.tensor([700, 2100, 4500], dtype=torch.int32, device="cuda")
+    pool0 = [torch.randn(b * pages, 16, hkv, 128, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(2)]
+    table = torch.randperm(b * pages, device="cuda", generator=gen).to(torch.int32).reshape(b, pages)
+    need = hk.paged_decode_workspace_bytes(b, h, 128, pages)
+    workspace = torch.empty(need, dtype=torch.uint8, device="cuda")
+    angle = torch.rand(pages * 16, 64, device="cuda", generator=gen)
+    cos, sin = angle.cos().to(torch.bfloat16), angle.sin().to(torch.bfloat16)
+    q0 = torch.randn(b, 1, h, 128, device="cuda", generator=gen).to(torch.bfloat16)
+
+    def chain(sync):
+        k, v = (p.clone() for p in pool0)
+        q, seen = q0, []
+        for i in range(40):
+            start = start0 + i
+            hk.paged_kv_append_rotary(q[:, :, :hkv].contiguous(), q[:, :, hkv:2 * hkv].contiguous(), k, v, table, start,
+                                      cos, sin)
+            if sync:
+                torch.cuda.synchronize()
+            q, lse = hk.paged_decode(q, k, v, table, start + 1, workspace=workspace)
+            if sync:
+                torch.cuda.synchronize()
+            seen += [q, lse]
+        return seen
+
+    for a, b_ in zip(chain(False), chain(True)):
+        assert torch.equal(a, b_)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("n,d", [(200, 64), (1000, 128)])
+def test_three_call_backward_behind_its_forward(n, d, causal):
+    """delta, the gradients and the shuffle each read what the kernel before them wrote, and the next pass overwrites it."""
+    gen = torch.Generator("cuda").manual_seed(14)
+    q, k, v, d_o = (torch.randn(2, n, x, d, device="cuda", generator=gen).to(torch.bfloat16) for x in (4, 2, 2, 4))
+
+    def chain(sync):
+        seen, x, o, lse = [], q, torch.empty_like(q), torch.empty(2, 4, 1, n, device="cuda")
+        delta, dq_in = torch.empty_like(lse), torch.empty(2, 4, n, d, dtype=torch.bfloat16, device="cuda")
+        dk, dv = torch.empty_like(k), torch.empty_like(v)
+        for i in range(10):
+            dq = torch.empty_like(q)
+            for step in (lambda: hk.attn_fwd(x, k, v, causal=causal, out=o, lse=lse),
+                         lambda: hk.attn_bwd_prep(o, d_o, delta=delta),
+                         lambda: hk.attn_bwd(x, k, v, d_o, lse, delta, causal=causal, dq=dq_in, dk=dk, dv=dv,
+                                             dq_layout=_native.HK_DQ_BHND),
+                         lambda: hk.dq_shuffle(dq_in, dq)):
+                step()
+                if sync:
+                    torch.cuda.synchronize()
+            seen.append(dq)
+            x = dq
+        return [*seen, delta, dk, dv, o, lse]
+
+    for a, b in zip(chain(False), chain(True)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_events_of_another_stream_are_waited_for(captured):
+    """A dependent launch behind a wait for an event reads what that event stands for, in a stream and in a graph."""
+    gen = torch.Generator("cuda").manual_seed(15)
+    src = [torch.randn(1, 256, 4, 64, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(6)]
+    cos, sin = (torch.randn(256, 32, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(2))
+    big = torch.randn(4096, 4096, device="cuda", generator=gen)
+    side = torch.cuda.Stream()
+    x, y = torch.zeros_like(src[0]), src[0].clone()
+    outs = [torch.empty_like(x) for _ in src]
+
+    def calls():
+        main = torch.cuda.current_stream()
+        for s, o in zip(src, outs):
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                torch.mm(big, big)  # some hundred microseconds
+                x.copy_(s)
+            hk.rotary_bnhd(y, cos, sin, out=y)  # the kernel before in the same stream is done long before that
+            main.wait_stream(side)
+            hk.rotary_bnhd(x, cos, sin, out=o)
+
+    expected = [hk.rotary_bnhd(s, cos, sin) for s in src]
+    torch.cuda.synchronize()
+    if captured:
+        torch.mm(big, big)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            calls()
+        graph.replay()
+        for o in outs:
+            o.zero_()
+        x.zero_()
+        graph.replay()
+    else:
+        calls()
+    torch.cuda.synchronize()
+    for a, b in zip(outs, expected):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("d", [64, 128])
 def test_long_forward_between_dependent_launches(d, causal):

@@ -8,8 +8,18 @@ from hipkittens_b200 import _native
 pytestmark = pytest.mark.gpu
 
 
+_gen = None
+
+
+@pytest.fixture(autouse=True)
+def _seeded():
+    """One generator per test, so that no two tensors of a test are alike: an argument taken for another shows."""
+    global _gen
+    _gen = torch.Generator("cuda").manual_seed(7)
+
+
 def _rand(*shape):
-    return torch.randn(shape, device="cuda", generator=torch.Generator("cuda").manual_seed(7)).to(torch.bfloat16)
+    return torch.randn(shape, device="cuda", generator=_gen).to(torch.bfloat16)
 
 
 class _Nothing:
@@ -50,19 +60,48 @@ def test_paged_entries(monkeypatch):
     pools = [_rand(9, 16, 2, 128) for _ in range(2)]
     table = torch.randperm(9, device="cuda").to(torch.int32)[:8].reshape(2, 4).contiguous()
     lens = torch.tensor([50, 64], dtype=torch.int32, device="cuda")
-    new, start = _rand(2, 3, 2, 128), (lens - 3).to(torch.int32)
+    k_new, v_new, start = _rand(2, 3, 2, 128), _rand(2, 3, 2, 128), (lens - 3).to(torch.int32)
     cos, sin = _rand(64, 64), _rand(64, 64)
+    q1, q3, x = _rand(2, 1, 8, 128), _rand(2, 3, 8, 128), _rand(2, 60, 4, 128)
 
     def append(fn, *extra):
         k, v = (p.clone() for p in pools)
-        fn(new, new, k, v, table, start, *extra)
+        fn(k_new, v_new, k, v, table, start, *extra)
         return k, v
 
     _both(monkeypatch, lambda: append(hk.paged_kv_append))
     _both(monkeypatch, lambda: append(hk.paged_kv_append_rotary, cos, sin))
-    _both(monkeypatch, lambda: hk.paged_decode(_rand(2, 1, 8, 128), *pools, table, lens))
-    _both(monkeypatch, lambda: hk.attn_fwd_paged(_rand(2, 3, 8, 128), *pools, table, lens))
-    _both(monkeypatch, lambda: hk.rotary_bnhd(_rand(2, 60, 4, 128), cos, sin, pos_offset=4))
+    for scale in (None, 0.3):
+        _both(monkeypatch, lambda: hk.paged_decode(q1, *pools, table, lens, softmax_scale=scale))
+        _both(monkeypatch, lambda: hk.attn_fwd_paged(q3, *pools, table, lens, causal=True, softmax_scale=scale))
+    _both(monkeypatch, lambda: hk.rotary_bnhd(x, cos, sin, pos_offset=4))
+    need = hk.paged_decode_workspace_bytes(2, 8, 128, 4)
+    out, lse = torch.empty_like(q1), torch.empty(2, 8, 1, 1, device="cuda")
+    r = _both(monkeypatch, lambda: hk.paged_decode(q1, *pools, table, lens, out=out, lse=lse,
+                                                   workspace=torch.empty(max(need, 256), dtype=torch.uint8, device="cuda")))
+    assert r[0] is out and r[1] is lse
+
+
+@pytest.mark.parametrize("causal", [False, True])
+def test_attn_bwd_strided(monkeypatch, causal):
+    q, kv, d_o = _rand(2, 130, 4, 64), _rand(2, 200, 2, 2, 64), _rand(2, 130, 4, 64)
+    k, v = kv.unbind(2)
+    for lens in (None, torch.tensor([200, 140], dtype=torch.int32, device="cuda")):
+        for scale in (None, 0.3, 1):
+            o, lse = hk.attn_fwd(q, k, v, causal=causal, softmax_scale=scale, kv_lens=lens)
+
+            def grads():
+                dq, dkv = torch.full_like(q, 7), torch.full_like(kv, 7)
+                _native.attn_bwd_strided(q, k, v, o, d_o, lse, dq, *dkv.unbind(2), causal=causal, softmax_scale=scale,
+                                         kv_lens=lens)
+                return dq, dkv
+
+            dq, dkv = _both(monkeypatch, grads)
+            delta = hk.attn_bwd_prep(o, d_o)
+            ref = hk.attn_bwd(q, k.contiguous(), v.contiguous(), d_o, lse, delta, causal=causal, softmax_scale=scale,
+                              kv_lens=lens)
+            for got, want in zip((dq, dkv[:, :, 0], dkv[:, :, 1]), ref):
+                assert torch.equal(got, want)
 
 
 def test_what_was_refused_stays_refused(monkeypatch):
@@ -80,6 +119,27 @@ def test_what_was_refused_stays_refused(monkeypatch):
         lambda: hk.attn_fwd(*(t[..., :48].contiguous() for t in (q, k, k))),
         lambda: hk.rotary_bnhd(q, k[0, :32, 0], k[0, :32, 0]),
         lambda: hk.rotary_bnhd(q, k[0, :, 0].contiguous(), k[0, :, 0].contiguous(), pos_offset=-1),
+    ]
+    q1, pool = _rand(2, 1, 4, 128), _rand(9, 16, 2, 128)
+    table, lens = torch.zeros(2, 4, dtype=torch.int32, device="cuda"), torch.ones(2, dtype=torch.int32, device="cuda")
+    new, tab = _rand(2, 1, 2, 128), _rand(64, 64)
+    calls += [
+        lambda: hk.paged_decode(q1.float(), pool, pool, table, lens),
+        lambda: hk.paged_decode(q1, pool, pool[:8], table, lens),
+        lambda: hk.paged_decode(q1, pool, pool, table.long(), lens),
+        lambda: hk.paged_decode(q1, pool, pool, table, lens[:1]),
+        lambda: hk.paged_decode(q1, pool, pool, table, lens.cpu()),
+        lambda: hk.paged_decode(q1, pool, pool, table[:, ::2], lens),
+        lambda: hk.paged_decode(q1[:, :, :3].contiguous(), pool, pool, table, lens),
+        lambda: hk.paged_decode(q1, pool, pool, table, lens, workspace=torch.empty(16, dtype=torch.uint8, device="cuda")),
+        lambda: hk.attn_fwd_paged(q1, pool, pool[..., :64].contiguous(), table, lens),
+        lambda: hk.attn_fwd_paged(q1, pool, pool, table, lens, out=q1.float()),
+        lambda: hk.paged_kv_append(new, new.float(), pool, pool, table, lens),
+        lambda: hk.paged_kv_append(new, new, pool, pool, table, lens.float()),
+        lambda: hk.paged_kv_append_rotary(new, new, pool, pool, table, lens, tab, tab[:32]),
+        lambda: _native.attn_bwd_strided(q, k, k, q, q[:, :32], lse, q.clone(), k.clone(), k.clone()),
+        lambda: _native.attn_bwd_strided(q, k, k, q, q, lse[:, :2], q.clone(), k.clone(), k.clone()),
+        lambda: _native.attn_bwd_strided(q, k, k, q, q, lse, q.float(), k.clone(), k.clone()),
     ]
     for call in calls:
         with pytest.raises(RuntimeError) as native:
