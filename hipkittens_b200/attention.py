@@ -64,10 +64,16 @@ def _backward(ctx, q, k, v, O, L, dO_bnhd, dQ, dK, dV):
     assert dO_bnhd.shape == O.shape, f"dO shape mismatch: expected {tuple(O.shape)}, got {dO_bnhd.shape}"
     assert dO_bnhd.is_cuda and dO_bnhd.device == O.device, "dO must be on correct CUDA device"
     dO = dO_bnhd.to(torch.bfloat16).contiguous()
-    # saved-tensor hooks may give a tensor back in another layout than it was saved in
-    q, k, v = (t if _tma_viewable(t) else t.contiguous() for t in (q, k, v))
-    attn_bwd_strided(q, k, v, O, dO, L, dQ, dK, dV, causal=ctx.causal, softmax_scale=ctx.softmax_scale,
-                     kv_lens=ctx.kv_lens)
+    rest = dict(causal=ctx.causal, softmax_scale=ctx.softmax_scale, kv_lens=ctx.kv_lens)
+    try:
+        attn_bwd_strided(q, k, v, O, dO, L, dQ, dK, dV, **rest)
+    except RuntimeError:
+        # saved-tensor hooks may have given q, k or v back in a layout that the kernels cannot read (looked for only here,
+        # where the call was refused: the look takes 4 us)
+        dense = [t if _tma_viewable(t) else t.contiguous() for t in (q, k, v)]
+        if all(a is b for a, b in zip(dense, (q, k, v))):
+            raise
+        attn_bwd_strided(*dense, O, dO, L, dQ, dK, dV, **rest)
     _blocking_status(O.device, "backward")
 
 
