@@ -121,7 +121,7 @@ static_assert(BwdSmem<128>::kDynBytes <= 232448, "shared memory budget of one CT
 // D/8 lanes per (batch, position, head) row, 16 bytes of O and of dO per lane; bound by HBM (O and dO are read once).
 // A thread takes kRowPassUnroll rows and requests all of them before it reduces the first: with one row per thread
 // the 32 bytes a thread had in flight left HBM at 5.7 TB/s (B16 N2048 H64 D128: 187 us), with four it
-// reads 7.0 TB/s (154 us). grid = ceil(rows / row_pass_rows(D)), block = 256.
+// reads 7.0 TB/s (154 us). grid = ceil(rows / row_pass_rows(D / 8)), block = 256.
 constexpr int kRowPassUnroll = 4;
 __host__ __device__ constexpr int row_pass_rows(int lanes_per_row) { return 8 * (32 / lanes_per_row) * kRowPassUnroll; }
 
@@ -420,8 +420,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int warp = tid >> 5;
   const int lane = tid & 31;
 
-  if ((smem_u32(bwd_smem) & 1023u) != 0) {
-    grid_dep_wait();  // uniform over the CTA; nothing has been allocated yet
+  if ((smem_u32(bwd_smem) & 1023u) != 0) {  // uniform over the CTA; nothing has been allocated yet
+    grid_dep_wait();
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusSmemAlign);
     return;
   }

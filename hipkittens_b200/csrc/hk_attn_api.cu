@@ -18,6 +18,7 @@
 #define HK_BWD_PARTS 2
 #include "attn_bwd_sm100.cuh"
 #include "attn_fwd_sm100.cuh"
+#include "dependent_launch.cuh"
 #include "key_padding_sm100.cuh"
 #include "paged_decode_sm100.cuh"
 #include "paged_kv_append_sm100.cuh"
@@ -296,10 +297,15 @@ __global__ void bounded_wait_selftest_kernel(int* status, unsigned long long lim
   if (!ok && threadIdx.x == 0) atomicCAS(status, hk::kStatusOk, hk::kStatusTimeout);
 }
 
-// Whether an attention kernel is launched so that it may start under the tail of the one before it: up to about 100
-// tiles (two heads x 128 x 128 in the forward, one in the backward) per CTA, some 0.2 ms. There a launch and a
-// prologue are a visible share; long kernels gain nothing and measured 0.3 to 1 % slower in a loop (B16 N4096 H16 D64
-// forward 1 449 -> 1 462 us, B4 T512 chunked prefill 343 -> 346 us).
+// Whether an attention kernel is launched so that it may start under the tail of the one before it: up to 100 tiles per CTA
+// (two heads x 128 x 128 in the forward, one in the backward), where a launch and a prologue are a visible share of it.
+// The tiles are counted as if nothing were masked. A causal call has about half of them, and a paged one those of its
+// contexts, which the host does not know, and not of its block table's width: such calls are launched the ordinary way
+// from half the time on, or earlier.
+// us per call in a loop, dependent / ordinary, at 28, 62, 111, 221 and 443 tiles per CTA (H32/8 D128, B1 N2048, N3072, N4096,
+// B2 and B4 N4096): non-causal 65.8 / 67.9, 134.8 / 136.8, 232.0 / 233.7, 415.7 / 417.0, 830.7 / 830.1; causal
+// 39.0 / 40.3, 77.2 / 79.4, 117.7 / 120.4, 230.7 / 229.8, 456.6 / 452.8. Append and paged chunk, 8 x 512 tokens on contexts
+// of 4096 (221 tiles): 487.8 / 479.2, and so the line is no higher.
 bool short_kernel(long long tiles, int grid) { return tiles <= 100ll * grid; }
 
 template <int D, bool CAUSAL>
@@ -336,16 +342,16 @@ void set_bwd_decode(hk::BwdParams& p, int per_unit, int per_pos, int inner, int 
 
 // Whether the causal dK/dV kernel takes its key blocks in pairs (j, nbk - 1 - j), which all cost the same, or singly, the
 // longest of all units first, which leaves no round badly filled whatever their number.
-// Pairs lose the idle part of their last round, and about half of what the missing partner of a middle block (odd counts)
-// leaves idle; the other half is made up by CTAs that drift apart. Single blocks run through many units at a time, so a unit's Q and dO,
-// which its blocks share, come from HBM once the units in flight hold more than L2 keeps. The line is where the two
-// losses meet, fitted to 581 measured shapes (D 64 and 128, 4 to 314 units, 2 to 68 blocks, groups of 1 to 8,
-// pairs 0.61 to 1.00 full): in dK/dV and dQ together a shape takes 0.1 % longer than with the better dealing on average,
-// 2.7 % at worst; always pairs would be 25 % off at worst, always single blocks 10 %. At most 5 % idle stay in
-// pairs, where single blocks gain 2.6 % at best.
-// us, pairs / single: 12 blocks (B2 N384 H8/2 D128) 34.6 / 25.1 and B4 N4096 H32/8 D128 (pairs 0.865 full, 256 MB of Q and
-// dO) 920 / 859, dK/dV alone; with dQ, D128 H16/4: B48 N2048 (0.943 full, 768 MB) 2467 / 2680, B24 N2048 (0.865, 384 MB)
-// 1280 / 1310, B24 N512 (0.649, 96 MB) 152 / 130.
+// Pairs lose the idle part of their last round, and about half of what the missing partner of a middle block (odd
+// counts) leaves idle; the other half is made up by CTAs that drift apart. Single blocks run through many units at a
+// time, so a unit's Q and dO, which its blocks share, come from HBM once the units in flight hold more than L2 keeps.
+// The line is where the two losses meet, fitted to 581 measured shapes (D 64 and 128, 4 to 314 units, 2 to 68 blocks,
+// groups of 1 to 8, pairs 0.61 to 1.00 full): in dK/dV and dQ together a shape takes 0.1 % longer than with the better
+// dealing on average, 2.7 % at worst; always pairs would be 25 % off at worst, always single blocks 10 %. At most 5 %
+// idle stay in pairs, where single blocks gain 2.6 % at best.
+// us, pairs / single: 12 blocks (B2 N384 H8/2 D128) 34.6 / 25.1 and B4 N4096 H32/8 D128 (pairs 0.865 full, 256 MB of Q
+// and dO) 920 / 859, dK/dV alone; with dQ, D128 H16/4: B48 N2048 (0.943 full, 768 MB) 2467 / 2680, B24 N2048 (0.865,
+// 384 MB) 1280 / 1310, B24 N512 (0.649, 96 MB) 152 / 130.
 bool deal_in_pairs(int units, int G, int N, int nbk, int D, int sm_count) {
   const long long pairs = 1ll * units * ((nbk + 1) / 2), rounds = (pairs + sm_count - 1) / sm_count;
   const double slots = double(rounds * sm_count);

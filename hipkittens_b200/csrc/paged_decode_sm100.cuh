@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dependent_launch.cuh"
 #include "sm100_ptx.cuh"
 
 namespace hk {
@@ -313,8 +314,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(c
 // grid = (H, S), block = 128 threads (one per output column). Merges the per-chunk partials of
 // sequences that span more than one chunk.
 __global__ void __launch_bounds__(kDecodeD) paged_decode_combine_kernel(const DecodeParams p) {
-  ptx::grid_dep_wait();
-  ptx::grid_dep_launch();  // the split grid has completed and its partials are visible
+  ptx::grid_dep_wait();  // from here on the split grid has completed and its partials are visible
+  ptx::grid_dep_launch();
   const int head = blockIdx.x, seq = blockIdx.y;
   const int ctx = min(p.ctx_lens[seq], p.max_pages * kPageTokens);  // clamped as in the split kernel, which reports it
   const int d = threadIdx.x;
@@ -357,24 +358,6 @@ __global__ void __launch_bounds__(kDecodeD) paged_decode_combine_kernel(const De
   for (int i = 0; i < n_splits; ++i) acc += s_w[i] * ws_o[(slot0 + i) * kDecodeD + d];
   p.o[(size_t(seq) * p.H + head) * kDecodeD + d] = __float2bfloat16(acc / s_L);
   if (d == 0) p.lse[size_t(seq) * p.H + head] = s_M * p.scale + __logf(s_L);
-}
-
-// Launch with programmatic stream serialization (see ptx::grid_dep_wait, which every kernel launched so executes), or, with
-// `early` false, an ordinary launch.
-template <typename... Params, typename... Args>
-cudaError_t launch_dependent(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
-                             cudaStream_t stream, const Args&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = early ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
 inline int prepare_decode_kernels(char* err, size_t err_len) {

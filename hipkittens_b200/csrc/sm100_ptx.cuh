@@ -37,18 +37,20 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---------------------------------------------------------------- dependent launch
-// Kernels are launched with programmatic stream serialization: their CTAs may start while the kernel before them in the
-// stream is finishing, and run their prologue (barriers, TMEM, descriptor prefetch) under its tail. grid_dep_wait() is
-// every thread's first step before it touches global memory: it returns when the kernels before have completed and their
-// writes are visible. It also makes completion transitive (a kernel only completes after the one before it), so no
-// CTA may leave without it. grid_dep_launch() lets the next kernel do the same, once every CTA of this one has got there.
+// Kernels but the long attention ones, the padding-mask kernel and the self-test are launched with programmatic stream
+// serialization (launch_dependent): their CTAs may start while the kernel before them in the stream is finishing, and run
+// their prologue (barriers, TMEM, descriptor prefetch) under its tail. The order is prologue, grid_dep_wait(),
+// grid_dep_launch(), and then the first access to global memory.
+// grid_dep_wait() returns when the kernels before have completed and their writes are visible. It also makes completion
+// transitive (a kernel only completes after the one before it), so no CTA may leave without it. grid_dep_launch() lets
+// the next kernel start, once every CTA of this one has got there: only behind the wait, or that kernel could run
+// while the one two before it is still writing what it reads.
 // Nothing that a kernel before may have written is read through the non-coherent path (__ldg, or const __restrict__, which
 // lets the compiler choose it): that path wants data that nobody writes while the grid exists, and the grid exists while
 // the kernel before is still writing; nor does the "memory" clobber hold such loads behind the wait. Plain loads cost
 // nothing (B16 N2048 H64 D128 backward through the three calls 6 761 us with either, batch-64 decode 181.6 us with either).
-// What it is worth (us per pass in a loop, before -> after): B1 N256 D64 forward
-// 8.3 -> 7.0, rotary twice and attention of a 1511-token prompt 43.2 -> 38.3, one-token append and decode 16.4 -> 12.2;
-// nothing beyond 0.3 ms, where attention kernels are launched the ordinary way (see launch_dependent).
+// What dependent launches are worth (us per pass in a loop, before -> after): B1 N256 D64 forward 8.3 -> 7.0, rotary twice
+// and attention of a 1511-token prompt 43.2 -> 38.3, one-token append and decode 16.4 -> 12.2.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
