@@ -120,8 +120,9 @@ static_assert(BwdSmem<128>::kDynBytes <= 232448, "shared memory budget of one CT
 // ------------------------------------------------------------------------------------ delta = rowsum(dO * O)
 // D/8 lanes per (batch, position, head) row, 16 bytes of O and of dO per lane; bound by HBM (O and dO are read once).
 // A thread takes kRowPassUnroll rows and requests all of them before it reduces the first: with one row per thread
-// the 32 bytes a thread had in flight left HBM at 5.7 TB/s (B16 N2048 H64 D128: 187 us), with four it
-// reads 7.0 TB/s (154 us). grid = ceil(rows / row_pass_rows(D / 8)), block = 256.
+// the 32 bytes a thread had in flight left HBM at 5.6 TB/s (B16 N2048 H64 D128, 1.07 GB: 191 us in a loop, 199 alone),
+// with four it reads 6.9 TB/s (154 and 156 us). Streaming loads, without a branch around them: as plain ones behind one
+// they took 158 and 163 us, as non-coherent ones 151 and 159 (which ptx::grid_dep_wait rules out). grid = ceil(rows / row_pass_rows(D / 8)), block = 256.
 constexpr int kRowPassUnroll = 4;
 __host__ __device__ constexpr int row_pass_rows(int lanes_per_row) { return 8 * (32 / lanes_per_row) * kRowPassUnroll; }
 
@@ -140,12 +141,9 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
   ptx::grid_dep_launch();
 #pragma unroll
   for (int u = 0; u < kRowPassUnroll; ++u) {
-    const int row = row0 + u * kRowsPerWarp;
-    a[u] = b[u] = make_uint4(0, 0, 0, 0);
-    if (row < rows) {
-      a[u] = reinterpret_cast<const uint4*>(o + static_cast<size_t>(row) * D)[sub];
-      b[u] = reinterpret_cast<const uint4*>(d_o + static_cast<size_t>(row) * D)[sub];
-    }
+    const int row = min(row0 + u * kRowsPerWarp, rows - 1);  // a row beyond the last: that one again, and not stored
+    a[u] = __ldcs(reinterpret_cast<const uint4*>(o + static_cast<size_t>(row) * D) + sub);
+    b[u] = __ldcs(reinterpret_cast<const uint4*>(d_o + static_cast<size_t>(row) * D) + sub);
   }
 #pragma unroll
   for (int u = 0; u < kRowPassUnroll; ++u) {
@@ -173,8 +171,8 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
 
 // ------------------------------------------------------------------------------------ dQ [B,H,N,D] -> [B,N,H,D]
 // Pure byte movement, bound by HBM: 16-byte units, kRowPassUnroll of them per thread, all requested before the first is
-// written (B16 N2048 H64 D128: 201 us with one unit per thread and three 64-bit divisions for it,
-// 164 us now). VEC: units per row (16 or 8; 0 = any, `vec` says how many).
+// written (B16 N2048 H64 D128: 201 us in a loop and 208 alone with one unit per thread and three 64-bit divisions for it,
+// 160 and 168 us now: 6.7 TB/s). VEC: units per row (16 or 8; 0 = any, `vec` says how many).
 // grid = ceil(rows * vec / (256 * kRowPassUnroll)), block = 256.
 template <int VEC>
 __global__ void __launch_bounds__(256) attn_dq_shuffle_kernel(const uint4* src, uint4* dst,

@@ -47,8 +47,8 @@ __device__ __forceinline__ bool elect_one() {
 // while the one two before it is still writing what it reads.
 // Nothing that a kernel before may have written is read through the non-coherent path (__ldg, or const __restrict__, which
 // lets the compiler choose it): that path wants data that nobody writes while the grid exists, and the grid exists while
-// the kernel before is still writing; nor does the "memory" clobber hold such loads behind the wait. Plain loads cost
-// nothing (B16 N2048 H64 D128 backward through the three calls 6 761 us with either, batch-64 decode 181.6 us with either).
+// the kernel before is still writing; nor does the "memory" clobber hold such loads behind the wait. Coherent
+// loads cost 2 % of the prep kernel's time in a loop (see there) and nothing that shows in the others.
 // What dependent launches are worth (us per pass in a loop, before -> after): B1 N256 D64 forward 8.3 -> 7.0, rotary twice
 // and attention of a 1511-token prompt 43.2 -> 38.3, one-token append and decode 16.4 -> 12.2.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
