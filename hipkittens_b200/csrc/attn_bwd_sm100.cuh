@@ -120,9 +120,10 @@ static_assert(BwdSmem<128>::kDynBytes <= 232448, "shared memory budget of one CT
 // ------------------------------------------------------------------------------------ delta = rowsum(dO * O)
 // D/8 lanes per (batch, position, head) row, 16 bytes of O and of dO per lane; bound by HBM (O and dO are read once).
 // A thread takes kRowPassUnroll rows and requests all of them before it reduces the first: with one row per thread
-// the 32 bytes a thread had in flight left HBM at 5.6 TB/s (B16 N2048 H64 D128, 1.07 GB: 191 us in a loop, 199 alone),
-// with four it reads 6.9 TB/s (154 and 156 us). Streaming loads, without a branch around them: as plain ones behind one
-// they took 158 and 163 us, as non-coherent ones 151 and 159 (which ptx::grid_dep_wait rules out). grid = ceil(rows / row_pass_rows(D / 8)), block = 256.
+// the 32 bytes a thread had in flight left HBM at 5.6 TB/s (B16 N2048 H64 D128, 1.07 GB: 190 us in a loop, 198 alone),
+// with four it reads 7.0 TB/s (152 and 153 us; B4 N2048: 51 -> 41 and 58 -> 48). Streaming loads, without a branch around
+// them, and stores behind them all: plain loads behind a branch took 154 to 158 and 163 us, non-coherent ones 151 and
+// 159 (which ptx::grid_dep_wait rules out). grid = ceil(rows / row_pass_rows(D / 8)), block = 256.
 constexpr int kRowPassUnroll = 4;
 __host__ __device__ constexpr int row_pass_rows(int lanes_per_row) { return 8 * (32 / lanes_per_row) * kRowPassUnroll; }
 
@@ -145,9 +146,9 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
     a[u] = __ldcs(reinterpret_cast<const uint4*>(o + static_cast<size_t>(row) * D) + sub);
     b[u] = __ldcs(reinterpret_cast<const uint4*>(d_o + static_cast<size_t>(row) * D) + sub);
   }
+  float sum[kRowPassUnroll];
 #pragma unroll
   for (int u = 0; u < kRowPassUnroll; ++u) {
-    const int row = row0 + u * kRowsPerWarp;
     const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w};
     const uint32_t bw[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
     float acc = 0.f;
@@ -160,11 +161,16 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
     }
 #pragma unroll
     for (int off = kLanesPerRow / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    sum[u] = acc;
+  }
+#pragma unroll
+  for (int u = 0; u < kRowPassUnroll; ++u) {  // behind all loads: a store among them would hold the later ones back
+    const int row = row0 + u * kRowsPerWarp;
     if (row < rows && sub == 0) {
       int bn, h, bi, n;
       fd_h.divmod(row, bn, h);
       fd_n.divmod(bn, bi, n);
-      delta[(static_cast<size_t>(bi) * H + h) * N + n] = acc;
+      delta[(static_cast<size_t>(bi) * H + h) * N + n] = sum[u];
     }
   }
 }
