@@ -5,7 +5,8 @@
 and L [B,H,1,N] fp32 are allocated here, O is returned in the input dtype and (q, k, v, O, L) are saved for the backward
 pass. Like the reference's ``tk_kernel_fwd.dispatch_fwd`` and its three backward calls (hipkittens.py:64-119), forward
 and backward each return when the device is done and raise if a kernel reported a failure; they synchronise once for
-that, not after each kernel.
+that, not after each kernel. A ``key_padding_mask`` is looked at on the device, and its verdict is read, by one more
+synchronisation, behind the forward: a mask that cannot be honoured raises after the kernels have run on clamped lengths.
 
 Differences: bf16 tensors are read through strided TMA descriptors and gradients written through strides, so there are
 no ``.contiguous()`` copies of q, k and v (hipkittens.py:37-39) in either direction, and the modules' packed
@@ -136,7 +137,7 @@ def _attend(q, packed, causal, softmax_scale, key_padding_mask):
     else:
         views = packed.unbind(dim=2) if q is None else (q, *packed.unbind(dim=2))
         out = HipAttnFunction.apply(*views, causal, softmax_scale, kv_lens)
-    # read here, behind the forward's own synchronisation: whatever the mask, the lengths are clamped by the kernels
+    # read here, when the forward is done and this does not wait for it: whatever the mask, the kernels clamp the lengths
     if bad is not None and int(bad) != 0:
         raise ValueError(_BAD_MASK)
     return out.to((packed if q is None else q).dtype).contiguous()
