@@ -63,6 +63,7 @@ struct DeviceState {
   bool ready = false;     // set once init_device succeeded; a failed attempt is retried by the next call
   int sm_count = 0;
   int cc_major = 0;
+  hk::DecodeLimits decode;
   int* status = nullptr;       // the status word, device address (kernels write it only when something went wrong)
   int* status_host = nullptr;  // ... and host address: mapped memory, so that reading it needs no copy
 };
@@ -156,7 +157,7 @@ int init_device(int device) {
   if ((rc = prepare_fwd_kernels<128, true>()) != HK_OK) return rc;
   if ((rc = prepare_fwd_kernels<64, false>()) != HK_OK) return rc;
   if ((rc = prepare_fwd_kernels<64, true>()) != HK_OK) return rc;
-  if ((rc = hk::prepare_decode_kernels(g_cuda_err, sizeof(g_cuda_err))) != HK_OK) return rc;
+  if ((rc = hk::prepare_decode_kernels(g_cuda_err, sizeof(g_cuda_err), st.sm_count, &st.decode)) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<128, false>()) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<128, true>()) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<64, false>()) != HK_OK) return rc;
@@ -822,7 +823,7 @@ int hk_attn_paged_decode(const void* q, const void* k_pages, const void* v_pages
   p.workspace = workspace;
   p.status = st->status;
   int launched = 0;
-  cudaError_t e = hk::launch_paged_decode(p, st->sm_count, static_cast<cudaStream_t>(cuda_stream), &launched);
+  cudaError_t e = hk::launch_paged_decode(p, st->decode, static_cast<cudaStream_t>(cuda_stream), &launched);
   g_launches.fetch_add(launched, std::memory_order_relaxed);
   if (e != cudaSuccess) return cuda_fail(e, "paged decode launch");
   return HK_OK;
@@ -996,6 +997,7 @@ struct StaticDecodeState {
   std::mutex mu;
   bool ready = false;       // a failed set-up is retried by the next call
   int sm_count = 0;
+  hk::DecodeLimits decode;
   void* scratch = nullptr;  // device address of g_decode_static_scratch on this device
   int* status = nullptr;    // device address of g_decode_static_status on this device
 };
@@ -1018,7 +1020,7 @@ int init_static_decode(int device) {
     snprintf(g_cuda_err, sizeof(g_cuda_err), "static decode scratch has no usable device address");
     return HK_ECUDA;
   }
-  return hk::prepare_decode_kernels(g_cuda_err, sizeof(g_cuda_err));
+  return hk::prepare_decode_kernels(g_cuda_err, sizeof(g_cuda_err), st.sm_count, &st.decode);
 }
 
 }  // namespace
@@ -1079,7 +1081,7 @@ extern "C" int hk_attn_paged_decode_static(const void* q, const void* k_pages, c
   p.workspace = st.scratch;  // the looked-up device address, never the host-side symbol
   p.status = st.status;
   int launched = 0;
-  cudaError_t e = hk::launch_paged_decode(p, st.sm_count, stream, &launched);
+  cudaError_t e = hk::launch_paged_decode(p, st.decode, stream, &launched);
   g_launches.fetch_add(launched, std::memory_order_relaxed);
   if (e != cudaSuccess) return cuda_fail(e, "paged decode launch");
   if (status_out) {

@@ -2,14 +2,16 @@
 // reached through a block table. The reference has no such kernel; the math is the forward's
 // (kernels/attn/gqa/kernel.cpp:569-573 for L) applied to one query row that sees its whole context.
 //
-// Split-K layout: a CTA owns a chunk of 512 or 1024 consecutive tokens of one (sequence, kv head) and all
-// G = H / H_KV query heads of that kv head, so every K/V byte of the context is read exactly once.
-// Inside the CTA each of the 4 warps streams its own pages (page w, w+4, ...) through a private
-// cp.async ring of 16-byte copies; scores and the PV product run on mma.sync m16n8k16 (bf16, fp32
-// accumulate) with the G heads in the 16-row M dimension, which is far more than an HBM-bound kernel
-// needs and keeps the CUDA cores free for address generation and the exponentials.
-// Sequences that fit one chunk are finished in place; longer ones leave per-chunk (O, m, l) partials
-// in the workspace, which `paged_decode_combine_kernel` merges.
+// Split-K layout: a CTA owns part of the context of one (sequence, kv head) and all G = H / H_KV query heads of that kv
+// head, so every K/V byte of the context is read exactly once. Inside the CTA each of the 4 or 8 warps streams its own
+// pages through a private cp.async ring of 16-byte copies; scores and the PV product run on mma.sync m16n8k16 (bf16,
+// fp32 accumulate) with the G heads in the 16-row M dimension, which is far more than an HBM-bound kernel needs and keeps
+// the CUDA cores free for address generation and the exponentials.
+// The CTAs of one (sequence, kv head) are a cluster, which splits the context evenly whatever its length and merges the
+// partial results through distributed shared memory: one launch, nothing in the workspace. Where that would leave the GPU
+// to a few CTAs (decode_pick_shape), a CTA takes a chunk of 512 or 1024 consecutive tokens instead; contexts of one chunk
+// are finished in place, longer ones leave per-chunk (O, m, l) partials in the workspace, which
+// `paged_decode_combine_kernel` merges.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -25,13 +27,12 @@ constexpr int kPageTokens = 16;
 constexpr int kDecodeD = 128;
 constexpr int kChunkPagesMin = 32;                    // pages per CTA: 32 (512 tokens) or 64 (1024 tokens),
 constexpr int kChunkPagesMax = 64;                    // chosen per launch by decode_pick_chunk_pages
-constexpr int kDecodeWarps = 4;
-constexpr int kDecodeThreads = kDecodeWarps * 32;
 constexpr int kDecodeStages = 3;                      // pages in flight per warp
 constexpr int kSlabBytes = kPageTokens * kDecodeD * 2;   // one page of one kv head: 4 KB
 constexpr int kStageBytes = 2 * kSlabBytes;           // K slab + V slab
-constexpr int kDecodeSmemBytes = kDecodeWarps * kDecodeStages * kStageBytes;  // 96 KB
+constexpr int decode_smem_bytes(int warps) { return warps * kDecodeStages * kStageBytes; }  // 96 or 192 KB
 constexpr int kMaxCombineSplits = 256;
+constexpr int kMaxCluster = 16;
 
 enum : int { kStatusBadPage = 2, kStatusBadLen = 4 };  // 3 is the backward kernels' kStatusSmemAlign
 
@@ -54,12 +55,59 @@ struct DecodeParams {
 __host__ __device__ inline int decode_max_splits(int max_pages) {
   return (max_pages + kChunkPagesMin - 1) / kChunkPagesMin;
 }
-// 1024-token chunks halve the partial results and were measured 4-5 % faster on the 64-sequence workload
+// Chunks: 1024-token chunks halve the partial results and were measured 4-5 % faster on the 64-sequence workload
 // (94.5 % vs 90.7 % of the copy bandwidth); 512-token chunks keep more CTAs in flight when the batch is
 // small. Take the large chunk when it still gives every SM two rounds of two CTAs.
 inline int decode_pick_chunk_pages(int S, int H_KV, int max_pages, int sm_count) {
   const long long ctas = 1ll * S * H_KV * ((max_pages + kChunkPagesMax - 1) / kChunkPagesMax);
   return ctas >= 4ll * sm_count ? kChunkPagesMax : kChunkPagesMin;
+}
+// What the device holds at once of the split kernel, by the size of its clusters (filled by prepare_decode_kernels).
+struct DecodeLimits {
+  int sm_count = 0;
+  int clusters4[kMaxCluster + 1] = {};  // clusters of so many CTAs of 4 warps (two per SM)
+  int clusters8 = 0;                    // clusters of kMaxCluster CTAs of 8 warps (one per SM)
+};
+
+// How the context of one (sequence, kv head), a unit, is spread: over a cluster of CTAs of 4 or 8 warps, or, with
+// cluster = 0, over chunks that a second kernel combines. The host knows the block table's width and not the contexts;
+// clusters spread each context evenly, so the width matters only for the most that one CTA may meet.
+//  * Clusters as large as keeps all units in one wave, and no larger: a cluster behind the first wave starts when a whole
+//    one fits, and one size too many costs more than it gives. us, chunks / clusters of that size / of another, H_KV 8 unless
+//    said: 1 x 3250 tokens 10.4 / 7.6 (16) / 8.0 (8); 4 x 750 10.1 / 6.3 (8) / 6.7 (4), 11.4 (16); 8 x 2500 20.6 / 17.0
+//    (4) / 22.6 (2), 19.0 (8); 40 x 1650 of H_KV 1 13.3 / 10.9 (6) / 14.1 (7).
+//  * Units for more than a wave in clusters of 3: CTAs of their own, of 8 warps while one per SM is enough or contexts may be
+//    above 1024 tokens: 16 x 1250 20.5 / 15.0, 32 x 600 18.8 / 14.5 (8 warps: 15.0), 64 x 300 21.1 / 16.6 (21.7), 32 x 2000
+//    52.4 / 45.1 (4 warps: 48.3). Clusters of several waves gain up to 5 % on long contexts (64 x 4350: 182 / 174 in
+//    clusters of 4), but where most of the table's width is empty their idle CTAs cost more than those of the chunks (64 x 300
+//    tokens in tables for 8192: 24 / 47), so those stay in chunks.
+//  * Few units with long contexts: 16 CTAs of 4 warps fall behind the chunks from some 700 tokens each on (1 x 14000 13.5 /
+//    14.7); up to 6 units the CTAs can have 8 warps (H_KV 1, 1 x 16000: 11.7 / 11.0, 4 warps 12.5; below 4096 tokens 4
+//    warps are better, 1 x 2000: 9.4 / 5.4, 8 warps 6.2).
+//  * One long context among short ones is shared by its own cluster only (12.5 us per 1000 tokens of a CTA of 4 warps, 5.5
+//    with 8), where chunks would spread it over the GPU (1 x 2000 beside 31 x 100: 10.6 / 14.0); so no more than 2048 (2560)
+//    tokens per CTA.
+struct DecodeShape {
+  int cluster, warps;
+};
+inline DecodeShape decode_pick_shape(int S, int H_KV, int max_pages, const DecodeLimits& lim) {
+  const long long units = 1ll * S * H_KV;
+  constexpr DecodeShape kChunks{0, 4};
+  int cluster = kMaxCluster, warps = 4;
+  while (cluster > 1 && lim.clusters4[cluster] < units) --cluster;
+  if (cluster < 3) {
+    cluster = 1;
+    warps = units <= lim.sm_count || max_pages > 64 ? 8 : 4;
+    if (max_pages > 160) return kChunks;
+  } else if (max_pages > 256 && units <= lim.clusters8) {
+    cluster = kMaxCluster;
+    warps = 8;
+    if (max_pages > 64 * cluster) return kChunks;
+  } else if (max_pages > (cluster == kMaxCluster ? 44 : 128) * cluster) {
+    return kChunks;
+  }
+  const int useful = (max_pages + warps - 1) / warps;  // a page per warp
+  return {cluster < useful ? cluster : useful, warps};
 }
 // Workspace: partial O as fp32 [S][H][splits][128], then (m, l) pairs as fp32 [S][H][splits][2].
 // Shapes the two kernels can be launched for: the combine kernel holds one weight per split in shared memory
@@ -108,11 +156,26 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// Cluster barrier (threads that have left are not waited for) and reads of another CTA's shared memory.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
 }  // namespace dec
 
-// grid = (max_splits, H_KV, S), block = 128 threads, dynamic smem = kDecodeSmemBytes.
-template <int G>
-__global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(const DecodeParams p) {
+// grid = (max_splits, H_KV, S), or (cluster size, H_KV, S) in clusters along x; block = 32 W threads, dynamic smem =
+// decode_smem_bytes(W).
+template <int G, bool CLUSTER, int W>
+__global__ void __launch_bounds__(W * 32, W == 8 ? 1 : 2) paged_decode_split_kernel(const DecodeParams p) {
   using namespace dec;
   extern __shared__ __align__(128) uint8_t dsmem[];
   ptx::grid_dep_wait();
@@ -125,22 +188,39 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(c
     ctx = p.max_pages * kPageTokens;
     if (threadIdx.x == 0) atomicCAS(p.status, 0, kStatusBadLen);
   }
-  const int chunk_tokens = p.chunk_pages * kPageTokens;
-  const int tok0 = split * chunk_tokens;
-  if (tok0 >= ctx) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int total_pages = (ctx + kPageTokens - 1) / kPageTokens;
-  const int page0 = split * p.chunk_pages;
-  const int chunk_pages = min(p.chunk_pages, total_pages - page0);
-  // this warp's pages: page0 + warp + 4*i
-  const int my_pages = (chunk_pages - warp + kDecodeWarps - 1) / kDecodeWarps;
+  // This warp's pages: page_first, page_first + page_step, ... below page_end. A CTA of a cluster takes every n_used-th
+  // group of four, so that whatever the length the live CTAs of a cluster differ by a page per warp at most.
+  int n_used, page_first, page_step, page_end;
+  if constexpr (CLUSTER) {
+    if (ctx <= 0) {  // defined output for an empty context
+      if (split == 0) {
+        for (int i = threadIdx.x; i < G * kDecodeD; i += W * 32)
+          p.o[(size_t(seq) * p.H + kvh * G) * kDecodeD + i] = __float2bfloat16(0.f);
+        if (threadIdx.x < G) p.lse[size_t(seq) * p.H + kvh * G + threadIdx.x] = -INFINITY;
+      }
+      return;
+    }
+    n_used = min(static_cast<int>(gridDim.x), (total_pages + W - 1) / W);  // a page for every warp of a live CTA
+    if (split >= n_used) return;  // the cluster's barriers count the threads that are left
+    page_first = split * W + warp;
+    page_step = n_used * W;
+    page_end = total_pages;
+  } else {
+    if (split * p.chunk_pages * kPageTokens >= ctx) return;
+    n_used = 1;
+    page_first = split * p.chunk_pages + warp;
+    page_step = W;
+    page_end = min(split * p.chunk_pages + p.chunk_pages, total_pages);
+  }
   const float c = p.scale_log2;
 
-  // page ids of this warp, one per lane (at most kChunkPagesMax / 4 = 16 are used)
+  // page ids of this warp, one per lane: no warp has more than 32 pages (decode_pick_shape and the chunk sizes see to it)
   int my_id = 0;
-  if (lane < my_pages) {
-    my_id = p.block_table[size_t(seq) * p.max_pages + page0 + warp + kDecodeWarps * lane];
+  if (const int page = page_first + lane * page_step; page < page_end) {
+    my_id = p.block_table[size_t(seq) * p.max_pages + page];
     if (my_id < 0 || my_id >= p.num_pages) {
       atomicCAS(p.status, 0, kStatusBadPage);  // never dereference an id outside the pool
       my_id = 0;
@@ -167,7 +247,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(c
   // chunks (16 tokens x 16 chunks) of K and of V; chunk index is XOR-swizzled with the token so that
   // ldmatrix reads are bank-conflict free.
   auto fetch = [&](int i) {
-    if (i < my_pages) {
+    if (page_first + i * page_step < page_end) {
       const int id = __shfl_sync(0xffffffffu, my_id, i);
       const size_t base = (size_t(id) * kPageTokens) * row_elems + size_t(kvh) * kDecodeD;
       const uint32_t st = ring + (i % kDecodeStages) * kStageBytes;
@@ -192,16 +272,18 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(c
 #pragma unroll
   for (int i = 0; i < kDecodeStages - 1; ++i) fetch(i);
 
-  for (int i = 0; i < my_pages; ++i) {
+  for (int i = 0, page = page_first; page < page_end; ++i, page += page_step) {
     fetch(i + kDecodeStages - 1);
     cp_async_wait<kDecodeStages - 1>();
     __syncwarp();
     const uint32_t sK = ring + (i % kDecodeStages) * kStageBytes;
     const uint32_t sV = sK + kSlabBytes;
 
-    // ---- S[16 x 16 tokens] = Q K^T
+    // ---- S[16 x 16 tokens] = Q K^T, in two halves of the head dimension: a warp has one page at a time, and with one
+    // accumulator per 8 tokens the eight products on it wait for one another
     float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     {
+      float sd[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
       const int mi = lane >> 3, r = lane & 7;
       const int tok = r + 8 * (mi >> 1);
 #pragma unroll
@@ -209,12 +291,17 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(c
         const int ch = ks * 2 + (mi & 1);
         uint32_t b0, b1, b2, b3;
         ldmatrix_x4(sK + tok * 256 + ((ch ^ (tok & 7)) << 4), b0, b1, b2, b3);
-        mma_16816(sc[0], qa[ks][0], 0u, qa[ks][1], 0u, b0, b1);
-        mma_16816(sc[1], qa[ks][0], 0u, qa[ks][1], 0u, b2, b3);
+        mma_16816(ks & 1 ? sd[0] : sc[0], qa[ks][0], 0u, qa[ks][1], 0u, b0, b1);
+        mma_16816(ks & 1 ? sd[1] : sc[1], qa[ks][0], 0u, qa[ks][1], 0u, b2, b3);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        sc[0][e] += sd[0][e];
+        sc[1][e] += sd[1][e];
       }
     }
     // ---- online softmax over this page (row g, tokens nt*8 + 2t + {0,1})
-    const int tok_base = (page0 + warp + kDecodeWarps * i) * kPageTokens;
+    const int tok_base = page * kPageTokens;
     float sv[4] = {sc[0][0], sc[0][1], sc[1][0], sc[1][1]};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -266,8 +353,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(c
   // ---- merge the 4 warps through shared memory (the ring is idle now)
   __syncthreads();
   float* sm_o = reinterpret_cast<float*>(dsmem);                    // [4][8][128]
-  float* sm_m = sm_o + kDecodeWarps * 8 * kDecodeD;                 // [4][8]
-  float* sm_l = sm_m + kDecodeWarps * 8;                            // [4][8]
+  float* sm_m = sm_o + W * 8 * kDecodeD;                 // [4][8]
+  float* sm_l = sm_m + W * 8;                            // [4][8]
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     float2 v2 = make_float2(oacc[j][0], oacc[j][1]);
@@ -278,34 +365,95 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) paged_decode_split_kernel(c
     sm_l[warp * 8 + g] = l;
   }
   __syncthreads();
-  const int d = threadIdx.x;  // 128 threads <-> 128 output columns
-  const int n_splits = (ctx + chunk_tokens - 1) / chunk_tokens;
+  // 128 threads <-> 128 output columns; with 8 warps each half of them takes every other head of the group
+  constexpr int kHalves = W / 4, kHeads = (G + kHalves - 1) / kHalves;
+  const int d = threadIdx.x & (kDecodeD - 1), h0 = threadIdx.x / kDecodeD;
+  // per head of this thread: reference maximum, row sum and this thread's column of the CTA's share
+  float M[kHeads], L[kHeads], acc[kHeads];
+#pragma unroll
+  for (int i = 0; i < kHeads; ++i) {
+    const int h = min(i * kHalves + h0, G - 1);
+    M[i] = sm_m[h];
+#pragma unroll
+    for (int w = 1; w < W; ++w) M[i] = fmaxf(M[i], sm_m[w * 8 + h]);
+    acc[i] = L[i] = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const float wgt = ptx::ex2_approx((sm_m[w * 8 + h] - M[i]) * c);
+      acc[i] += wgt * sm_o[(w * 8 + h) * kDecodeD + d];
+      L[i] += wgt * sm_l[w * 8 + h];
+    }
+  }
+  if constexpr (CLUSTER) {
+    if (n_used > 1) {
+      // ---- merge the CTAs of the cluster: each leaves its share in its own shared memory, and CTA r reads all of
+      // head r, r + n_used, ... in the order of the ranks
+      float* cl_o = sm_l + W * 8;          // [G][128]
+      float* cl_ml = cl_o + 8 * kDecodeD;  // [G][2]
+#pragma unroll
+      for (int i = 0; i < kHeads; ++i) {
+        const int h = i * kHalves + h0;
+        if (h >= G) break;
+        cl_o[h * kDecodeD + d] = acc[i];
+        if (d == 0) {
+          cl_ml[2 * h] = M[i];
+          cl_ml[2 * h + 1] = L[i];
+        }
+      }
+      cluster_arrive();
+      cluster_wait();
+      for (int h = split * kHalves + h0; h < G; h += n_used * kHalves) {
+        float m_r[kMaxCluster], l_r[kMaxCluster], o_r[kMaxCluster];
+        const uint32_t a_ml = ptx::smem_u32(cl_ml + 2 * h), a_o = ptx::smem_u32(cl_o + h * kDecodeD + d);
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r) {
+          m_r[r] = -INFINITY;
+          l_r[r] = o_r[r] = 0.f;
+          if (r < n_used) {
+            const uint32_t ml = map_to_rank(a_ml, r);
+            m_r[r] = ld_cluster(ml);
+            l_r[r] = ld_cluster(ml + 4);
+            o_r[r] = ld_cluster(map_to_rank(a_o, r));
+          }
+        }
+        float Mc = m_r[0];
+#pragma unroll
+        for (int r = 1; r < kMaxCluster; ++r) Mc = fmaxf(Mc, m_r[r]);
+        float sum = 0.f, out = 0.f;
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r) {
+          const float wgt = ptx::ex2_approx((m_r[r] - Mc) * c);
+          sum += wgt * l_r[r];
+          out += wgt * o_r[r];
+        }
+        const size_t row = size_t(seq) * p.H + kvh * G + h;
+        p.o[row * kDecodeD + d] = __float2bfloat16(out / sum);
+        if (d == 0) p.lse[row] = Mc * p.scale + __logf(sum);
+      }
+      cluster_arrive();  // nobody leaves while its shared memory is being read
+      cluster_wait();
+      return;
+    }
+  }
+  const int n_splits = CLUSTER ? 1 : (total_pages + p.chunk_pages - 1) / p.chunk_pages;
   const int max_splits = decode_max_splits(p.max_pages);
   float* ws_o = reinterpret_cast<float*>(p.workspace);
   const size_t o_bytes = (size_t(p.S) * p.H * max_splits * kDecodeD * sizeof(float) + 255) & ~size_t(255);
   float* ws_ml = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.workspace) + o_bytes);
 #pragma unroll
-  for (int h = 0; h < G; ++h) {
-    float M = sm_m[h];
-#pragma unroll
-    for (int w = 1; w < kDecodeWarps; ++w) M = fmaxf(M, sm_m[w * 8 + h]);
-    float acc = 0.f, lsum = 0.f;
-#pragma unroll
-    for (int w = 0; w < kDecodeWarps; ++w) {
-      const float wgt = ptx::ex2_approx((sm_m[w * 8 + h] - M) * c);
-      acc += wgt * sm_o[(w * 8 + h) * kDecodeD + d];
-      lsum += wgt * sm_l[w * 8 + h];
-    }
-    const int head = kvh * G + h;
+  for (int i = 0; i < kHeads; ++i) {
+    const int h = i * kHalves + h0;
+    if (h >= G) break;
+    const size_t row = size_t(seq) * p.H + kvh * G + h;
     if (n_splits == 1) {
-      p.o[(size_t(seq) * p.H + head) * kDecodeD + d] = __float2bfloat16(acc / lsum);
-      if (d == 0) p.lse[size_t(seq) * p.H + head] = M * p.scale + __logf(lsum);
+      p.o[row * kDecodeD + d] = __float2bfloat16(acc[i] / L[i]);
+      if (d == 0) p.lse[row] = M[i] * p.scale + __logf(L[i]);
     } else {
-      const size_t slot = (size_t(seq) * p.H + head) * max_splits + split;
-      ws_o[slot * kDecodeD + d] = acc;
+      const size_t slot = row * max_splits + split;
+      ws_o[slot * kDecodeD + d] = acc[i];
       if (d == 0) {
-        ws_ml[slot * 2] = M;
-        ws_ml[slot * 2 + 1] = lsum;
+        ws_ml[slot * 2] = M[i];
+        ws_ml[slot * 2 + 1] = L[i];
       }
     }
   }
@@ -360,36 +508,79 @@ __global__ void __launch_bounds__(kDecodeD) paged_decode_combine_kernel(const De
   if (d == 0) p.lse[size_t(seq) * p.H + head] = s_M * p.scale + __logf(s_L);
 }
 
-inline int prepare_decode_kernels(char* err, size_t err_len) {
-  cudaError_t e;
-#define HK_PREP(G)                                                                                      \
-  e = cudaFuncSetAttribute(paged_decode_split_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                           kDecodeSmemBytes);                                                           \
-  if (e != cudaSuccess) {                                                                               \
-    snprintf(err, err_len, "decode kernel attribute: %s", cudaGetErrorString(e));                       \
-    return -3;                                                                                          \
+template <int G, bool CLUSTER, int W>
+cudaError_t prepare_decode_kernel() {
+  auto* fn = paged_decode_split_kernel<G, CLUSTER, W>;
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem_bytes(W));
+  if (e != cudaSuccess || !CLUSTER) return e;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+template <int G>
+cudaError_t prepare_decode_kernels_of() {
+  cudaError_t e = prepare_decode_kernel<G, false, 4>();
+  if (e == cudaSuccess) e = prepare_decode_kernel<G, true, 4>();
+  if (e == cudaSuccess) e = prepare_decode_kernel<G, true, 8>();
+  return e;
+}
+// Clusters of n CTAs that the current device holds at once (0: not even one, as on a slice of a GPU).
+template <typename Kernel>
+int clusters_held(Kernel* fn, int warps, int n) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n);
+  cfg.blockDim = dim3(warps * 32);
+  cfg.dynamicSmemBytes = decode_smem_bytes(warps);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = n;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int held = 0;
+  if (cudaOccupancyMaxActiveClusters(&held, fn, &cfg) == cudaSuccess) return held;
+  cudaGetLastError();
+  return 0;
+}
+inline int prepare_decode_kernels(char* err, size_t err_len, int sm_count, DecodeLimits* lim) {
+  for (auto* prepare : {prepare_decode_kernels_of<1>, prepare_decode_kernels_of<2>, prepare_decode_kernels_of<3>,
+                        prepare_decode_kernels_of<4>, prepare_decode_kernels_of<5>, prepare_decode_kernels_of<6>,
+                        prepare_decode_kernels_of<7>, prepare_decode_kernels_of<8>}) {
+    const cudaError_t e = prepare();
+    if (e != cudaSuccess) {
+      snprintf(err, err_len, "decode kernel attribute: %s", cudaGetErrorString(e));
+      return -3;
+    }
   }
-  HK_PREP(1) HK_PREP(2) HK_PREP(3) HK_PREP(4) HK_PREP(5) HK_PREP(6) HK_PREP(7) HK_PREP(8)
-#undef HK_PREP
+  lim->sm_count = sm_count;
+  for (int n = 2; n <= kMaxCluster; ++n) lim->clusters4[n] = clusters_held(paged_decode_split_kernel<8, true, 4>, 4, n);
+  lim->clusters8 = clusters_held(paged_decode_split_kernel<8, true, 8>, 8, kMaxCluster);
   return 0;
 }
 
-inline cudaError_t launch_paged_decode(DecodeParams p, int sm_count, cudaStream_t stream, int* launched) {
-  p.chunk_pages = decode_pick_chunk_pages(p.S, p.H_KV, p.max_pages, sm_count);
+template <int G>
+cudaError_t launch_decode_split(const DecodeParams& p, int splits, int cluster, int warps, cudaStream_t stream) {
+  const dim3 grid(cluster ? cluster : splits, p.H_KV, p.S);
+  if (cluster == 0)
+    return launch_dependent(true, paged_decode_split_kernel<G, false, 4>, grid, 128, decode_smem_bytes(4), stream, p);
+  auto* fn = warps == 8 ? paged_decode_split_kernel<G, true, 8> : paged_decode_split_kernel<G, true, 4>;
+  return launch_dependent(true, fn, grid, warps * 32, decode_smem_bytes(warps), stream, ClusterX{unsigned(cluster)}, p);
+}
+
+inline cudaError_t launch_paged_decode(DecodeParams p, const DecodeLimits& lim, cudaStream_t stream, int* launched) {
+  const DecodeShape shape = decode_pick_shape(p.S, p.H_KV, p.max_pages, lim);
+  const int cluster = shape.cluster, warps = shape.warps;
+  p.chunk_pages = decode_pick_chunk_pages(p.S, p.H_KV, p.max_pages, lim.sm_count);
   const int splits = (p.max_pages + p.chunk_pages - 1) / p.chunk_pages;
   if (splits > kMaxCombineSplits) return cudaErrorInvalidValue;
-  const dim3 grid(splits, p.H_KV, p.S);
-  const int G = p.H / p.H_KV;
   cudaError_t e;
-  switch (G) {
+  switch (p.H / p.H_KV) {
 #define HK_CASE(g) \
-  case g: e = launch_dependent(true, paged_decode_split_kernel<g>, grid, kDecodeThreads, kDecodeSmemBytes, stream, p); break;
+  case g: e = launch_decode_split<g>(p, splits, cluster, warps, stream); break;
     HK_CASE(1) HK_CASE(2) HK_CASE(3) HK_CASE(4) HK_CASE(5) HK_CASE(6) HK_CASE(7) HK_CASE(8)
 #undef HK_CASE
     default: return cudaErrorInvalidValue;
   }
   *launched += 1;
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || cluster) return e;
   e = launch_dependent(true, paged_decode_combine_kernel, dim3(p.H, p.S), kDecodeD, 0, stream, p);
   *launched += 1;
   return e;
