@@ -81,6 +81,7 @@ struct BwdParams {
   FastDiv fd_group;     // causal: items of a full group
   FastDiv fd_in_grp, fd_in_grp_last;  // causal: items per key block / query tile in a full group, in the last group
   int n_pairs;          // causal dK/dV kernel: pairs of key blocks (j, NBK - 1 - j) over all units; 0: single blocks
+  int dq_waits;         // dQ kernel: starts its work only when the dK/dV kernel has ended
   FastDiv fd_pairs;     // pairs per unit, (NBK + 1) / 2; single blocks: units
   float scale;
   float scale_log2;
@@ -1008,7 +1009,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   volatile uint32_t* abortp = abort_word;
-  grid_dep_wait();
+  // Launched as a dependent of the dK/dV kernel, which it does not read from: its CTAs take over the SMs as that kernel
+  // leaves them. What both read is complete, because the dK/dV kernel has waited for it before it let this one start.
+  // The wait for the dK/dV kernel is the last thing a CTA does, so that who waits for this kernel waits for both.
+  if (p.dq_waits) grid_dep_wait();
   grid_dep_launch();
   // TMEM columns: S [0,128)  dP [128,256)  dQ [256,256+D)  dS (bf16, 64 packed columns) [384,448).
   // Nothing aliases: S and dP are free for the next tile as soon as they are in registers.
@@ -1328,6 +1332,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     tc_fence_after();
     tmem_dealloc(tmem, kTmemCols);
   }
+  grid_dep_wait();
 }
 
 }  // namespace HK_BWD_NS

@@ -391,7 +391,8 @@ int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count) {
 
 template <int D, bool CAUSAL>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-               hk::BwdParams p, int B, int N, int NK, int H, int H_KV, int sm_count, cudaStream_t stream) {
+               hk::BwdParams p, int B, int N, int NK, int H, int H_KV, bool dq_beside, int sm_count,
+               cudaStream_t stream) {
   const int nbq = (N + hk::kBlockM - 1) / hk::kBlockM;   // query tiles
   const int nbk = (NK + hk::kBlockN - 1) / hk::kBlockN;  // key blocks
   if (static_cast<long long>(B) * H * nbq > 0x3fffffffll || static_cast<long long>(B) * H_KV * nbk > 0x3fffffffll)
@@ -406,13 +407,19 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   HK_CUDA(hk::launch_dependent(short_kernel(tiles, grid), Lay::template dkdv<D>(), grid, Lay::kThreads,
                                hk::BwdSmem<D>::kDynBytes, stream, tq, tk, tv, tdo, p));
   g_launches.fetch_add(1, std::memory_order_relaxed);
+  // The dQ kernel runs on the SMs that the dK/dV kernel leaves: us per backward in a loop, one after the other / so (D128
+  // unless said): B1 N512 H8/8 23.6 / 15.3, B2 N384 H8/2 causal 34.6 / 27.4, B2 N2000 H3/1 D64 86.9 / 69.0, B1 N1024 H8/1
+  // 121 / 109, B16 N2048 H64/8 6733 / 6648. Where few SMs are left (from three quarters of them taken on, in one round), the
+  // few CTAs that start early cost the longest dK/dV CTAs more than they give (B5 N300 H32/8 causal, 120 of 148:
+  // 53.3 / 61.4; B4, 96 of 148: 49.1 / 43.6).
+  p.dq_waits = !dq_beside || (grid < sm_count && 4 * grid > 3 * sm_count);
   p.n_items = B * H * nbq;
   grid = p.n_items < sm_count ? p.n_items : sm_count;
   set_bwd_decode(p, (H / H_KV) * nbq, H / H_KV, CAUSAL ? H / H_KV : nbq, grid, CAUSAL);
 #ifdef HK_TRACE
   p.trace = g_trace_bwd_kernel == 1 ? trace_buf : nullptr;
 #endif
-  HK_CUDA(hk::launch_dependent(short_kernel(tiles, grid), Lay::template dq<D>(), grid, Lay::kThreads,
+  HK_CUDA(hk::launch_dependent(!p.dq_waits || short_kernel(tiles, grid), Lay::template dq<D>(), grid, Lay::kThreads,
                                hk::BwdSmem<D>::kDynBytes, stream, tq, tk, tv, tdo, p));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return HK_OK;
@@ -611,6 +618,15 @@ struct BwdStrides {
   const long long *q, *k, *v, *dq, *dk, *dv;
 };
 
+// Whether two [B, N, H, D] tensors of 16-bit elements, given by address and strides, may share memory.
+static bool overlap(const void* a, const long long* a_strides, const void* b, const long long* b_strides, int B, int N, int H,
+                    int D) {
+  auto end = [&](const void* p, const long long* s) {
+    return reinterpret_cast<uintptr_t>(p) + 2 * ((B - 1) * s[0] + (N - 1) * s[1] + (H - 1) * s[2] + D);
+  };
+  return reinterpret_cast<uintptr_t>(a) < end(b, b_strides) && reinterpret_cast<uintptr_t>(b) < end(a, a_strides);
+}
+
 // Shared tail of the backward entries. o != null: delta is computed here first.
 static int bwd_launch(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse,
                       float* delta, void* dq, void* dk, void* dv, int B, int N, int NK, int H, int H_KV, int D,
@@ -669,10 +685,13 @@ static int bwd_launch(const void* q, const void* k, const void* v, const void* o
 #ifdef HK_TRACE
   p.trace = g_trace_buf;
 #endif
-  if (D == 128) return causal ? launch_bwd<128, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, st->sm_count, stream)
-                              : launch_bwd<128, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, st->sm_count, stream);
-  return causal ? launch_bwd<64, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, st->sm_count, stream)
-                : launch_bwd<64, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, st->sm_count, stream);
+  // The dQ kernel starts while the dK/dV kernel is still reading, unless it would write over what that reads: dQ in the place
+  // of Q or of dO is as good as anywhere else when one kernel follows the other.
+  const bool dq_beside = !overlap(dq, s.dq, q, s.q, B, N, H, D) && !overlap(dq, s.dq, d_o, dos, B, N, H, D);
+  if (D == 128) return causal ? launch_bwd<128, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, stream)
+                              : launch_bwd<128, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, stream);
+  return causal ? launch_bwd<64, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, stream)
+                : launch_bwd<64, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, stream);
 }
 
 int hk_attn_bwd_cross(const void* q, const void* k, const void* v, const void* d_o, const float* lse,

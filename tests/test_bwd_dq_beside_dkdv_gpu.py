@@ -1,0 +1,62 @@
+"""The dQ kernel runs beside the dK/dV kernel: whoever comes behind it waits for both, and dQ in the place of Q or dO is written
+when nobody reads those any more. Results are those of the two kernels one after the other, bit for bit."""
+import pytest
+import torch
+
+import hipkittens_b200 as hk
+from hipkittens_b200 import _native
+
+pytestmark = pytest.mark.gpu
+
+# few dK/dV CTAs, most SMs taken, more than a round of them; both layouts of the kernels
+SHAPES = [(1, 300, 8, 1, 128, True), (1, 512, 8, 8, 128, False), (2, 200, 6, 2, 64, False), (5, 300, 32, 8, 128, True),
+          (3, 700, 16, 16, 64, True)]
+
+
+def inputs(B, N, H, HK, D, causal):
+    gen = torch.Generator(device="cuda").manual_seed(N)
+
+    def rand(h):
+        return torch.randn((B, N, h, D), generator=gen, device="cuda", dtype=torch.bfloat16)
+
+    q, k, v, d_o = rand(H), rand(HK), rand(HK), rand(H)
+    o, lse = hk.attn_fwd(q, k, v, causal=causal)
+    return q, k, v, d_o, o, lse
+
+
+def backward(q, k, v, o, d_o, lse, dq, causal):
+    dk, dv = torch.empty_like(k), torch.empty_like(v)
+    _native.attn_bwd_strided(q, k, v, o, d_o, lse, dq, dk, dv, causal=causal)
+    return dq, dk, dv
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_dq_in_the_place_of_what_dkdv_reads(shape):
+    causal = shape[-1]
+    q, k, v, d_o, o, lse = inputs(*shape)
+    ref = [t.clone() for t in backward(q, k, v, o, d_o, lse, torch.empty_like(q), causal)]
+    for _ in range(5):
+        q2, d2 = q.clone(), d_o.clone()
+        for a, b in zip(backward(q2, k, v, o, d_o, lse, q2, causal), ref):
+            assert torch.equal(a, b)
+        for a, b in zip(backward(q, k, v, o, d2, lse, d2, causal), ref):
+            assert torch.equal(a, b)
+    assert _native.device_status(0) == 0
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_a_dependent_kernel_behind_it_finds_both_complete(shape):
+    B, N, H, HK, D, causal = shape
+    q, k, v, d_o, o, lse = inputs(*shape)
+    ref = [t.clone() for t in backward(q, k, v, o, d_o, lse, torch.empty_like(q), causal)]
+    ang = torch.arange(N, device="cuda")[:, None] / (1.0 + torch.arange(D // 2, device="cuda")[None])
+    cos, sin = ang.cos().bfloat16(), ang.sin().bfloat16()
+    want = [hk.rotary_bnhd(t, cos, sin) for t in ref]
+    for _ in range(10):
+        q2, k2 = q.clone(), k.clone()
+        dq, dk, dv = backward(q2, k2, v, o, d_o, lse, torch.empty_like(q), causal)
+        hk.rotary_bnhd(q2, cos, sin, out=q2)  # overwrites what both kernels read
+        hk.rotary_bnhd(k2, cos, sin, out=k2)
+        got = [hk.rotary_bnhd(t, cos, sin) for t in (dq, dk, dv)]
+        for a, b in zip((dq, dk, dv, *got), (*ref, *want)):
+            assert torch.equal(a, b)
