@@ -52,6 +52,8 @@ enum : int { kStatusSmemAlign = 3 };  // dynamic shared memory did not start on 
 #ifndef HK_BWD_EMU_CNT
 #define HK_BWD_EMU_CNT 1
 #endif
+constexpr int kMaxDkdvSplit = 8;  // CTAs that share a key block; larger clusters measured slower throughout
+
 constexpr int kBwdEmuMod = HK_BWD_EMU_MOD;
 constexpr int kBwdEmuCnt = HK_BWD_EMU_CNT;
 
@@ -81,6 +83,8 @@ struct BwdParams {
   FastDiv fd_group;     // causal: items of a full group
   FastDiv fd_in_grp, fd_in_grp_last;  // causal: items per key block / query tile in a full group, in the last group
   int n_pairs;          // causal dK/dV kernel: pairs of key blocks (j, NBK - 1 - j) over all units; 0: single blocks
+  int split;            // dK/dV kernel: CTAs of a cluster that share an item (1: none, and no clusters)
+  FastDiv fd_split;
   int dq_waits;         // dQ kernel: starts its work only when the dK/dV kernel has ended
   FastDiv fd_pairs;     // pairs per unit, (NBK + 1) / 2; single blocks: units
   float scale;
@@ -340,6 +344,28 @@ __device__ __forceinline__ void bwd_store_part_row(uint32_t taddr, __nv_bfloat16
   }
 }
 
+// The same columns, scaled, into a [128][D] fp32 tile in shared memory whose 16-byte units are exchanged inside a row by the
+// row's low bits, so that neither the rows of a warp here nor the units of a row there meet in a bank.
+template <int D>
+__device__ __forceinline__ void bwd_stage_part_row(uint32_t taddr, uint8_t* tile, int row, int part, float mul) {
+  constexpr int kCols = D / kBwdParts;
+  constexpr int kChunk = kCols >= 32 ? 32 : 16;
+#pragma unroll
+  for (int cc = 0; cc < kCols / kChunk; ++cc) {
+    uint32_t o[kChunk];
+    if constexpr (kChunk == 32) ptx::tmem_ld32(taddr + cc * 32, o);
+    else ptx::tmem_ld16(taddr, o);
+    ptx::tmem_wait_ld();
+#pragma unroll
+    for (int u = 0; u < kChunk / 4; ++u) {
+      const int unit = (part * kCols + cc * kChunk) / 4 + u;
+      *reinterpret_cast<float4*>(tile + row * (D * 4) + ((unit ^ (row & 7)) << 4)) =
+          make_float4(__uint_as_float(o[u * 4]) * mul, __uint_as_float(o[u * 4 + 1]) * mul,
+                      __uint_as_float(o[u * 4 + 2]) * mul, __uint_as_float(o[u * 4 + 3]) * mul);
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------ dK, dV
 struct DkdvItem {
   int b, kvh, j;   // batch, kv head, key block
@@ -350,7 +376,13 @@ struct DkdvItem {
   int cnt_i;       // query tiles per head this key block meets
   int n_iter;      // heads of the group x query tiles; 0 for a key block nobody sees (beyond kv_len, or causal
                    // with every query before it)
+  int n_first, n_end;    // this CTA's pairs: all of them, or its rank's share
+  int g_first, i_first;  // head and query tile of the first
+  int rank;
 };
+
+// First pair of rank r's share of n pairs.
+__device__ __forceinline__ int dkdv_share(int r, int ranks, int n) { return r * n / ranks; }
 
 // Work order: one (batch, kv head) unit's key blocks are adjacent so that the CTAs running at the same
 // time read the same Q / dO tiles from L2; an item index is unit * key blocks + key block.
@@ -360,8 +392,10 @@ struct DkdvItem {
 // (j, NBK - 1 - j) of the same unit, which all cost the same - a CTA's round 2r is the first block of its r-th pair and
 // round 2r + 1 the second (none for the middle block of an odd count) -, or singly (n_pairs = 0), the longest of all
 // units first, in snake order.
-template <bool CAUSAL>
-__device__ __forceinline__ int dkdv_item_for_round(const BwdParams& p, int round, int cta, int n_cta) {
+template <bool CAUSAL, bool SPLIT>
+__device__ __forceinline__ int dkdv_item_for_round(const BwdParams& p, int round) {
+  const int cta = SPLIT ? p.fd_split.div(blockIdx.x) : static_cast<int>(blockIdx.x);
+  const int n_cta = SPLIT ? p.n_items : static_cast<int>(gridDim.x);
   if (!CAUSAL) return item_for_round(p, round, cta, n_cta);
   if (p.n_pairs == 0) {
     const int k = round * n_cta + ((round & 1) ? n_cta - 1 - cta : cta);
@@ -380,7 +414,7 @@ __device__ __forceinline__ int dkdv_item_for_round(const BwdParams& p, int round
   return unit * nbk + j;
 }
 
-template <bool CAUSAL>
+template <bool CAUSAL, bool SPLIT>
 __device__ __forceinline__ DkdvItem decode_dkdv_item(const BwdParams& p, int idx) {
   DkdvItem w;
   const int NBQ = (p.N + kBlockM - 1) / kBlockM;   // query tiles
@@ -393,10 +427,24 @@ __device__ __forceinline__ DkdvItem decode_dkdv_item(const BwdParams& p, int idx
   w.i_min = CAUSAL ? max(w.j * kBlockN - w.off, 0) / kBlockM : 0;
   w.cnt_i = max(NBQ - w.i_min, 0);
   w.n_iter = (w.j * kBlockN >= w.kv_len) ? 0 : p.G * w.cnt_i;
+  w.n_first = w.g_first = w.i_first = w.rank = 0;
+  w.n_end = w.n_iter;
+  if constexpr (SPLIT) {
+    w.rank = static_cast<int>(blockIdx.x) - p.fd_split.div(blockIdx.x) * p.split;
+    w.n_first = dkdv_share(w.rank, p.split, w.n_iter);
+    w.n_end = dkdv_share(w.rank + 1, p.split, w.n_iter);
+    if (w.n_end > w.n_first) {
+      w.g_first = w.n_first / w.cnt_i;
+      w.i_first = w.n_first - w.g_first * w.cnt_i;
+    }
+  }
   return w;
 }
 
-template <int D, bool CAUSAL>
+// SPLIT: an item is shared by the CTAs of a cluster (p.split of them), each with its part of the (head, query tile) pairs; the
+// partial dK and dV are added up through distributed shared memory, row by row in the order of the ranks, so that the
+// gradients stay the same from run to run. One item per cluster and launch.
+template <int D, bool CAUSAL, bool SPLIT>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                      const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -407,6 +455,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   constexpr int kSub = SM::kSubTileBytes;
   constexpr int kChunks = D / 64;
   constexpr int RA = SM::kRingA, RB = SM::kRingB;
+  // In a cluster a CTA's own shared-memory addresses carry its rank above the 18 bits that a descriptor takes.
+  constexpr uint32_t kAddrMask = SPLIT ? 0x3ffffu : ~0u;
+  [[maybe_unused]] constexpr int kPartBytes = kBlockN * D * 4;  // SPLIT: partial dK, then dV, over the tiles
+  static_assert(2 * kPartBytes <= SM::kTiles * kTile, "the partial sums take the place of the tiles");
   enum { KV_FULL = 0, KV_EMPTY, ST_FULL, DP_FULL, P_FULL, DS_FULL, ACC_FULL, S_FREE, QA_FULL = 8, QA_EMPTY = 14,
          RB_FULL = 20, RB_EMPTY = 24, STAT_FULL = 28, STAT_EMPTY = 30, DP_FREE = 32, Y_FREE = 33, CTRL = 34 };
   static_assert(RA <= 6 && RB <= 4, "barrier slots");
@@ -502,12 +554,13 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #endif
     for (int round = 0; ok; ++round) {
       if (round >= p.total_rounds) break;
-      const int idx = dkdv_item_for_round<CAUSAL>(p, round, blockIdx.x, gridDim.x);
+      const int idx = dkdv_item_for_round<CAUSAL, SPLIT>(p, round);
       if (idx < 0) continue;  // a partial round leaves some CTAs without an item
-      const DkdvItem w = decode_dkdv_item<CAUSAL>(p, idx);
+      const DkdvItem w = decode_dkdv_item<CAUSAL, SPLIT>(p, idx);
       const bool pad_row = w.j * kBlockN + row >= w.kv_len;  // this key is padding (or lies beyond NK)
       const bool pad_block = (w.j + 1) * kBlockN > w.kv_len;  // uniform over the CTA: only such a block has padded keys
       if (w.n_iter == 0) {
+        if (SPLIT && w.rank != 0) continue;
         // nobody sees this key block (padding, or causal with every query before it): its gradients are zero and no
         // product was issued for it
         if (w.j * kBlockN + row < p.NK) {
@@ -522,7 +575,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         continue;
       }
       // i_rel: position of the pair's query tile among the cnt_i tiles of its head (n % cnt_i, without the division)
-      for (int n = 0, i_rel = 0; n < w.n_iter && ok; ++n, ++it, i_rel = (i_rel + 1 == w.cnt_i) ? 0 : i_rel + 1) {
+      if (SPLIT && w.n_first == w.n_end) continue;
+      for (int n = w.n_first, i_rel = w.i_first; n < w.n_end && ok; ++n, ++it, i_rel = (i_rel + 1 == w.cnt_i) ? 0 : i_rel + 1) {
         HK_STAMP(trole, 0);
         // a query tile the diagonal runs through: its first row does not see the block's last key (with an offset
         // that is not a multiple of the tile these are two tiles per head, else the one at the block's own position)
@@ -650,6 +704,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       if (!ok) break;
       ++acc_cnt;
       tc_fence_after();
+      if constexpr (SPLIT) {
+        bwd_stage_part_row<D>(tmem + lane_addr + cDK + part * (D / kBwdParts), bwd_smem, row, part, p.scale);
+        bwd_stage_part_row<D>(tmem + lane_addr + cDV + part * (D / kBwdParts), bwd_smem + kPartBytes, row, part, 1.0f);
+        continue;
+      }
       const bool row_exists = w.j * kBlockN + row < p.NK;  // keys of a partial last block beyond NK are computed, not stored
       const int key = w.j * kBlockN + row;
       bwd_store_part_row<D>(tmem + lane_addr + cDK + part * (D / kBwdParts),
@@ -657,6 +716,44 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       bwd_store_part_row<D>(tmem + lane_addr + cDV + part * (D / kBwdParts),
                             dv_row(p, w.b, key, w.kvh) + part * (D / kBwdParts), 1.0f, row_exists);
       tc_fence_before();  // orders these reads before the next item's first dV product (published through P_FULL)
+    }
+    if constexpr (SPLIT) {
+      __syncwarp();
+      cluster_arrive();
+      cluster_wait();
+      if (ok) {
+        // every n-th row of the key block is added up here
+        const DkdvItem w = decode_dkdv_item<CAUSAL, SPLIT>(p, dkdv_item_for_round<CAUSAL, SPLIT>(p, 0));
+        constexpr int kUnits = 2 * (D / 8);         // 8 columns each: dK, then dV
+        for (int u = tid; w.n_iter > 0; u += 32 * kBwdCW) {
+          const int r_row = w.rank + (u / kUnits) * p.split, unit = u % kUnits;
+          if (r_row >= kBlockN) break;
+          const bool is_dv = unit >= D / 8;
+          const int c8 = is_dv ? unit - D / 8 : unit;
+          float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          const uint32_t base = smem_u32(bwd_smem) + (is_dv ? kPartBytes : 0) + r_row * (D * 4);
+          for (int r = 0; r < p.split; ++r) {
+            if (dkdv_share(r, p.split, w.n_iter) == dkdv_share(r + 1, p.split, w.n_iter)) continue;  // it had nothing to do
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const float4 x = ld_cluster_f4(map_to_rank(base + (((c8 * 2 + h) ^ (r_row & 7)) << 4), r));
+              acc[h * 4 + 0] += x.x;
+              acc[h * 4 + 1] += x.y;
+              acc[h * 4 + 2] += x.z;
+              acc[h * 4 + 3] += x.w;
+            }
+          }
+          const int key = w.j * kBlockN + r_row;
+          if (key < p.NK) {
+            __nv_bfloat16* const dst = (is_dv ? dv_row(p, w.b, key, w.kvh) : dk_row(p, w.b, key, w.kvh)) + c8 * 8;
+            *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]),
+                                                        pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
+          }
+        }
+      }
+      __syncwarp();
+      cluster_arrive();  // nobody leaves while its partial sums are being read
+      cluster_wait();
     }
   } else {
     bwd_shrink_registers();
@@ -672,10 +769,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       bool ok = true;
       for (int round = 0; ok; ++round) {
         if (round >= p.total_rounds) break;
-        const int idx = dkdv_item_for_round<CAUSAL>(p, round, blockIdx.x, gridDim.x);
+        const int idx = dkdv_item_for_round<CAUSAL, SPLIT>(p, round);
         if (idx < 0) continue;  // a partial round leaves some CTAs without an item
-        const DkdvItem w = decode_dkdv_item<CAUSAL>(p, idx);
-        if (w.n_iter == 0) continue;  // key block wholly beyond this batch element's length: nothing to do
+        const DkdvItem w = decode_dkdv_item<CAUSAL, SPLIT>(p, idx);
+        if (w.n_first == w.n_end) continue;  // key block wholly beyond this batch element's length: nothing to do
         ok = mbar_wait(bars + KV_EMPTY, (item_cnt & 1) ^ 1, abortp, kWaitLimitCycles);
         if (!ok) break;
         ++item_cnt;
@@ -685,7 +782,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           tma_load_4d(sK + ch * kSub, &tmap_k, bars + KV_FULL, ch * 64, w.kvh, w.j * kBlockN, w.b);
           tma_load_4d(sV + ch * kSub, &tmap_v, bars + KV_FULL, ch * 64, w.kvh, w.j * kBlockN, w.b);
         }
-        for (int n = 0, g_rel = 0, i_rel = 0; n < w.n_iter && ok; ++n) {
+        for (int n = w.n_first, g_rel = w.g_first, i_rel = w.i_first; n < w.n_end && ok; ++n) {
           const int head = w.kvh * G + g_rel;  // n / cnt_i and n % cnt_i, counted instead of divided
           const int i = w.i_min + i_rel;
           if (++i_rel == w.cnt_i) {
@@ -720,10 +817,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       // Two threads issue because a thread that issues returns only a few MMAs ahead of the pipe: with one issuer
       // every commit and mbarrier wait between two products (~180 clocks) let the pipe run dry.
       constexpr uint32_t tile16 = kTile >> 4;
-      const uint32_t k_lo = smem_desc_lo(smem_u32(sK), 16);
-      const uint32_t v_lo = smem_desc_lo(smem_u32(sV), 16);
-      const uint32_t q_lo0 = smem_desc_lo(smem_u32(sQ), 16);       // K-major view (B of S^T)
-      const uint32_t do_lo0 = smem_desc_lo(smem_u32(sDO), 16);     // K-major view (B of dP^T)
+      const uint32_t k_lo = smem_desc_lo(kAddrMask & smem_u32(sK), 16);
+      const uint32_t v_lo = smem_desc_lo(kAddrMask & smem_u32(sV), 16);
+      const uint32_t q_lo0 = smem_desc_lo(kAddrMask & smem_u32(sQ), 16);       // K-major view (B of S^T)
+      const uint32_t do_lo0 = smem_desc_lo(kAddrMask & smem_u32(sDO), 16);     // K-major view (B of dP^T)
       uint32_t item_cnt = 0, it = 0;
       int qa = 0, rb = 0;
       uint32_t qa_par = 0, rb_par = 0;
@@ -734,14 +831,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #endif
       for (int round = 0; ok; ++round) {
         if (round >= p.total_rounds) break;
-        const int idx = dkdv_item_for_round<CAUSAL>(p, round, blockIdx.x, gridDim.x);
+        const int idx = dkdv_item_for_round<CAUSAL, SPLIT>(p, round);
         if (idx < 0) continue;  // a partial round leaves some CTAs without an item
-        const DkdvItem w = decode_dkdv_item<CAUSAL>(p, idx);
-        if (w.n_iter == 0) continue;  // key block wholly beyond this batch element's length: nothing to do
+        const DkdvItem w = decode_dkdv_item<CAUSAL, SPLIT>(p, idx);
+        if (w.n_first == w.n_end) continue;  // key block wholly beyond this batch element's length: nothing to do
         ok = iss_wait(bars + KV_FULL, item_cnt & 1, abortp, kWaitLimitCycles);
         if (!ok) break;
         ++item_cnt;
-        for (int n = 0; n < w.n_iter && ok; ++n, ++it) {
+        for (int n = w.n_first; n < w.n_end && ok; ++n, ++it) {
           // S^T(n): dP^T of the previous pair has been read out of X (first pair ever: passes at once); with a
           // region of its own, S^T(n) only waits for S^T(n-1) to be read
           ok = iss_wait(bars + (kSplitX ? S_FREE : DP_FREE), (it & 1) ^ 1, abortp, kWaitLimitCycles) &&
@@ -783,8 +880,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       constexpr uint32_t tile16 = kTile >> 4;
       constexpr uint32_t idesc = make_idesc_bf16(kBlockM, D, true);
       constexpr uint32_t desc_hi = smem_desc_hi(1024);
-      const uint32_t q_mn0 = smem_desc_lo(smem_u32(sQ), kSub);     // MN-major view (B of dK)
-      const uint32_t do_mn0 = smem_desc_lo(smem_u32(sDO), kSub);   // MN-major view (B of dV)
+      const uint32_t q_mn0 = smem_desc_lo(kAddrMask & smem_u32(sQ), kSub);     // MN-major view (B of dK)
+      const uint32_t do_mn0 = smem_desc_lo(kAddrMask & smem_u32(sDO), kSub);   // MN-major view (B of dV)
       uint32_t it = 0;
       int qa = 0, rb = 0;
       uint32_t qa_par = 0, rb_par = 0;
@@ -795,11 +892,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #endif
       for (int round = 0; ok; ++round) {
         if (round >= p.total_rounds) break;
-        const int idx = dkdv_item_for_round<CAUSAL>(p, round, blockIdx.x, gridDim.x);
+        const int idx = dkdv_item_for_round<CAUSAL, SPLIT>(p, round);
         if (idx < 0) continue;  // a partial round leaves some CTAs without an item
-        const DkdvItem w = decode_dkdv_item<CAUSAL>(p, idx);
-        if (w.n_iter == 0) continue;  // key block wholly beyond this batch element's length: nothing to do
-        for (int n = 0; n < w.n_iter && ok; ++n, ++it) {
+        const DkdvItem w = decode_dkdv_item<CAUSAL, SPLIT>(p, idx);
+        if (w.n_first == w.n_end) continue;  // key block wholly beyond this batch element's length: nothing to do
+        for (int n = w.n_first; n < w.n_end && ok; ++n, ++it) {
           ok = iss_wait(bars + P_FULL, it & 1, abortp, kWaitLimitCycles) &&
                iss_wait(bars + RB_FULL + rb, rb_par, abortp, kWaitLimitCycles);
           if (!ok) break;
@@ -809,7 +906,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             const uint32_t b_lo = do_mn0 + rb * tile16;
 #pragma unroll
             for (int k = 0; k < kBlockN / 16; ++k)
-              umma_ts_lohi(tmem + cDV, tmem + cY + k * 8, b_lo + k * 128, desc_hi, idesc, (n > 0 || k > 0) ? 1u : 0u);
+              umma_ts_lohi(tmem + cDV, tmem + cY + k * 8, b_lo + k * 128, desc_hi, idesc, (n > w.n_first || k > 0) ? 1u : 0u);
             umma_commit(bars + RB_EMPTY + rb);  // second of two arrivals
           }
           HK_STAMP(3, 11);
@@ -826,7 +923,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             const uint32_t b_lo = q_mn0 + qa * tile16;
 #pragma unroll
             for (int k = 0; k < kBlockN / 16; ++k)
-              umma_ts_lohi(tmem + cDK, tmem + cY + 64 + k * 8, b_lo + k * 128, desc_hi, idesc, (n > 0 || k > 0) ? 1u : 0u);
+              umma_ts_lohi(tmem + cDK, tmem + cY + 64 + k * 8, b_lo + k * 128, desc_hi, idesc, (n > w.n_first || k > 0) ? 1u : 0u);
             // S^T of this stage (issuer A) completed before dS^T could be computed, so this one arrival frees Q
             umma_commit(bars + QA_EMPTY + qa);
             umma_commit(bars + Y_FREE);
@@ -865,12 +962,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       };
       for (int round = 0; ok; ++round) {
         if (round >= p.total_rounds) break;
-        const int idx = dkdv_item_for_round<CAUSAL>(p, round, blockIdx.x, gridDim.x);
+        const int idx = dkdv_item_for_round<CAUSAL, SPLIT>(p, round);
         if (idx < 0) continue;  // a partial round leaves some CTAs without an item
-        const DkdvItem w = decode_dkdv_item<CAUSAL>(p, idx);
-        if (w.n_iter == 0) continue;  // key block wholly beyond this batch element's length: nothing to do
-        fetch(w, 0);
-        for (int n = 0; n < w.n_iter && ok; ++n, ++it) {
+        const DkdvItem w = decode_dkdv_item<CAUSAL, SPLIT>(p, idx);
+        if (w.n_first == w.n_end) continue;  // key block wholly beyond this batch element's length: nothing to do
+        fetch(w, w.n_first);
+        for (int n = w.n_first; n < w.n_end && ok; ++n, ++it) {
           const int ss = it & 1;
           ok = mbar_wait(bars + STAT_EMPTY + ss, ((it >> 1) & 1) ^ 1, abortp, kWaitLimitCycles);
           ok = __all_sync(0xffffffffu, ok);
@@ -882,9 +979,16 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(bars + STAT_FULL + ss);
-          if (n + 1 < w.n_iter) fetch(w, n + 1);
+          if (n + 1 < w.n_end) fetch(w, n + 1);
         }
       }
+    }
+    if constexpr (SPLIT) {
+      __syncwarp();
+      cluster_arrive();
+      cluster_wait();
+      cluster_arrive();
+      cluster_wait();
     }
   }
 

@@ -5,6 +5,8 @@
 
 namespace hk {
 
+constexpr int kMaxCluster = 16;  // above 8 a kernel needs cudaFuncAttributeNonPortableClusterSizeAllowed
+
 // CTAs per cluster along x, which divides the grid's x.
 struct ClusterX {
   unsigned n;
@@ -41,6 +43,25 @@ template <typename... Params, typename... Args>
 cudaError_t launch_dependent(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
                              cudaStream_t stream, const Args&... args) {
   return launch_dependent(early, kernel, grid, block, smem, stream, ClusterX{1}, args...);
+}
+
+// Clusters of n CTAs that the current device holds at once (0: not even one, as on a slice of a GPU).
+template <typename Kernel>
+int clusters_held(Kernel* fn, int threads, size_t smem, int n) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = n;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int held = 0;
+  if (cudaOccupancyMaxActiveClusters(&held, fn, &cfg) == cudaSuccess) return held;
+  cudaGetLastError();
+  return 0;
 }
 
 }  // namespace hk

@@ -2,6 +2,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -64,6 +65,7 @@ struct DeviceState {
   int sm_count = 0;
   int cc_major = 0;
   hk::DecodeLimits decode;
+  int bwd_clusters[hk::kMaxDkdvSplit + 1] = {};  // clusters of so many dK/dV CTAs that the device holds at once
   int* status = nullptr;       // the status word, device address (kernels write it only when something went wrong)
   int* status_host = nullptr;  // ... and host address: mapped memory, so that reading it needs no copy
 };
@@ -100,14 +102,14 @@ template <>
 struct BwdLayout<false> {
   static constexpr int kThreads = hk::bwd16::kBwdThreads, kRegsAtLaunch = hk::bwd16::kBwdRegsAtLaunch;
   static constexpr bool kExactRegs = hk::bwd16::kBwdRegsGrown != hk::bwd16::kBwdRegsAtLaunch;
-  template <int D> static constexpr auto dkdv() { return &hk::bwd16::attn_bwd_dkdv_kernel<D, false>; }
+  template <int D, bool SPLIT> static constexpr auto dkdv() { return &hk::bwd16::attn_bwd_dkdv_kernel<D, false, SPLIT>; }
   template <int D> static constexpr auto dq() { return &hk::bwd16::attn_bwd_dq_kernel<D, false>; }
 };
 template <>
 struct BwdLayout<true> {
   static constexpr int kThreads = hk::bwd8::kBwdThreads, kRegsAtLaunch = hk::bwd8::kBwdRegsAtLaunch;
   static constexpr bool kExactRegs = hk::bwd8::kBwdRegsGrown != hk::bwd8::kBwdRegsAtLaunch;
-  template <int D> static constexpr auto dkdv() { return &hk::bwd8::attn_bwd_dkdv_kernel<D, true>; }
+  template <int D, bool SPLIT> static constexpr auto dkdv() { return &hk::bwd8::attn_bwd_dkdv_kernel<D, true, SPLIT>; }
   template <int D> static constexpr auto dq() { return &hk::bwd8::attn_bwd_dq_kernel<D, true>; }
 };
 
@@ -134,9 +136,11 @@ int prepare_bwd_kernel(Kernel* fn, int dyn_bytes, const char* name, int regs_at_
 template <int D, bool CAUSAL>
 int prepare_bwd_kernels() {
   using Lay = BwdLayout<CAUSAL>;
-  int rc = prepare_bwd_kernel(Lay::template dkdv<D>(), hk::BwdSmem<D>::kDynBytes, "attn_bwd_dkdv_kernel",
-                              Lay::kRegsAtLaunch, Lay::kExactRegs);
-  if (rc != HK_OK) return rc;
+  int rc = HK_OK;
+  for (auto* fn : {Lay::template dkdv<D, false>(), Lay::template dkdv<D, true>()})
+    if ((rc = prepare_bwd_kernel(fn, hk::BwdSmem<D>::kDynBytes, "attn_bwd_dkdv_kernel", Lay::kRegsAtLaunch,
+                                 Lay::kExactRegs)) != HK_OK)
+      return rc;
   return prepare_bwd_kernel(Lay::template dq<D>(), hk::BwdSmem<D>::kDynBytes, "attn_bwd_dq_kernel", Lay::kRegsAtLaunch,
                             Lay::kExactRegs);
 }
@@ -162,6 +166,8 @@ int init_device(int device) {
   if ((rc = prepare_bwd_kernels<128, true>()) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<64, false>()) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<64, true>()) != HK_OK) return rc;
+  for (int n = 2; n <= hk::kMaxDkdvSplit; ++n)
+    st.bwd_clusters[n] = hk::clusters_held(BwdLayout<false>::dkdv<128, true>(), BwdLayout<false>::kThreads, hk::BwdSmem<128>::kDynBytes, n);
   // the one allocation this library makes: the status word (last, so that a failure above leaves nothing behind). It
   // lies in mapped host memory: a blocking call reads it after its synchronisation, and a 4-byte copy from device
   // memory to a pageable variable took 18 us of every one of them.
@@ -366,11 +372,66 @@ bool deal_in_pairs(int units, int G, int N, int nbk, int D, int sm_count) {
   return idle <= (lost > 0.05 ? lost : 0.05);
 }
 
+// How many CTAs share a key block of the dK/dV kernel: with few K/V heads there are few blocks, each with all query tiles of
+// the group's heads, and most SMs would have none. Estimated in (query tile, key block) pairs (about 2 us each): a CTA
+// costs its pairs and 2 more, one of a cluster of n 5 + 0.75 n more (launch, first loads, the merge); a call ends when its
+// longest CTA does, when the clusters that the device holds at once are through, or when all SMs have done dK/dV and dQ
+// (half the time per pair), whichever is last. Fitted to 61 shapes of 1 to 300 blocks: the estimate's choice takes 1.5 %
+// longer than the best on average, never to split 20 %. us per backward, 1 / chosen: B1 N1024 H8/1 D128 causal 108 / 33 (8),
+// B1 N4096 H8/1 D128 488 / 214 (4), B1 N8192 H8/1 D128 causal 936 / 423 (3), B1 N2048 H8/1 D64 causal 164 / 38 (8),
+// B2 N384 H8/2 D128 causal 28 / 21 (4), B2 N1024 H16/4 D128 87 / 71 (2).
+// A block's sums are split in other places than those of a call that does not, so a batch element's gradients are not
+// those of the same element in a larger batch to the last bit. Clusters of several waves are therefore taken only for
+// half the time, and pairs of CTAs not for causal calls.
+int dkdv_split(int units, int G, int N, int NK, bool causal, int sm_count, const int* clusters) {
+  const int nbq = (N + hk::kBlockM - 1) / hk::kBlockM, nbk = (NK + hk::kBlockN - 1) / hk::kBlockN;
+  if (1ll * units * nbk > 2ll * sm_count) return 1;
+  const int items = units * nbk;
+  double longest = 0, pairs = 0;  // of one unit, as if no keys were padding
+  for (int j = 0; j < nbk; ++j) {
+    const long long first = causal ? 1ll * j * hk::kBlockN - (NK - N) : 0;  // the first query that sees the block
+    const long long tiles = nbq - (first > 0 ? first / hk::kBlockM : 0);
+    const double n = tiles > 0 ? double(G) * tiles : 0;
+    longest = n > longest ? n : longest;
+    pairs += n;
+  }
+  const double dq_work = 0.5 * units * pairs + 1.0 * units * G * nbq;
+  auto estimate = [&](int n, int held) {
+    const double more = n == 1 ? 2.0 : 5.0 + 0.75 * n;
+    const double top = std::ceil(longest / n) + more, mean = pairs / nbk / n + more;
+    double span;
+    if (causal) span = std::max(top, items * mean / held + (items > held ? 0.5 * mean : 0.0));
+    else span = std::ceil(double(items) / held) * top;
+    return std::max(span, (items * n * mean + dq_work) / sm_count);
+  };
+  const double alone = estimate(1, sm_count);
+  int best = 1;
+  double best_time = alone;
+  for (int n = causal ? 3 : 2; n <= hk::kMaxDkdvSplit; ++n) {
+    if (clusters[n] == 0) continue;
+    const double t = estimate(n, clusters[n]);
+    if (t < best_time && t < (items <= clusters[n] ? 0.95 : 0.5) * alone) {
+      best = n;
+      best_time = t;
+    }
+  }
+  return best;
+}
+
 // Deals the key blocks to CTAs (dkdv_item_for_round); returns the grid.
 template <int D, bool CAUSAL>
-int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count) {
+int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count, const int* clusters) {
   const int units = p.B * p.H_KV;
   p.n_items = units * nbk;
+  p.split = dkdv_split(units, p.H / p.H_KV, p.N, p.NK, CAUSAL, sm_count, clusters);
+  if (p.split > 1) {  // one cluster per item, the longest first
+    p.fd_split = hk::FastDiv(p.split);
+    set_bwd_decode(p, nbk, 1, 1, p.n_items, false);
+    p.n_pairs = 0;
+    p.fd_pairs = hk::FastDiv(units);
+    p.total_rounds = 1;
+    return p.n_items * p.split;
+  }
   int grid = p.n_items < sm_count ? p.n_items : sm_count;
   set_bwd_decode(p, nbk, 1, 1, grid, false);
   p.n_pairs = 0;
@@ -392,27 +453,31 @@ int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count) {
 template <int D, bool CAUSAL>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                hk::BwdParams p, int B, int N, int NK, int H, int H_KV, bool dq_beside, int sm_count,
-               cudaStream_t stream) {
+               const int* clusters, cudaStream_t stream) {
   const int nbq = (N + hk::kBlockM - 1) / hk::kBlockM;   // query tiles
   const int nbk = (NK + hk::kBlockN - 1) / hk::kBlockN;  // key blocks
   if (static_cast<long long>(B) * H * nbq > 0x3fffffffll || static_cast<long long>(B) * H_KV * nbk > 0x3fffffffll)
     return HK_EINVAL;  // work items are indexed with int
-  int grid = deal_dkdv<D, CAUSAL>(p, nbk, sm_count);
+  int grid = deal_dkdv<D, CAUSAL>(p, nbk, sm_count, clusters);
 #ifdef HK_TRACE
   long long* const trace_buf = p.trace;
   p.trace = g_trace_bwd_kernel == 0 ? trace_buf : nullptr;
 #endif
   using Lay = BwdLayout<CAUSAL>;
   const long long tiles = 1ll * B * H * nbq * nbk;
-  HK_CUDA(hk::launch_dependent(short_kernel(tiles, grid), Lay::template dkdv<D>(), grid, Lay::kThreads,
-                               hk::BwdSmem<D>::kDynBytes, stream, tq, tk, tv, tdo, p));
+  const auto dkdv = p.split > 1 ? Lay::template dkdv<D, true>() : Lay::template dkdv<D, false>();
+  HK_CUDA(hk::launch_dependent(short_kernel(tiles, grid), dkdv, grid, Lay::kThreads, hk::BwdSmem<D>::kDynBytes, stream,
+                               hk::ClusterX{unsigned(p.split)}, tq, tk, tv, tdo, p));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   // The dQ kernel runs on the SMs that the dK/dV kernel leaves: us per backward in a loop, one after the other / so (D128
-  // unless said): B1 N512 H8/8 23.6 / 15.3, B2 N384 H8/2 causal 34.6 / 27.4, B2 N2000 H3/1 D64 86.9 / 69.0, B1 N1024 H8/1
-  // 121 / 109, B16 N2048 H64/8 6733 / 6648. Where few SMs are left (from three quarters of them taken on, in one round), the
-  // few CTAs that start early cost the longest dK/dV CTAs more than they give (B5 N300 H32/8 causal, 120 of 148:
-  // 53.3 / 61.4; B4, 96 of 148: 49.1 / 43.6).
-  p.dq_waits = !dq_beside || (grid < sm_count && 4 * grid > 3 * sm_count);
+  // unless said): B1 N512 H8/8 23.6 / 15.3, B2 N384 H8/2 causal 34.6 / 27.4, B2 N2000 H3/1 D64 86.9 / 69.0, B1 N4096 H16/16
+  // causal 227 / 210, B12 N2048 H16/16 1361 / 1351. Above 500 tiles per CTA there is nothing in it (B4 N4096 H32/8 causal
+  // 1733 / 1748, B16 N2048 H64/8 6733 / 6648 and, on another box, 6600 / 6749), and those stay as they were. Where few SMs are left and the longest blocks have most of the pairs (causal,
+  // groups of 3 heads and more, three quarters of the SMs taken in one round of single blocks), the few CTAs that start
+  // early cost those blocks more than they give: B5 N300 H32/8 (120 of 148) 53.3 / 61.4, B7 N457 H32/4 104 / 117; but
+  // B4 N300 H32/8 49.1 / 43.6, B4 N1104 H8/4 63 / 61, B6 N1467 H2/2 D64 39 / 29, B1 N4096 H32/8 (pairs) 456 / 391.
+  p.dq_waits = !dq_beside || tiles > 500ll * grid ||
+               (CAUSAL && p.split == 1 && p.n_pairs == 0 && p.G >= 3 && grid < sm_count && 4 * grid > 3 * sm_count);
   p.n_items = B * H * nbq;
   grid = p.n_items < sm_count ? p.n_items : sm_count;
   set_bwd_decode(p, (H / H_KV) * nbq, H / H_KV, CAUSAL ? H / H_KV : nbq, grid, CAUSAL);
@@ -688,10 +753,10 @@ static int bwd_launch(const void* q, const void* k, const void* v, const void* o
   // The dQ kernel starts while the dK/dV kernel is still reading, unless it would write over what that reads: dQ in the place
   // of Q or of dO is as good as anywhere else when one kernel follows the other.
   const bool dq_beside = !overlap(dq, s.dq, q, s.q, B, N, H, D) && !overlap(dq, s.dq, d_o, dos, B, N, H, D);
-  if (D == 128) return causal ? launch_bwd<128, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, stream)
-                              : launch_bwd<128, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, stream);
-  return causal ? launch_bwd<64, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, stream)
-                : launch_bwd<64, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, stream);
+  if (D == 128) return causal ? launch_bwd<128, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, st->bwd_clusters, stream)
+                              : launch_bwd<128, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, st->bwd_clusters, stream);
+  return causal ? launch_bwd<64, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, st->bwd_clusters, stream)
+                : launch_bwd<64, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, st->bwd_clusters, stream);
 }
 
 int hk_attn_bwd_cross(const void* q, const void* k, const void* v, const void* d_o, const float* lse,

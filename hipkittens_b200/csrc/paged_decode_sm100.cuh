@@ -32,7 +32,6 @@ constexpr int kSlabBytes = kPageTokens * kDecodeD * 2;   // one page of one kv h
 constexpr int kStageBytes = 2 * kSlabBytes;           // K slab + V slab
 constexpr int decode_smem_bytes(int warps) { return warps * kDecodeStages * kStageBytes; }  // 96 or 192 KB
 constexpr int kMaxCombineSplits = 256;
-constexpr int kMaxCluster = 16;
 
 enum : int { kStatusBadPage = 2, kStatusBadLen = 4 };  // 3 is the backward kernels' kStatusSmemAlign
 
@@ -154,20 +153,6 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// Cluster barrier (threads that have left are not waited for) and reads of another CTA's shared memory.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, int rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ float ld_cluster(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
 }
 
 }  // namespace dec
@@ -400,8 +385,8 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 1 : 2) paged_decode_split_ker
           cl_ml[2 * h + 1] = L[i];
         }
       }
-      cluster_arrive();
-      cluster_wait();
+      ptx::cluster_arrive();
+      ptx::cluster_wait();
       for (int h = split * kHalves + h0; h < G; h += n_used * kHalves) {
         float m_r[kMaxCluster], l_r[kMaxCluster], o_r[kMaxCluster];
         const uint32_t a_ml = ptx::smem_u32(cl_ml + 2 * h), a_o = ptx::smem_u32(cl_o + h * kDecodeD + d);
@@ -410,10 +395,10 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 1 : 2) paged_decode_split_ker
           m_r[r] = -INFINITY;
           l_r[r] = o_r[r] = 0.f;
           if (r < n_used) {
-            const uint32_t ml = map_to_rank(a_ml, r);
-            m_r[r] = ld_cluster(ml);
-            l_r[r] = ld_cluster(ml + 4);
-            o_r[r] = ld_cluster(map_to_rank(a_o, r));
+            const uint32_t ml = ptx::map_to_rank(a_ml, r);
+            m_r[r] = ptx::ld_cluster(ml);
+            l_r[r] = ptx::ld_cluster(ml + 4);
+            o_r[r] = ptx::ld_cluster(ptx::map_to_rank(a_o, r));
           }
         }
         float Mc = m_r[0];
@@ -430,8 +415,8 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 1 : 2) paged_decode_split_ker
         p.o[row * kDecodeD + d] = __float2bfloat16(out / sum);
         if (d == 0) p.lse[row] = Mc * p.scale + __logf(sum);
       }
-      cluster_arrive();  // nobody leaves while its shared memory is being read
-      cluster_wait();
+      ptx::cluster_arrive();  // nobody leaves while its shared memory is being read
+      ptx::cluster_wait();
       return;
     }
   }
@@ -522,24 +507,6 @@ cudaError_t prepare_decode_kernels_of() {
   if (e == cudaSuccess) e = prepare_decode_kernel<G, true, 8>();
   return e;
 }
-// Clusters of n CTAs that the current device holds at once (0: not even one, as on a slice of a GPU).
-template <typename Kernel>
-int clusters_held(Kernel* fn, int warps, int n) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(n);
-  cfg.blockDim = dim3(warps * 32);
-  cfg.dynamicSmemBytes = decode_smem_bytes(warps);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = n;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int held = 0;
-  if (cudaOccupancyMaxActiveClusters(&held, fn, &cfg) == cudaSuccess) return held;
-  cudaGetLastError();
-  return 0;
-}
 inline int prepare_decode_kernels(char* err, size_t err_len, int sm_count, DecodeLimits* lim) {
   for (auto* prepare : {prepare_decode_kernels_of<1>, prepare_decode_kernels_of<2>, prepare_decode_kernels_of<3>,
                         prepare_decode_kernels_of<4>, prepare_decode_kernels_of<5>, prepare_decode_kernels_of<6>,
@@ -551,8 +518,8 @@ inline int prepare_decode_kernels(char* err, size_t err_len, int sm_count, Decod
     }
   }
   lim->sm_count = sm_count;
-  for (int n = 2; n <= kMaxCluster; ++n) lim->clusters4[n] = clusters_held(paged_decode_split_kernel<8, true, 4>, 4, n);
-  lim->clusters8 = clusters_held(paged_decode_split_kernel<8, true, 8>, 8, kMaxCluster);
+  for (int n = 2; n <= kMaxCluster; ++n) lim->clusters4[n] = clusters_held(paged_decode_split_kernel<8, true, 4>, 4 * 32, decode_smem_bytes(4), n);
+  lim->clusters8 = clusters_held(paged_decode_split_kernel<8, true, 8>, 8 * 32, decode_smem_bytes(8), kMaxCluster);
   return 0;
 }
 
