@@ -17,14 +17,16 @@
 //                         already in the A-operand position of dV += P^T dO and dK += dS^T Q.
 //   attn_bwd_dq_kernel    one query tile of 128 rows stays in shared memory; the K/V tiles stream past it:
 //                         S = Q K^T, dP = dO V^T, dQ += dS K.
-// Both kernels are persistent (one CTA per SM, 640 threads by default): warps 0-15 do the element-wise work
-// (four threads per TMEM lane, 32 columns each), then one warp each for the TMA producer, the two UMMA-issuing
+// Both kernels are persistent (one CTA per SM, 384 threads): warps 0-7 do the element-wise work
+// (two threads per TMEM lane, 64 columns each), then one warp each for the TMA producer, the two UMMA-issuing
 // roles and, in the dK/dV kernel, the loader of the per-row statistics.
 // TMEM is laid out so that a score-shaped accumulator is free for the next product as soon as the element-wise
 // warps hold it in registers (its bf16 successor goes elsewhere: see the column maps in the kernels).
 //
 // Any sequence length works (the reference's kernels need a multiple of 256): TMA zero-fills the rows of a partial
 // last tile, their statistics are read as zero, and their gradient rows are not stored.
+
+#pragma once
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -34,28 +36,19 @@
 #include "attn_fwd_sm100.cuh"
 #include "sm100_ptx.cuh"
 
-// This header may be included more than once: the part that does not depend on the thread layout is compiled
-// once; the main kernels and their helpers are compiled into namespace hk::HK_BWD_NS with HK_BWD_PARTS threads per
-// TMEM lane, so that a translation unit can hold two layouts (the 8-warp one serves the causal instantiations,
-// where it measured 3 to 7 % faster; the 16-warp one the others).
-#ifndef HK_ATTN_BWD_SHARED_PART
-#define HK_ATTN_BWD_SHARED_PART
 namespace hk {
 
 enum : int { kStatusSmemAlign = 3 };  // dynamic shared memory did not start on a 1024-byte boundary
 
-// Of every kBwdEmuMod column pairs of a score row, kBwdEmuCnt take their exponentials from the cubic polynomial on the
-// FMA pipe (ptx::ex2_poly2, relative error 1e-4, far inside the bf16 rounding of P and dS) instead of the MUFU.
-#ifndef HK_BWD_EMU_MOD
-#define HK_BWD_EMU_MOD 4
-#endif
-#ifndef HK_BWD_EMU_CNT
-#define HK_BWD_EMU_CNT 1
-#endif
+// Of every kBwdEmuMod column pairs of a score row, one takes its exponentials from the cubic polynomial on the FMA pipe
+// (ptx::ex2_poly2, relative error 1e-4, far inside the bf16 rounding of P and dS) instead of the MUFU. One of four at
+// D = 64 (none: 2 to 4 % slower), one of eight at D = 128, where there are twice the products per exponential (none, one
+// of eight, one of four, back to back at the power cap: B16 N2048 H64/8 6 665 / 6 669 / 6 707 us, B4 N4096 H32/8 causal
+// 1 816 / 1 815 / 1 823).
+template <int D>
+constexpr int kBwdEmuMod = D == 64 ? 4 : 8;
 constexpr int kMaxDkdvSplit = 8;  // CTAs that share a key block; larger clusters measured slower throughout
 
-constexpr int kBwdEmuMod = HK_BWD_EMU_MOD;
-constexpr int kBwdEmuCnt = HK_BWD_EMU_CNT;
 
 struct BwdParams {
   const float* lse;     // [B,H,1,N] from the forward pass (natural log)
@@ -215,38 +208,24 @@ __global__ void __launch_bounds__(256) attn_dq_shuffle_kernel(const uint4* src, 
     if (idx0 + u * 256 < total) dst[idx0 + u * 256] = val[u];
 }
 
-// Dynamic shared memory of both main kernels: tiles first (1024-byte aligned for the 128-byte swizzle),
-// then the (L, delta) stages, then the mbarriers and two control words.
-}  // namespace hk
-#endif  // HK_ATTN_BWD_SHARED_PART
-
-#ifndef HK_BWD_NS
-#define HK_BWD_NS bwd_layout
-#endif
-namespace hk {
-namespace HK_BWD_NS {
-
-
-// Element-wise warps: kBwdParts threads share one TMEM lane (one score row), each owning 128 / kBwdParts columns.
-// 4 parts = 16 element-wise warps (4 per scheduler) in a 640-thread CTA without register re-allocation; 2 parts =
-// 8 warps in a 384-thread CTA that re-balances registers like the forward kernel. Sixteen warps measured 1 to 2 %
-// faster on the non-causal shapes, eight 3 to 7 % faster on the causal ones (every barrier the issuers wait for
-// collects half as many arrivals); 4 is the default when nothing is said.
-#ifndef HK_BWD_PARTS
-#define HK_BWD_PARTS 4
-#endif
-constexpr int kBwdParts = HK_BWD_PARTS;
-static_assert(kBwdParts == 2 || kBwdParts == 4, "2 or 4 threads per TMEM lane");
+// Dynamic shared memory of both main kernels: tiles first (1024-byte aligned for the 128-byte swizzle), then the (L, delta)
+// stages, then the mbarriers and two control words.
+//
+// Element-wise warps: two threads share one TMEM lane (one score row), each owning 64 of its columns; 8 such warps in a
+// 384-thread CTA that re-balances registers like the forward kernel. Sixteen warps of 32 columns (640 threads of 96
+// registers) take as many instructions, but every barrier the issuers wait for collects twice the arrivals: back to back
+// at the power cap, 16 / 8 warps, B16 N2048 H64/8 D128 6 722 / 6 576 us, B16 N4096 H16 D64 4 613 / 4 428, B12 N2048 H16
+// D128 1 347 / 1 320; causal shapes 3 to 7 %.
+constexpr int kBwdParts = 2;
 constexpr int kBwdCW = 4 * kBwdParts;              // element-wise warps
 constexpr int kBwdPC = 128 / kBwdParts;            // score columns per element-wise thread
 constexpr int kBwdThreads = 32 * (kBwdCW + 4);     // + TMA producer, two UMMA issuers, statistics loader (idle in dQ)
 // Register budget: all warps start with kBwdRegsAtLaunch; the element-wise warps then grow by exactly what the
 // other four warps give up (setmaxnreg only moves registers inside the CTA's own allocation: asking for more than
-// was released would block forever): 8 x (208 - 168) = 4 x (168 - 88). With 4 parts (640 threads) every thread keeps
-// its 96 registers: the element-wise code fits, and no re-allocation is done.
-constexpr int kBwdRegsAtLaunch = kBwdParts == 2 ? 168 : 96;
-constexpr int kBwdRegsGrown = kBwdParts == 2 ? 208 : 96;
-constexpr int kBwdRegsShrunk = kBwdParts == 2 ? 88 : 96;
+// was released would block forever): 8 x (208 - 168) = 4 x (168 - 88).
+constexpr int kBwdRegsAtLaunch = 168;
+constexpr int kBwdRegsGrown = 208;
+constexpr int kBwdRegsShrunk = 88;
 static_assert(kBwdCW * (kBwdRegsGrown - kBwdRegsAtLaunch) == 4 * (kBwdRegsAtLaunch - kBwdRegsShrunk),
               "registers taken by the element-wise warps must equal the registers released by the other warps");
 
@@ -255,21 +234,12 @@ __device__ __forceinline__ void bwd_ld_part(uint32_t taddr, uint32_t* r) {
 #pragma unroll
   for (int c = 0; c < kBwdPC / 32; ++c) ptx::tmem_ld32(taddr + c * 32, r + c * 32);
 }
-__device__ __forceinline__ void bwd_st_packed(uint32_t taddr, const uint32_t* r) {
-  if constexpr (kBwdPC == 64) ptx::tmem_st32(taddr, r);
-  else ptx::tmem_st16(taddr, r);
-}
+__device__ __forceinline__ void bwd_st_packed(uint32_t taddr, const uint32_t* r) { ptx::tmem_st32(taddr, r); }
 __device__ __forceinline__ void bwd_grow_registers() {
-  if constexpr (kBwdParts == 2) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
-    static_assert(kBwdParts != 2 || kBwdRegsGrown == 208, "keep the immediate above in step");
-  }
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kBwdRegsGrown));
 }
 __device__ __forceinline__ void bwd_shrink_registers() {
-  if constexpr (kBwdParts == 2) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-    static_assert(kBwdParts != 2 || kBwdRegsShrunk == 88, "keep the immediate above in step");
-  }
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kBwdRegsShrunk));
 }
 
 // ------------------------------------------------------------------------------------ shared helpers
@@ -317,13 +287,12 @@ __device__ __forceinline__ void bwd_issue_ts(uint32_t d_tmem, uint32_t a_tmem, u
 // Accumulator rows (this thread's TMEM lane, D / kBwdParts columns from `taddr`) -> bf16 -> global, scaled.
 template <int D>
 __device__ __forceinline__ void bwd_store_part_row(uint32_t taddr, __nv_bfloat16* dst, float mul, bool row_exists) {
-  constexpr int kCols = D / kBwdParts;  // 64, 32 or 16
-  constexpr int kChunk = kCols >= 32 ? 32 : 16;
+  constexpr int kCols = D / kBwdParts;  // 64 or 32
+  constexpr int kChunk = 32;
 #pragma unroll
   for (int cc = 0; cc < kCols / kChunk; ++cc) {
     uint32_t o[kChunk];
-    if constexpr (kChunk == 32) ptx::tmem_ld32(taddr + cc * 32, o);
-    else ptx::tmem_ld16(taddr, o);
+    ptx::tmem_ld32(taddr + cc * 32, o);
     ptx::tmem_wait_ld();
     if (!row_exists) continue;  // the TMEM load above is warp-collective, the store is per row
     uint32_t r[kChunk / 2];
@@ -349,12 +318,11 @@ __device__ __forceinline__ void bwd_store_part_row(uint32_t taddr, __nv_bfloat16
 template <int D>
 __device__ __forceinline__ void bwd_stage_part_row(uint32_t taddr, uint8_t* tile, int row, int part, float mul) {
   constexpr int kCols = D / kBwdParts;
-  constexpr int kChunk = kCols >= 32 ? 32 : 16;
+  constexpr int kChunk = 32;
 #pragma unroll
   for (int cc = 0; cc < kCols / kChunk; ++cc) {
     uint32_t o[kChunk];
-    if constexpr (kChunk == 32) ptx::tmem_ld32(taddr + cc * 32, o);
-    else ptx::tmem_ld16(taddr, o);
+    ptx::tmem_ld32(taddr + cc * 32, o);
     ptx::tmem_wait_ld();
 #pragma unroll
     for (int u = 0; u < kChunk / 4; ++u) {
@@ -608,15 +576,15 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             const uint64_t xb = fma2(pack2(__uint_as_float(su[q4 * 4 + 2]), __uint_as_float(su[q4 * 4 + 3])), c2,
                                      pack2(l4.z, l4.w));
             float x0, x1, x2, x3;
-            // all 16 compute warps take their exponentials at the same time, which makes this phase MUFU-bound
+            // all compute warps take their exponentials at the same time, which makes this phase MUFU-bound
             // (16 results per clock and SM): a share of the column pairs goes through the FMA-pipe polynomial
-            if ((2 * q4) % kBwdEmuMod < kBwdEmuCnt) unpack2(ex2_poly2(xa), x0, x1);
+            if ((2 * q4) % kBwdEmuMod<D> == 0) unpack2(ex2_poly2(xa), x0, x1);
             else {
               unpack2(xa, x0, x1);
               x0 = ex2_approx(x0);
               x1 = ex2_approx(x1);
             }
-            if ((2 * q4 + 1) % kBwdEmuMod < kBwdEmuCnt) unpack2(ex2_poly2(xb), x2, x3);
+            if ((2 * q4 + 1) % kBwdEmuMod<D> == 0) unpack2(ex2_poly2(xb), x2, x3);
             else {
               unpack2(xb, x2, x3);
               x2 = ex2_approx(x2);
@@ -1180,7 +1148,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             float x0, x1;
             const uint64_t x2 = fma2(pack2(__uint_as_float(su[2 * i]), __uint_as_float(su[2 * i + 1])), c2, nl2);
             // a share of the column pairs through the FMA-pipe polynomial, as in the dK/dV kernel
-            if (i % kBwdEmuMod < kBwdEmuCnt) unpack2(ex2_poly2(x2), x0, x1);
+            if (i % kBwdEmuMod<D> == 0) unpack2(ex2_poly2(x2), x0, x1);
             else {
               unpack2(x2, x0, x1);
               x0 = ex2_approx(x0);
@@ -1439,7 +1407,4 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   grid_dep_wait();
 }
 
-}  // namespace HK_BWD_NS
 }  // namespace hk
-#undef HK_BWD_NS
-#undef HK_BWD_PARTS

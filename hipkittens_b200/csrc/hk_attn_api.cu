@@ -10,13 +10,6 @@
 #include <mutex>
 
 #include "../../include/hk_attn.h"
-// The backward kernels are compiled in two thread layouts (see the header): 16 element-wise warps for the
-// non-causal instantiations, 8 for the causal ones.
-#define HK_BWD_NS bwd16
-#define HK_BWD_PARTS 4
-#include "attn_bwd_sm100.cuh"
-#define HK_BWD_NS bwd8
-#define HK_BWD_PARTS 2
 #include "attn_bwd_sm100.cuh"
 #include "attn_fwd_sm100.cuh"
 #include "dependent_launch.cuh"
@@ -95,34 +88,15 @@ int prepare_fwd_kernels() {
   return prepare_fwd_kernel<D, CAUSAL, hk::kLongFwdDependent<D, CAUSAL>>();
 }
 
-// The layout that serves an instantiation, with its kernels and launch constants.
-template <bool CAUSAL>
-struct BwdLayout;
-template <>
-struct BwdLayout<false> {
-  static constexpr int kThreads = hk::bwd16::kBwdThreads, kRegsAtLaunch = hk::bwd16::kBwdRegsAtLaunch;
-  static constexpr bool kExactRegs = hk::bwd16::kBwdRegsGrown != hk::bwd16::kBwdRegsAtLaunch;
-  template <int D, bool SPLIT> static constexpr auto dkdv() { return &hk::bwd16::attn_bwd_dkdv_kernel<D, false, SPLIT>; }
-  template <int D> static constexpr auto dq() { return &hk::bwd16::attn_bwd_dq_kernel<D, false>; }
-};
-template <>
-struct BwdLayout<true> {
-  static constexpr int kThreads = hk::bwd8::kBwdThreads, kRegsAtLaunch = hk::bwd8::kBwdRegsAtLaunch;
-  static constexpr bool kExactRegs = hk::bwd8::kBwdRegsGrown != hk::bwd8::kBwdRegsAtLaunch;
-  template <int D, bool SPLIT> static constexpr auto dkdv() { return &hk::bwd8::attn_bwd_dkdv_kernel<D, true, SPLIT>; }
-  template <int D> static constexpr auto dq() { return &hk::bwd8::attn_bwd_dq_kernel<D, true>; }
-};
-
 template <typename Kernel>
-int prepare_bwd_kernel(Kernel* fn, int dyn_bytes, const char* name, int regs_at_launch, bool exact) {
+int prepare_bwd_kernel(Kernel* fn, int dyn_bytes, const char* name) {
   HK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_bytes));
   cudaFuncAttributes attr;
   HK_CUDA(cudaFuncGetAttributes(&attr, fn));
-  // With register re-balancing between warps (the 8-warp layout) the count at launch has to be exact, as for the
-  // forward kernel: refuse to launch a build it would not add up in. Without it any count that fits is fine.
-  if (exact ? attr.numRegs != regs_at_launch : attr.numRegs > regs_at_launch) {
+  // the count at launch has to be exact, as for the forward kernel: refuse to launch a build it would not add up in
+  if (attr.numRegs != hk::kBwdRegsAtLaunch) {
     snprintf(g_cuda_err, sizeof(g_cuda_err), "%s compiled to %d registers, expected %d", name, attr.numRegs,
-             regs_at_launch);
+             hk::kBwdRegsAtLaunch);
     return HK_EUNSUPPORTED;
   }
   if (attr.sharedSizeBytes != 0) {  // the kernels assume their dynamic shared memory starts the CTA's window
@@ -135,14 +109,10 @@ int prepare_bwd_kernel(Kernel* fn, int dyn_bytes, const char* name, int regs_at_
 
 template <int D, bool CAUSAL>
 int prepare_bwd_kernels() {
-  using Lay = BwdLayout<CAUSAL>;
   int rc = HK_OK;
-  for (auto* fn : {Lay::template dkdv<D, false>(), Lay::template dkdv<D, true>()})
-    if ((rc = prepare_bwd_kernel(fn, hk::BwdSmem<D>::kDynBytes, "attn_bwd_dkdv_kernel", Lay::kRegsAtLaunch,
-                                 Lay::kExactRegs)) != HK_OK)
-      return rc;
-  return prepare_bwd_kernel(Lay::template dq<D>(), hk::BwdSmem<D>::kDynBytes, "attn_bwd_dq_kernel", Lay::kRegsAtLaunch,
-                            Lay::kExactRegs);
+  for (auto* fn : {hk::attn_bwd_dkdv_kernel<D, CAUSAL, false>, hk::attn_bwd_dkdv_kernel<D, CAUSAL, true>})
+    if ((rc = prepare_bwd_kernel(fn, hk::BwdSmem<D>::kDynBytes, "attn_bwd_dkdv_kernel")) != HK_OK) return rc;
+  return prepare_bwd_kernel(hk::attn_bwd_dq_kernel<D, CAUSAL>, hk::BwdSmem<D>::kDynBytes, "attn_bwd_dq_kernel");
 }
 
 int init_device(int device) {
@@ -167,7 +137,7 @@ int init_device(int device) {
   if ((rc = prepare_bwd_kernels<64, false>()) != HK_OK) return rc;
   if ((rc = prepare_bwd_kernels<64, true>()) != HK_OK) return rc;
   for (int n = 2; n <= hk::kMaxDkdvSplit; ++n)
-    st.bwd_clusters[n] = hk::clusters_held(BwdLayout<false>::dkdv<128, true>(), BwdLayout<false>::kThreads, hk::BwdSmem<128>::kDynBytes, n);
+    st.bwd_clusters[n] = hk::clusters_held(hk::attn_bwd_dkdv_kernel<128, true, true>, hk::kBwdThreads, hk::BwdSmem<128>::kDynBytes, n);
   // the one allocation this library makes: the status word (last, so that a failure above leaves nothing behind). It
   // lies in mapped host memory: a blocking call reads it after its synchronisation, and a 4-byte copy from device
   // memory to a pageable variable took 18 us of every one of them.
@@ -463,10 +433,9 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   long long* const trace_buf = p.trace;
   p.trace = g_trace_bwd_kernel == 0 ? trace_buf : nullptr;
 #endif
-  using Lay = BwdLayout<CAUSAL>;
   const long long tiles = 1ll * B * H * nbq * nbk;
-  const auto dkdv = p.split > 1 ? Lay::template dkdv<D, true>() : Lay::template dkdv<D, false>();
-  HK_CUDA(hk::launch_dependent(short_kernel(tiles, grid), dkdv, grid, Lay::kThreads, hk::BwdSmem<D>::kDynBytes, stream,
+  const auto dkdv = p.split > 1 ? hk::attn_bwd_dkdv_kernel<D, CAUSAL, true> : hk::attn_bwd_dkdv_kernel<D, CAUSAL, false>;
+  HK_CUDA(hk::launch_dependent(short_kernel(tiles, grid), dkdv, grid, hk::kBwdThreads, hk::BwdSmem<D>::kDynBytes, stream,
                                hk::ClusterX{unsigned(p.split)}, tq, tk, tv, tdo, p));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   // The dQ kernel runs on the SMs that the dK/dV kernel leaves: us per backward in a loop, one after the other / so (D128
@@ -484,7 +453,7 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
 #ifdef HK_TRACE
   p.trace = g_trace_bwd_kernel == 1 ? trace_buf : nullptr;
 #endif
-  HK_CUDA(hk::launch_dependent(!p.dq_waits || short_kernel(tiles, grid), Lay::template dq<D>(), grid, Lay::kThreads,
+  HK_CUDA(hk::launch_dependent(!p.dq_waits || short_kernel(tiles, grid), hk::attn_bwd_dq_kernel<D, CAUSAL>, grid, hk::kBwdThreads,
                                hk::BwdSmem<D>::kDynBytes, stream, tq, tk, tv, tdo, p));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return HK_OK;
