@@ -420,6 +420,49 @@ int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count, const int* clusters) {
   return grid;
 }
 
+// The dQ kernel may run on the SMs that the dK/dV kernel (of `grid` CTAs) leaves, or behind it. Returns its CTAs, negative if
+// they wait for the dK/dV kernel.
+//  * With a CTA for every SM those that find an SM early do their share and the others start when the dK/dV kernel has
+//    ended. That fills gaps (us behind / beside, in a loop: B1 N512 H8/8 D128 23.6 / 15.3, B4 N1024 H12 D64 85 / 70, B2 N2615
+//    H8 D64 153 / 129, B6 N820 H16 D128 141 / 135), but two kernels at a time also cost the key blocks that are still
+//    running: longer calls are better off one after the other (D128 B2 N4096 H4 193 / 203, B13 N505 H32/8 203 / 215; B1
+//    N4096 H32/8 causal 392 / 408; D64 B6 N7554 H6/2 1 981 / 2 067). So do calls of causal groups of 3 heads and more that
+//    take three quarters of the SMs in one round of single blocks (B5 N300 H32/8 53 / 61, B7 N457 H32/4 104 / 117).
+//  * When the last round of key blocks leaves many SMs free, these are dealt all of dQ, if that is estimated to end sooner: in
+//    the pairs of dkdv_split, a dQ item costs 1 and 0.45 per pair alone, 1.5 and 0.65 beside dK/dV. us behind / all SMs /
+//    the free ones (D128 unless said): B5 N512 H32/8 108 / 101 / 78, B1 N2500 H32/8 420 / 383 / 285, B11 N1000 H16/2 D64
+//    263 / 281 / 217, B6 N900 H12/4 141 / 149 / 130, B4 N293 H16 D64 32 / 30 / 25.
+template <int D, bool CAUSAL>
+int dq_ctas(const hk::BwdParams& p, int nbq, int nbk, int grid, int sm_count) {
+  const long long items = 1ll * p.B * p.H * nbq;
+  const int all = items < sm_count ? int(items) : sm_count;
+  double round = 0, pairs = nbk;    // of a round of dK/dV, of an item of dQ
+  long long rounds = 1, last = -1;  // last: CTAs busy in the last round; -1: blocks of every length, in no rounds
+  if (p.split > 1) {
+    if (!CAUSAL) {
+      round = std::ceil(double(p.G) * nbq / p.split) + 5.0 + 0.75 * p.split;
+      last = grid;
+    }
+  } else if (!CAUSAL || p.n_pairs > 0) {
+    const long long units = CAUSAL ? p.n_pairs : p.n_items;
+    round = CAUSAL ? p.G * (nbq + 1.0) + 4.0 : double(p.G) * nbq + 2.0;
+    if (CAUSAL) pairs = 0.5 * (nbk + 1);
+    rounds = (units + grid - 1) / grid;
+    last = units - (rounds - 1) * grid;
+  }
+  const long long free = sm_count - last;
+  if (last >= 0 && free > 0) {
+    if (items <= free) return all;
+    const double behind = rounds * round + std::ceil(double(items) / sm_count) * (1.0 + 0.45 * pairs);
+    const double beside = (rounds - 1) * round + std::ceil(double(items) / double(free)) * (1.5 + 0.65 * pairs);
+    if (std::max(rounds * round, beside) < 0.97 * behind) return int(free);
+  }
+  const long long tiles = 1ll * p.B * p.H * nbq * nbk;
+  const bool long_call = tiles > (D == 64 ? 300ll : CAUSAL ? 120ll : 40ll) * grid;
+  const bool long_blocks = CAUSAL && p.split == 1 && p.n_pairs == 0 && p.G >= 3 && grid < sm_count && 4 * grid > 3 * sm_count;
+  return long_call || long_blocks ? -all : all;
+}
+
 template <int D, bool CAUSAL>
 int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                hk::BwdParams p, int B, int N, int NK, int H, int H_KV, bool dq_beside, int sm_count,
@@ -438,17 +481,10 @@ int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   HK_CUDA(hk::launch_dependent(short_kernel(tiles, grid), dkdv, grid, hk::kBwdThreads, hk::BwdSmem<D>::kDynBytes, stream,
                                hk::ClusterX{unsigned(p.split)}, tq, tk, tv, tdo, p));
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  // The dQ kernel runs on the SMs that the dK/dV kernel leaves: us per backward in a loop, one after the other / so (D128
-  // unless said): B1 N512 H8/8 23.6 / 15.3, B2 N384 H8/2 causal 34.6 / 27.4, B2 N2000 H3/1 D64 86.9 / 69.0, B1 N4096 H16/16
-  // causal 227 / 210, B12 N2048 H16/16 1361 / 1351. Above 500 tiles per CTA there is nothing in it (B4 N4096 H32/8 causal
-  // 1733 / 1748, B16 N2048 H64/8 6733 / 6648 and, on another box, 6600 / 6749), and those stay as they were. Where few SMs are left and the longest blocks have most of the pairs (causal,
-  // groups of 3 heads and more, three quarters of the SMs taken in one round of single blocks), the few CTAs that start
-  // early cost those blocks more than they give: B5 N300 H32/8 (120 of 148) 53.3 / 61.4, B7 N457 H32/4 104 / 117; but
-  // B4 N300 H32/8 49.1 / 43.6, B4 N1104 H8/4 63 / 61, B6 N1467 H2/2 D64 39 / 29, B1 N4096 H32/8 (pairs) 456 / 391.
-  p.dq_waits = !dq_beside || tiles > 500ll * grid ||
-               (CAUSAL && p.split == 1 && p.n_pairs == 0 && p.G >= 3 && grid < sm_count && 4 * grid > 3 * sm_count);
+  const int ctas = dq_ctas<D, CAUSAL>(p, nbq, nbk, grid, sm_count);
+  p.dq_waits = !dq_beside || ctas < 0;
   p.n_items = B * H * nbq;
-  grid = p.n_items < sm_count ? p.n_items : sm_count;
+  grid = !p.dq_waits ? ctas : (p.n_items < sm_count ? p.n_items : sm_count);
   set_bwd_decode(p, (H / H_KV) * nbq, H / H_KV, CAUSAL ? H / H_KV : nbq, grid, CAUSAL);
 #ifdef HK_TRACE
   p.trace = g_trace_bwd_kernel == 1 ? trace_buf : nullptr;
