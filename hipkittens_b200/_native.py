@@ -415,16 +415,21 @@ def attn_bwd_strided(
     _check(rc, "hk_attn_bwd_strided")
 
 
-def key_padding_lens(mask: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+def key_padding_lens(mask: torch.Tensor, bad: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """Key lengths int32 [B] of a CUDA bool mask [B, N] (True = keep), and an int32 scalar tensor that is non-zero if a
-    row does not keep a prefix of at least one key. Asynchronous on torch's current stream."""
+    row does not keep a prefix of at least one key. Asynchronous on torch's current stream.
+
+    `bad`: a zero int32 scalar in pinned host memory, for a caller that synchronises anyway and then reads it without a copy;
+    it has to stay alive until then. By default the scalar is on the mask's device."""
     b, n = mask.shape
     mask = mask.contiguous()
-    buf = torch.zeros(b + 1, dtype=torch.int32, device=mask.device)
+    lens = torch.empty(b, dtype=torch.int32, device=mask.device)
+    if bad is None:
+        bad = torch.zeros((), dtype=torch.int32, device=mask.device)
     s = torch.cuda.current_stream(mask.device)
-    _check(capi().hk_key_padding_lens(mask.data_ptr(), buf.data_ptr(), buf.data_ptr() + 4 * b, b, n, mask.device.index,
+    _check(capi().hk_key_padding_lens(mask.data_ptr(), lens.data_ptr(), bad.data_ptr(), b, n, mask.device.index,
                                       s.cuda_stream), "hk_key_padding_lens")
-    return buf[:b], buf[b]
+    return lens, bad
 
 
 def dq_shuffle(dq_bhnd: torch.Tensor, dq_bnhd: Optional[torch.Tensor] = None,

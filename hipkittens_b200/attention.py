@@ -5,8 +5,8 @@
 and L [B,H,1,N] fp32 are allocated here, O is returned in the input dtype and (q, k, v, O, L) are saved for the backward
 pass. Like the reference's ``tk_kernel_fwd.dispatch_fwd`` and its three backward calls (hipkittens.py:64-119), forward
 and backward each return when the device is done and raise if a kernel reported a failure; they synchronise once for
-that, not after each kernel. A ``key_padding_mask`` is looked at on the device, and its verdict is read, by one more
-synchronisation, behind the forward: a mask that cannot be honoured raises after the kernels have run on clamped lengths.
+that, not after each kernel. A ``key_padding_mask`` is looked at on the device, and its verdict is read behind the forward's
+synchronisation: a mask that cannot be honoured raises after the kernels have run on clamped lengths.
 
 Differences: bf16 tensors are read through strided TMA descriptors and gradients written through strides, so there are
 no ``.contiguous()`` copies of q, k and v (hipkittens.py:37-39) in either direction, and the modules' packed
@@ -129,18 +129,26 @@ class _PackedAttnFunction(Function):
 
 def _attend(q, packed, causal, softmax_scale, key_padding_mask):
     """Attention of q (None: the first of the packed tensors) over a packed projection [B, S, 2 or 3, H, D]."""
-    kv_lens = bad = None
-    if key_padding_mask is not None:
-        kv_lens, bad = _lens_from_key_padding_mask(key_padding_mask, packed)
-    if _packed_viewable(packed) and (q is None or _tma_viewable(q)):
-        out = _PackedAttnFunction.apply(q, packed, bool(causal), softmax_scale, kv_lens)
+    if key_padding_mask is None:
+        out = _apply(q, packed, causal, softmax_scale, None)
     else:
-        views = packed.unbind(dim=2) if q is None else (q, *packed.unbind(dim=2))
-        out = HipAttnFunction.apply(*views, causal, softmax_scale, kv_lens)
-    # read here, when the forward is done and this does not wait for it: whatever the mask, the kernels clamp the lengths
-    if bad is not None and int(bad) != 0:
-        raise ValueError(_BAD_MASK)
+        kv_lens, bad = _lens_from_key_padding_mask(key_padding_mask, packed)
+        try:
+            out = _apply(q, packed, causal, softmax_scale, kv_lens)
+        except BaseException:
+            torch.cuda.synchronize(packed.device)  # the flag may still be written: it is given back only then
+            raise
+        # whatever the mask, the kernels clamp the lengths
+        if bad.item() != 0:
+            raise ValueError(_BAD_MASK)
     return out.to((packed if q is None else q).dtype).contiguous()
+
+
+def _apply(q, packed, causal, softmax_scale, kv_lens):
+    if _packed_viewable(packed) and (q is None or _tma_viewable(q)):
+        return _PackedAttnFunction.apply(q, packed, bool(causal), softmax_scale, kv_lens)
+    views = packed.unbind(dim=2) if q is None else (q, *packed.unbind(dim=2))
+    return HipAttnFunction.apply(*views, causal, softmax_scale, kv_lens)
 
 
 _BAD_MASK = "only right-padded key_padding_mask (a kept prefix of at least one key per row) is supported"
@@ -148,14 +156,16 @@ _BAD_MASK = "only right-padded key_padding_mask (a kept prefix of at least one k
 
 def _lens_from_key_padding_mask(mask: torch.Tensor, packed: torch.Tensor):
     """(B, S) bool, True = keep (base.py:88-89) -> int32 key lengths, for masks that keep a prefix of each row
-    (right padding, what padded batches have), and a flag on the device: non-zero if a row is anything else, which
+    (right padding, what padded batches have), and a flag that becomes non-zero if a row is anything else, which
     cannot be expressed as lengths and is refused."""
     if mask.dim() != 2 or mask.shape[1] != packed.shape[1] or mask.dtype != torch.bool:
         raise ValueError("key_padding_mask must be a bool tensor (batch, seqlen), True = keep")
     assert packed.is_cuda, "All tensors must be on CUDA device"
     if mask.device != packed.device:
         raise RuntimeError("key_padding_mask must be on the device of q, k and v")
-    return key_padding_lens(mask)
+    # pinned memory, which the forward's synchronisation makes readable: a flag on the device cost a fill, a copy and a
+    # synchronisation of its own
+    return key_padding_lens(mask, torch.zeros((), dtype=torch.int32, pin_memory=True))
 
 
 class HipSelfAttention(nn.Module):

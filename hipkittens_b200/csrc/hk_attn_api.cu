@@ -800,9 +800,9 @@ int hk_key_padding_lens(const unsigned char* mask, int32_t* lens, int32_t* bad, 
   DeviceScope scope;
   int rc = scope.enter(device, &st);
   if (rc != HK_OK) return rc;
-  hk::key_padding_lens_kernel<<<B, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(mask, lens, bad, N);
+  HK_CUDA(hk::launch_dependent(true, hk::key_padding_lens_kernel, B, 256, 0, static_cast<cudaStream_t>(cuda_stream), mask, lens,
+                               bad, N));
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  HK_CUDA(cudaGetLastError());
   return HK_OK;
 }
 

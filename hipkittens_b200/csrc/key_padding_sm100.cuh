@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sm100_ptx.cuh"
+
 namespace hk {
 
 // grid = B, block = 256. lens[b] = number of kept keys of row b; *bad (zero on entry) is raised by a row that does not
@@ -12,6 +14,8 @@ namespace hk {
 // operations need for it; a row is N bytes, so this is launch latency (about 3 us) and nothing else.
 __global__ void __launch_bounds__(256) key_padding_lens_kernel(const unsigned char* mask, int32_t* lens, int32_t* bad,
                                                                int N) {
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   const unsigned char* row = mask + static_cast<size_t>(blockIdx.x) * N;
   int kept = 0, end = 0;  // kept keys, and one past the last of them
   for (int i = threadIdx.x; i < N; i += 256) {

@@ -37,7 +37,7 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---------------------------------------------------------------- dependent launch
-// Kernels but the long attention ones, the padding-mask kernel and the self-test are launched with programmatic stream
+// Kernels but the long attention ones and the self-test are launched with programmatic stream
 // serialization (launch_dependent): their CTAs may start while the kernel before them in the stream is finishing, and run
 // their prologue (barriers, TMEM, descriptor prefetch) under its tail. The order is prologue, grid_dep_wait(),
 // grid_dep_launch(), and then the first access to global memory.

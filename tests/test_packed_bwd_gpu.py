@@ -139,3 +139,17 @@ def test_key_padding_lens(b, n):
         hole[0] = True
         hole[0, n // 2] = False
         assert int(_native.key_padding_lens(hole.cuda())[1]) != 0
+
+
+def test_a_refused_mask_leaves_the_next_call_alone():
+    """The verdict on a mask is a flag of its own per call, read behind the forward: refused and accepted masks in turn."""
+    qkv = _rand(2, 300, 3, 4, 64, seed=11)
+    good = torch.arange(300)[None].cuda() < torch.tensor([[300], [120]]).cuda()
+    bad = good.clone()
+    bad[1, 5] = False
+    module = HipSelfAttention()
+    ref = module(qkv, key_padding_mask=good)
+    for _ in range(3):
+        with pytest.raises(ValueError):
+            module(qkv, key_padding_mask=bad)
+        assert torch.equal(module(qkv, key_padding_mask=good), ref)
