@@ -106,7 +106,7 @@ int hk_attn_fwd_paged(const void* q, const void* k_pages, const void* v_pages, c
  *   D = 128, page_size = 16, H / H_KV from 1 to 8; S and H_KV at most 65535, max_pages_per_seq at most 8192
  *   (HK_EUNSUPPORTED beyond, and hk_attn_paged_decode_workspace_bytes then returns 0).
  *   workspace   : device scratch of at least hk_attn_paged_decode_workspace_bytes(...) bytes, 256-byte
- *                 aligned; holds the per-split partial results between the two kernels. */
+ *                 aligned; holds the per-split partial results between the two kernels of launches that need a second one. */
 size_t hk_attn_paged_decode_workspace_bytes(int S, int H, int D, int max_pages_per_seq, int page_size);
 int hk_attn_paged_decode(const void* q, const void* k_pages, const void* v_pages,
                          const int32_t* block_table, const int32_t* ctx_lens, void* o, float* lse,
@@ -139,7 +139,8 @@ int hk_attn_bwd_prep(const void* o, const void* d_o, float* delta, int B, int N,
  *   lse, delta : fp32 [B,H,1,N]
  *   D in {64, 128}; any N >= 1 (the reference needs a multiple of 256); tensor pointers 16-byte aligned, lse and
  *   delta 4-byte aligned; softmax_scale <= 0 selects 1/sqrt(D).
- * Results are bit-identical from run to run (no atomics). */
+ * Results are bit-identical from run to run (no atomics). With few key blocks (B, H_KV and N small) the sums of dK and dV are
+ * split over several CTAs, in places that depend on the whole call's shape. */
 int hk_attn_bwd(const void* q, const void* k, const void* v, const void* d_o, const float* lse, const float* delta,
                 void* dq, void* dk, void* dv, int B, int N, int H, int H_KV, int D, int causal, float softmax_scale,
                 int dq_layout, int device, void* cuda_stream);
