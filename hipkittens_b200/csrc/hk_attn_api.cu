@@ -574,6 +574,24 @@ static int fwd_launch(const void* q, const void* k, const void* v, void* o, floa
 #define HK_GROUP_MB 32
 #endif
     long long u = (static_cast<long long>(HK_GROUP_MB) << 20) / kv_bytes;
+    // A group is dealt in rounds of its own, so one with fewer items than the GPU has SMs leaves the others idle: few
+    // queries on many keys, or on a block table that is wide for its contexts (which the host does not know). It is then
+    // the smallest of what fills one to four rounds, or all units, that needs the fewest rounds.
+    // us, before / now, H64/8 D128 paged: 1 x 64 queries on 1000 keys, table of 8192 pages 71 / 23; 4 x 512 on 8192, 8192
+    // pages 1831 / 514; 16 x 512 on 2048, 2048 pages 994 / 482; H32/8 2 x 128 on 16000, 1000 pages 471 / 251. Contiguous, causal:
+    // 64 queries on 65536 keys 3449 / 890.
+    const long long units = 1ll * B * H_KV, sms = st->sm_count;
+    const long long per_unit = p.pair_heads ? 1ll * (G / 2) * nqb : 1ll * G * ((nqb + 1) / 2);
+    if (u < 1) u = 1;
+    if (u < units && u * per_unit < sms) {
+      auto rounds = [&](long long n) {
+        return units / n * ((n * per_unit + sms - 1) / sms) + (units % n * per_unit + sms - 1) / sms;
+      };
+      for (long long k = 1; k <= 5; ++k) {
+        const long long n = k == 5 || k * sms / per_unit > units ? units : k * sms / per_unit;
+        if (n > u && rounds(n) < rounds(u)) u = n;
+      }
+    }
     p.group_units = int(u < 1 ? 1 : (u > B * H_KV ? B * H_KV : u));
   }
   if (static_cast<long long>(B) * H * nqb > 0x3fffffffll) return HK_EINVAL;  // work items are indexed with int

@@ -106,3 +106,28 @@ def test_bad_page_id_is_reported_not_dereferenced():
     assert _native.device_status(0) == _native.HK_EBADPAGE
     o, l = hk.attn_fwd_paged(q.to(dev), kp.to(dev), vp.to(dev), bt.to(dev), cl.to(dev))
     assert _native.device_status(0) == 0 and torch.isfinite(o.float()).all()
+
+
+@pytest.mark.parametrize("s,t,ctx,h,hkv,d", [(1, 64, 1000, 8, 2, 128), (4, 300, 700, 6, 2, 64), (9, 130, 900, 16, 4, 128)])
+def test_a_wide_block_table_changes_the_work_order_only(s, t, ctx, h, hkv, d):
+    """The causal work order groups units by the table's capacity; whatever the groups, every query tile is served once and
+    its result is that of a table as wide as the contexts."""
+    dev = torch.device("cuda:0")
+    pages = (ctx + 15) // 16
+    gen = torch.Generator(device=dev).manual_seed(s)
+    q, kp, vp = (torch.randn(shape, generator=gen, device=dev).to(torch.bfloat16)
+                 for shape in ((s, t, h, d), (s * pages, 16, hkv, d), (s * pages, 16, hkv, d)))
+    ids = torch.randperm(s * pages, generator=gen, device=dev).view(s, pages).int()
+    lens = torch.tensor([ctx - 37 * i for i in range(s)], dtype=torch.int32, device=dev)
+    results = []
+    for width in (pages, 700, 4000, 8192):
+        table = torch.zeros((s, width), dtype=torch.int32, device=dev)
+        table[:, :pages] = ids
+        out = torch.full_like(q, float("nan"))
+        lse = torch.full((s, h, 1, t), float("nan"), device=dev)
+        hk.attn_fwd_paged(q, kp, vp, table, lens, causal=True, out=out, lse=lse)
+        assert _native.device_status(0) == 0
+        results.append((out, lse))
+    assert bool(torch.isfinite(results[0][0]).all())
+    for out, lse in results[1:]:
+        assert torch.equal(out, results[0][0]) and torch.equal(lse, results[0][1])
