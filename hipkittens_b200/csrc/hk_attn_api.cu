@@ -285,6 +285,21 @@ __global__ void bounded_wait_selftest_kernel(int* status, unsigned long long lim
 // of 4096 (221 tiles): 487.8 / 479.2, and so the line is no higher.
 bool short_kernel(long long tiles, int grid) { return tiles <= 100ll * grid; }
 
+// Units of a causal sweep group that has fewer items (`per_unit` each) than the GPU has SMs: the fewest of what fills one to
+// four rounds, or all units, that need the fewest rounds. Larger groups stay as they are.
+int group_for_fewest_rounds(long long u, long long units, long long per_unit, long long sms) {
+  u = std::max(1ll, std::min(u, units));
+  if (u == units || u * per_unit >= sms) return int(u);
+  auto rounds = [&](long long n) {
+    return units / n * ((n * per_unit + sms - 1) / sms) + (units % n * per_unit + sms - 1) / sms;
+  };
+  for (long long k = 1; k <= 5; ++k) {
+    const long long n = k == 5 ? units : std::min(units, k * sms / per_unit);
+    if (n > u && rounds(n) < rounds(u)) u = n;
+  }
+  return int(u);
+}
+
 template <int D, bool CAUSAL>
 int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
                const hk::FwdParams& p, int grid, cudaStream_t stream) {
@@ -575,24 +590,12 @@ static int fwd_launch(const void* q, const void* k, const void* v, void* o, floa
 #endif
     long long u = (static_cast<long long>(HK_GROUP_MB) << 20) / kv_bytes;
     // A group is dealt in rounds of its own, so one with fewer items than the GPU has SMs leaves the others idle: few
-    // queries on many keys, or on a block table that is wide for its contexts (which the host does not know). It is then
-    // the smallest of what fills one to four rounds, or all units, that needs the fewest rounds.
+    // queries on many keys, or on a block table that is wide for its contexts (which the host does not know).
     // us, before / now, H64/8 D128 paged: 1 x 64 queries on 1000 keys, table of 8192 pages 71 / 23; 4 x 512 on 8192, 8192
     // pages 1831 / 514; 16 x 512 on 2048, 2048 pages 994 / 482; H32/8 2 x 128 on 16000, 1000 pages 471 / 251. Contiguous, causal:
     // 64 queries on 65536 keys 3449 / 890.
-    const long long units = 1ll * B * H_KV, sms = st->sm_count;
     const long long per_unit = p.pair_heads ? 1ll * (G / 2) * nqb : 1ll * G * ((nqb + 1) / 2);
-    if (u < 1) u = 1;
-    if (u < units && u * per_unit < sms) {
-      auto rounds = [&](long long n) {
-        return units / n * ((n * per_unit + sms - 1) / sms) + (units % n * per_unit + sms - 1) / sms;
-      };
-      for (long long k = 1; k <= 5; ++k) {
-        const long long n = k == 5 || k * sms / per_unit > units ? units : k * sms / per_unit;
-        if (n > u && rounds(n) < rounds(u)) u = n;
-      }
-    }
-    p.group_units = int(u < 1 ? 1 : (u > B * H_KV ? B * H_KV : u));
+    p.group_units = group_for_fewest_rounds(u, 1ll * B * H_KV, per_unit, st->sm_count);
   }
   if (static_cast<long long>(B) * H * nqb > 0x3fffffffll) return HK_EINVAL;  // work items are indexed with int
   p.n_items = p.pair_heads ? B * H_KV * (G / 2) * nqb : B * H_KV * G * ((nqb + 1) / 2);
@@ -760,11 +763,13 @@ static int bwd_launch(const void* q, const void* k, const void* v, const void* o
   p.H_KV = H_KV;
   p.n_items = 0;
   {
-    // causal sweep groups: units whose Q, dO, K and V together stay within ~64 MB of L2
+    // causal sweep groups of the dQ kernel: units whose Q, dO, K and V together stay within ~64 MB of L2, in groups that
+    // need the fewest rounds (us per backward, before / now: B1 64 queries on 32768 keys H64/8 D128 894 / 555, B4 200 on 16384
+    // H16 D64 587 / 356, B2 512 on 16384 H8 D128 499 / 351)
     const int G = H / H_KV;
     const long long unit_bytes = 4ll * G * N * D + 4ll * NK * D;
-    long long u = (64ll << 20) / unit_bytes;
-    p.group_units = int(u < 1 ? 1 : (u > B * H_KV ? B * H_KV : u));
+    p.group_units = group_for_fewest_rounds((64ll << 20) / unit_bytes, 1ll * B * H_KV,
+                                            1ll * G * ((N + hk::kBlockM - 1) / hk::kBlockM), st->sm_count);
   }
   p.scale = softmax_scale > 0.f ? softmax_scale : 1.0f / std::sqrt(float(D));
   p.scale_log2 = p.scale * 1.4426950408889634f;
