@@ -60,3 +60,19 @@ def test_a_dependent_kernel_behind_it_finds_both_complete(shape):
         got = [hk.rotary_bnhd(t, cos, sin) for t in (dq, dk, dv)]
         for a, b in zip((dq, dk, dv, *got), (*ref, *want)):
             assert torch.equal(a, b)
+
+
+def test_dq_of_few_queries_on_many_keys_is_served_once():
+    """Groups of units of the causal dQ order: all units in one group here, two groups for the single batch elements."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+
+    def rand(n):
+        return torch.randn((3, n, 8, 128), generator=gen, device="cuda", dtype=torch.bfloat16)
+
+    q, d_o, k, v = rand(100), rand(100), rand(16384), rand(16384)
+    o, lse = hk.attn_fwd(q, k, v, causal=True)
+    got = backward(q, k, v, o, d_o, lse, torch.full_like(q, float("nan")), True)[0]
+    assert bool(torch.isfinite(got).all())
+    for i in range(3):
+        one = [t[i:i + 1].contiguous() for t in (q, k, v, o, d_o, lse)]
+        assert torch.equal(got[i:i + 1], backward(*one, torch.full_like(one[0], float("nan")), True)[0])
