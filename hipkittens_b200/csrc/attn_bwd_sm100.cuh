@@ -1010,7 +1010,7 @@ __device__ __forceinline__ DqItem decode_dq_item(const BwdParams& p, int idx) {
   }
   p.fd_hkv.divmod(unit, w.b, w.kvh);
   w.h = w.kvh * G + g;
-  w.kv_len = p.kv_lens ? min(max(p.kv_lens[w.b], 1), p.NK) : p.NK;
+  w.kv_len = p.kv_lens ? min(max(ptx::ld_gpu(p.kv_lens + w.b), 1), p.NK) : p.NK;
   w.off = w.kv_len - p.N;
   const int n_kv = (w.kv_len + kBlockN - 1) / kBlockN;
   // causal: the last row of the tile sees keys up to i*128 + 127 + off
@@ -1082,7 +1082,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   const uint32_t tmem = *tmem_slot;
   volatile uint32_t* abortp = abort_word;
   // Launched as a dependent of the dK/dV kernel, which it does not read from: its CTAs take over the SMs as that kernel
-  // leaves them. What both read is complete, because the dK/dV kernel has waited for it before it let this one start.
+  // leaves them. What both read is complete, because the dK/dV kernel has waited for it before it let this one start; what
+  // does not come by TMA is read past the SM's L1 all the same (ptx::ld_gpu says why).
   // The wait for the dK/dV kernel is the last thing a CTA does, so that who waits for this kernel waits for both.
   if (p.dq_waits) grid_dep_wait();
   grid_dep_launch();
@@ -1123,8 +1124,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         continue;
       }
-      const float nl = row_exists ? p.lse[srow] * -1.4426950408889634f : 0.f;
-      const float dl = row_exists ? p.delta[srow] : 0.f;
+      const float nl = row_exists ? ld_gpu(p.lse + srow) * -1.4426950408889634f : 0.f;
+      const float dl = row_exists ? ld_gpu(p.delta + srow) : 0.f;
       for (int n = 0; n < w.n_iter && ok; ++n, ++it) {
         // a key tile the diagonal (or the end of the kept keys) runs through: the tile's first row does not see
         // its last key

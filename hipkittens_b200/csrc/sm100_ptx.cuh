@@ -49,10 +49,26 @@ __device__ __forceinline__ bool elect_one() {
 // lets the compiler choose it): that path wants data that nobody writes while the grid exists, and the grid exists while
 // the kernel before is still writing; nor does the "memory" clobber hold such loads behind the wait. Coherent
 // loads cost 2 % of the prep kernel's time in a loop (see there) and nothing that shows in the others.
+// One kernel reads before it waits: the backward's dQ kernel, beside the dK/dV kernel in front of it. What it reads is of
+// kernels that have completed, since the dK/dV kernel has waited for them before it let this one start; but the wait makes
+// their writes visible to the grid that executes it, and nothing says so of a grid started from there. So it reads the
+// values that it does not fetch by TMA with ld_gpu(), which no cache of an SM answers, and waits at its end, so that
+// completion stays transitive.
 // What dependent launches are worth (us per pass in a loop, before -> after): B1 N256 D64 forward 8.3 -> 7.0, rotary twice
 // and attention of a 1511-token prompt 43.2 -> 38.3, one-token append and decode 16.4 -> 12.2.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Loads at the scope of the GPU: they are served by L2, whatever an SM's L1 holds.
+__device__ __forceinline__ float ld_gpu(const float* p) {
+  float v;
+  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_gpu(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

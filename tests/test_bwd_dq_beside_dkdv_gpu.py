@@ -76,3 +76,37 @@ def test_dq_of_few_queries_on_many_keys_is_served_once():
     for i in range(3):
         one = [t[i:i + 1].contiguous() for t in (q, k, v, o, d_o, lse)]
         assert torch.equal(got[i:i + 1], backward(*one, torch.full_like(one[0], float("nan")), True)[0])
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_every_call_reads_its_own_statistics_and_lengths(shape):
+    """L, delta and the key lengths of a call are written by the kernels just before its dK/dV kernel, into the buffers that
+    the call before it read: back to back, every call gives what it gives when each of them is waited for."""
+    B, N, H, HK, D, causal = shape
+    gen = torch.Generator(device="cuda").manual_seed(N + 1)
+    steps = []
+    for i in range(8):
+        q, k, v, d_o = (torch.randn((B, N, h, D), generator=gen, device="cuda", dtype=torch.bfloat16) * (1 + i % 3)
+                        for h in (H, HK, HK, H))
+        lens = torch.randint(1, N + 1, (B, 1), generator=gen, device="cuda")
+        steps.append((q, k, v, d_o, torch.arange(N, device="cuda")[None] < lens))
+
+    def chain(sync):
+        o, lse, seen = torch.empty_like(steps[0][0]), torch.empty((B, H, 1, N), device="cuda"), []
+        kv_lens = bad = None
+        for q, k, v, d_o, mask in steps:
+            del kv_lens, bad  # the next call's come to lie where they were
+            kv_lens, bad = _native.key_padding_lens(mask)
+            hk.attn_fwd(q, k, v, causal=causal, out=o, lse=lse, kv_lens=kv_lens)
+            if sync:
+                torch.cuda.synchronize()
+            grads = [torch.empty_like(t) for t in (q, k, v)]
+            _native.attn_bwd_strided(q, k, v, o, d_o, lse, *grads, causal=causal, kv_lens=kv_lens)
+            if sync:
+                torch.cuda.synchronize()
+            seen += grads
+        return seen
+
+    for a, b in zip(chain(False), chain(True)):
+        assert torch.equal(a, b)
+    assert _native.device_status(0) == 0
