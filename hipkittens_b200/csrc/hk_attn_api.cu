@@ -709,14 +709,15 @@ struct BwdStrides {
   const long long *q, *k, *v, *dq, *dk, *dv;
 };
 
-// Whether two [B, N, H, D] tensors of 16-bit elements, given by address and strides, may share memory.
-static bool overlap(const void* a, const long long* a_strides, const void* b, const long long* b_strides, int B, int N, int H,
-                    int D) {
-  auto end = [&](const void* p, const long long* s) {
-    return reinterpret_cast<uintptr_t>(p) + 2 * ((B - 1) * s[0] + (N - 1) * s[1] + (H - 1) * s[2] + D);
-  };
-  return reinterpret_cast<uintptr_t>(a) < end(b, b_strides) && reinterpret_cast<uintptr_t>(b) < end(a, a_strides);
-}
+// The addresses from the first byte of an input or output to behind its last, and whether two of them may share memory.
+struct Span {
+  uintptr_t begin, end;
+  Span(const void* p, long long bytes) : begin(reinterpret_cast<uintptr_t>(p)), end(begin + uintptr_t(bytes)) {}
+  // of a [B, N, H, D] tensor of 16-bit elements with these strides
+  Span(const void* p, const long long* strides, int B, int N, int H, int D)
+      : Span(p, 2 * ((B - 1) * strides[0] + (N - 1) * strides[1] + (H - 1) * strides[2] + D)) {}
+  bool meets(const Span& o) const { return begin < o.end && o.begin < end; }
+};
 
 // Shared tail of the backward entries. o != null: delta is computed here first.
 static int bwd_launch(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse,
@@ -779,8 +780,14 @@ static int bwd_launch(const void* q, const void* k, const void* v, const void* o
   p.trace = g_trace_buf;
 #endif
   // The dQ kernel starts while the dK/dV kernel is still reading, unless it would write over what that reads: dQ in the place
-  // of Q or of dO is as good as anywhere else when one kernel follows the other.
-  const bool dq_beside = !overlap(dq, s.dq, q, s.q, B, N, H, D) && !overlap(dq, s.dq, d_o, dos, B, N, H, D);
+  // of an input whose rows are read by the CTA that writes there, and before it does (Q and dO; K and V with one tile of
+  // each and as many K/V heads as heads), is as good as anywhere else when one kernel follows the other.
+  const Span out(dq, s.dq, B, N, H, D);
+  const long long stats = 4ll * B * H * N;
+  const bool dq_beside = !out.meets({q, s.q, B, N, H, D}) && !out.meets({d_o, dos, B, N, H, D}) &&
+                         !out.meets({k, s.k, B, NK, H_KV, D}) && !out.meets({v, s.v, B, NK, H_KV, D}) &&
+                         !out.meets({lse, stats}) && !out.meets({delta, stats}) &&
+                         !(kv_lens && out.meets({kv_lens, 4ll * B}));
   if (D == 128) return causal ? launch_bwd<128, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, st->bwd_clusters, stream)
                               : launch_bwd<128, false>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, st->bwd_clusters, stream);
   return causal ? launch_bwd<64, true>(tq, tk, tv, tdo, p, B, N, NK, H, H_KV, dq_beside, st->sm_count, st->bwd_clusters, stream)

@@ -110,3 +110,19 @@ def test_every_call_reads_its_own_statistics_and_lengths(shape):
     for a, b in zip(chain(False), chain(True)):
         assert torch.equal(a, b)
     assert _native.device_status(0) == 0
+
+
+@pytest.mark.parametrize("shape", [(1, 128, 8, 8, 128, False), (3, 100, 4, 4, 64, True), (40, 120, 8, 8, 128, True)])
+def test_dq_in_the_place_of_a_single_key_tile(shape):
+    """With one tile of queries and one of keys, and as many K/V heads as heads, a dQ tile may lie where the only K or V tile
+    that its CTA reads lay."""
+    causal = shape[-1]
+    q, k, v, d_o, o, lse = inputs(*shape)
+    ref = [t.clone() for t in backward(q, k, v, o, d_o, lse, torch.empty_like(q), causal)]
+    for _ in range(5):
+        k2, v2 = k.clone(), v.clone()
+        for a, b in zip(backward(q, k2, v, o, d_o, lse, k2, causal), ref):
+            assert torch.equal(a, b)
+        for a, b in zip(backward(q, k, v2, o, d_o, lse, v2, causal), ref):
+            assert torch.equal(a, b)
+    assert _native.device_status(0) == 0
