@@ -163,9 +163,9 @@ def _lens_from_key_padding_mask(mask: torch.Tensor, packed: torch.Tensor):
     assert packed.is_cuda, "All tensors must be on CUDA device"
     if mask.device != packed.device:
         raise RuntimeError("key_padding_mask must be on the device of q, k and v")
-    # pinned memory, which the forward's synchronisation makes readable: a flag on the device cost a fill, a copy and a
-    # synchronisation of its own
-    return key_padding_lens(mask, torch.zeros((), dtype=torch.int32, pin_memory=True))
+    # pinned memory (of the CPU, whatever the default device is), which the forward's synchronisation makes readable: a flag
+    # on the device cost a fill, a copy and a synchronisation of its own
+    return key_padding_lens(mask, torch.zeros((), dtype=torch.int32, device="cpu", pin_memory=True))
 
 
 class HipSelfAttention(nn.Module):

@@ -153,3 +153,18 @@ def test_a_refused_mask_leaves_the_next_call_alone():
         with pytest.raises(ValueError):
             module(qkv, key_padding_mask=bad)
         assert torch.equal(module(qkv, key_padding_mask=good), ref)
+
+
+@pytest.mark.parametrize("default", ["cuda", "cuda:0"])
+def test_a_mask_under_a_default_device(default):
+    """The verdict's flag lies in host memory wherever tensors are made by default."""
+    qkv = torch.randn(2, 80, 3, 2, 64, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda().requires_grad_()
+    mask = (torch.arange(80)[None] < torch.tensor([80, 33])[:, None]).cuda()
+    module = HipSelfAttention(causal=True)
+    ref = module(qkv, key_padding_mask=mask)
+    with torch.device(default):
+        out = module(qkv, key_padding_mask=mask)
+        out.backward(torch.ones_like(out))
+        with pytest.raises(ValueError):
+            module(qkv, key_padding_mask=~mask)
+    assert torch.equal(out, ref) and bool(torch.isfinite(qkv.grad).all())
