@@ -1046,6 +1046,17 @@ int hk_selftest_dkdv_in_pairs(int B, int Nq, int Nk, int H, int H_KV, int D, int
   return deal_in_pairs(B * H_KV, H / H_KV, Nq, nbk, D, sm_count) ? 1 : 0;
 }
 
+int hk_selftest_decode_shape(int S, int H_KV, int max_pages, int sm_count, const int* clusters, int clusters8, int* warps) {
+  if (!hk::decode_shape_supported(S, H_KV, max_pages) || sm_count <= 0 || !clusters || !warps) return HK_EINVAL;
+  hk::DecodeLimits lim;
+  lim.sm_count = sm_count;
+  for (int n = 2; n <= hk::kMaxCluster; ++n) lim.clusters4[n] = clusters[n];
+  lim.clusters8 = clusters8;
+  const hk::DecodeShape shape = hk::decode_pick_shape(S, H_KV, max_pages, lim);
+  *warps = shape.warps;
+  return shape.cluster;
+}
+
 int hk_selftest_fastdiv(void) {
   // host only: the multiply-and-shift division of the item decode against the division it replaces, for every
   // divisor up to 4096, divisors around every power of two, and dividends at the edges of [0, 2^31)

@@ -75,17 +75,29 @@ struct DecodeLimits {
 //    one fits, and one size too many costs more than it gives. us, chunks / clusters of that size / of another, H_KV 8 unless
 //    said: 1 x 3250 tokens 10.4 / 7.6 (16) / 8.0 (8); 4 x 750 10.1 / 6.3 (8) / 6.7 (4), 11.4 (16); 8 x 2500 20.6 / 17.0
 //    (4) / 22.6 (2), 19.0 (8); 40 x 1650 of H_KV 1 13.3 / 10.9 (6) / 14.1 (7).
-//  * Units for more than a wave in clusters of 3: CTAs of their own, of 8 warps while one per SM is enough or contexts may be
-//    above 1024 tokens: 16 x 1250 20.5 / 15.0, 32 x 600 18.8 / 14.5 (8 warps: 15.0), 64 x 300 21.1 / 16.6 (21.7), 32 x 2000
-//    52.4 / 45.1 (4 warps: 48.3). Clusters of several waves gain up to 5 % on long contexts (64 x 4350: 182 / 174 in
-//    clusters of 4), but where most of the table's width is empty their idle CTAs cost more than those of the chunks (64 x 300
-//    tokens in tables for 8192: 24 / 47), so those stay in chunks.
+//  * How much of one context a CTA may meet is bounded: the table may be as wide as it is for one long context among short
+//    ones, which its own cluster then reads alone (12.5 us per 1000 tokens of a CTA of 4 warps, 5.5 with 8), where chunks
+//    would spread it over the GPU. The lines are where that costs the one long context about as much as batches of equal
+//    lengths gain. us, chunks / this, one context as long as the table beside others of 100 tokens, then all that long, then
+//    all a quarter of that:
+//    CTAs of 4 warps in clusters, 64 pages each: 8 x 3072 tokens of H_KV 8 (48 pages each) 10.8 / 10.4, 22.3 / 16.6, 11.7 / 6.7; 8 x
+//    4096 10.8 / 12.4, 30.5 / 25.3, 11.9 / 7.2; 64 x 4096 of H_KV 1 9.8 / 11.9, 30.2 / 25.1, 12.3 / 7.3; behind the line 8 x 8192
+//    12.3 / 19.8, 53.7 / 45.2, 14.0 / 10.0.
+//    CTAs of their own of 8 warps (units for more than a wave in clusters of 3), 96 pages: 16 x 1408 10.8 / 10.7, 20.1 /
+//    15.3, 9.1 / 5.6; 32 x 1536 11.1 / 11.4, 43.2 / 36.7, 10.6 / 10.4; behind the line 12 x 2560 10.4 / 16.5, 29.1 / 24.5, 12.3 /
+//    7.2, 32 x 2048 10.3 / 14.0, 52.7 / 45.9, 12.5 / 11.9.
+//    Of 4 warps, while one wave of those with 8 is not enough, 64 pages: 24 x 1024 10.6 / 11.2, 22.8 / 19.7, 8.1 / 6.3; 32 x 1024
+//    10.6 / 12.5, 30.7 / 24.8, 8.6 / 6.3 (8 warps 8.9, 27.6, 9.1).
+//    With units for more than two waves of those of 8 they are the better ones throughout, and the chunks are slower with the one
+//    long context too: 80 pages, 64 x 1152 15.2 / 12.8, 57.6 / 49.9, 16.3 / 12.9 (8 warps 13.4, 55.2, 19.0).
+//    One wave of CTAs of 8 warps also serves 160 pages where the chunks need more than two waves: then all but the one long
+//    context gain most (18 x 2560 10.8 / 16.5, 40.9 / 32.6, 13.7 / 7.1, lengths evenly up to 2560 21.5 / 18.4).
+//  * Clusters of several waves gain up to 5 % on long contexts (64 x 4350: 182 / 174 in clusters of 4), but where most of the
+//    table's width is empty their idle CTAs cost more than those of the chunks (64 x 300 tokens in tables for 8192: 24 / 47),
+//    so those stay in chunks.
 //  * Few units with long contexts: 16 CTAs of 4 warps fall behind the chunks from some 700 tokens each on (1 x 14000 13.5 /
 //    14.7); up to 6 units the CTAs can have 8 warps (H_KV 1, 1 x 16000: 11.7 / 11.0, 4 warps 12.5; below 4096 tokens 4
 //    warps are better, 1 x 2000: 9.4 / 5.4, 8 warps 6.2).
-//  * One long context among short ones is shared by its own cluster only (12.5 us per 1000 tokens of a CTA of 4 warps, 5.5
-//    with 8), where chunks would spread it over the GPU (1 x 2000 beside 31 x 100: 10.6 / 14.0); so no more than 2048 (2560)
-//    tokens per CTA.
 struct DecodeShape {
   int cluster, warps;
 };
@@ -96,13 +108,15 @@ inline DecodeShape decode_pick_shape(int S, int H_KV, int max_pages, const Decod
   while (cluster > 1 && lim.clusters4[cluster] < units) --cluster;
   if (cluster < 3) {
     cluster = 1;
-    warps = units <= lim.sm_count || max_pages > 64 ? 8 : 4;
-    if (max_pages > 160) return kChunks;
+    const bool one_wave = units <= lim.sm_count, two_waves = units <= 2ll * lim.sm_count;
+    const bool many_chunks = units * max_pages > 4ll * lim.sm_count * kChunkPagesMin;
+    warps = one_wave || (two_waves && max_pages > 64) ? 8 : 4;
+    if (max_pages > (one_wave && many_chunks ? 160 : two_waves ? 96 : 80)) return kChunks;
   } else if (max_pages > 256 && units <= lim.clusters8) {
     cluster = kMaxCluster;
     warps = 8;
     if (max_pages > 64 * cluster) return kChunks;
-  } else if (max_pages > (cluster == kMaxCluster ? 44 : 128) * cluster) {
+  } else if (max_pages > (cluster == kMaxCluster ? 44 : 64) * cluster) {
     return kChunks;
   }
   const int useful = (max_pages + warps - 1) / warps;  // a page per warp

@@ -284,6 +284,12 @@ int hk_selftest_fastdiv(void);
  * of equal cost, 0 = singly, the longest first; a negative HK_E* code for what hk_attn_bwd_cross would refuse. */
 int hk_selftest_dkdv_in_pairs(int B, int Nq, int Nk, int H, int H_KV, int D, int sm_count);
 
+/* Host-only self-test: how hk_attn_paged_decode spreads the contexts of such a call on a GPU of sm_count SMs that holds
+ * clusters[n] clusters of n CTAs of 4 warps (n from 2 to 16) and clusters8 clusters of 16 CTAs of 8 warps: the size of a
+ * cluster (0: chunks and a combining kernel), and in *warps the warps of a CTA. */
+int hk_selftest_decode_shape(int S, int H_KV, int max_pages_per_seq, int sm_count, const int* clusters, int clusters8,
+                             int* warps);
+
 /* Number of kernels this library has launched in the calling process (all devices). */
 unsigned long long hk_kernel_launch_count(void);
 
