@@ -44,6 +44,7 @@ EXPORTED_SYMBOLS = (
     "hk_selftest_bounded_wait",
     "hk_selftest_fastdiv",
     "hk_selftest_dkdv_in_pairs",
+    "hk_selftest_bwd_dealing",
     "hk_selftest_decode_shape",
     "hk_kernel_launch_count",
     "hk_strerror",
@@ -130,6 +131,8 @@ def capi() -> ctypes.CDLL:
     lib.hk_selftest_fastdiv.restype = ci
     lib.hk_selftest_dkdv_in_pairs.argtypes = [ci] * 7
     lib.hk_selftest_dkdv_in_pairs.restype = ci
+    lib.hk_selftest_bwd_dealing.argtypes = [ci] * 8 + [ctypes.POINTER(ci)] * 2
+    lib.hk_selftest_bwd_dealing.restype = ci
     lib.hk_selftest_decode_shape.argtypes = [ci] * 4 + [ctypes.POINTER(ci), ci, ctypes.POINTER(ci)]
     lib.hk_selftest_decode_shape.restype = ci
     lib.hk_kernel_launch_count.argtypes = []

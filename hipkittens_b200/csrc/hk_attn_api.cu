@@ -438,15 +438,25 @@ int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count, const int* clusters) {
 // The dQ kernel may run on the SMs that the dK/dV kernel (of `grid` CTAs) leaves, or behind it. Returns its CTAs, negative if
 // they wait for the dK/dV kernel.
 //  * With a CTA for every SM those that find an SM early do their share and the others start when the dK/dV kernel has
-//    ended. That fills gaps (us behind / beside, in a loop: B1 N512 H8/8 D128 23.6 / 15.3, B4 N1024 H12 D64 85 / 70, B2 N2615
-//    H8 D64 153 / 129, B6 N820 H16 D128 141 / 135), but two kernels at a time also cost the key blocks that are still
-//    running: longer calls are better off one after the other (D128 B2 N4096 H4 193 / 203, B13 N505 H32/8 203 / 215; B1
-//    N4096 H32/8 causal 392 / 408; D64 B6 N7554 H6/2 1 981 / 2 067). So do calls of causal groups of 3 heads and more that
-//    take three quarters of the SMs in one round of single blocks (B5 N300 H32/8 53 / 61, B7 N457 H32/4 104 / 117).
+//    ended. That fills gaps (us behind / beside, in a loop: B1 N512 H8/8 D128 23.6 / 15.3, B4 N1024 H12 D64 85 / 70, B6 N567
+//    H4 D128 causal 29.3 / 23.8, B1 N2560 H8 D64 causal 56.4 / 42.7), but two kernels at a time also cost the key blocks that
+//    are still running: longer calls are better off one after the other (D128 B2 N4096 H4 193 / 203, B13 N505 H32/8 203 /
+//    215; B1 N4096 H32/8 causal 392 / 408; D64 B6 N7554 H6/2 1 981 / 2 067). So are those whose key blocks all run long, and
+//    as long, while dQ comes to them: groups of heads on blocks for 5/8 of a round of the SMs and more (B5 N1408 H8/2 D64 101
+//    / 118, B4 N940 H16/8 D64 89 / 105, B3 N1405 H16/4 D64 116 / 129) or with a last round more than a quarter full (B6
+//    N1129 H16/4 D64 164 / 189), single heads with one more than 0.6 full (B8 N2176 H4 D64 166 / 182; 0.4 full: B9 N1100 H8
+//    D128 180 / 167); of causal blocks, whose lengths differ, groups of 3 heads and more on 3/4 to 1.4 rounds (B5 N300 H32/8
+//    53 / 61, B7 N457 H32/4 104 / 117, B2 N1280 H64/8 D128 233 / 259, B3 N2073 H16/4 D64 151 / 162) unless there are
+//    24 lengths of them (B5 N4218 H4/1 D64 254 / 241); either with groups of 8 from 3/8 of a round on (B4 N295 H64/8 D64 68 /
+//    81, B10 N256 H32/4 D64 causal 49 / 55); and pairs (B9 N2857 H8/4 D64 348 / 360; 0.98 to 1.11 of the time behind). Of
+//    2465 shapes of 20 to 600 us, 5 take more than 2.5 % longer than behind in a loop, 5 % at most (121 and 21 % without these
+//    lines); what the lines give up of calls waited for one by one is 0.1 % on average.
 //  * When the last round of key blocks leaves many SMs free, these are dealt all of dQ, if that is estimated to end sooner: in
 //    the pairs of dkdv_split, a dQ item costs 1 and 0.45 per pair alone, 1.5 and 0.65 beside dK/dV. us behind / all SMs /
-//    the free ones (D128 unless said): B5 N512 H32/8 108 / 101 / 78, B1 N2500 H32/8 420 / 383 / 285, B11 N1000 H16/2 D64
-//    263 / 281 / 217, B6 N900 H12/4 141 / 149 / 130, B4 N293 H16 D64 32 / 30 / 25.
+//    the free ones (D128 unless said), calls waited for one by one: B5 N512 H32/8 108 / 101 / 78, B1 N2500 H32/8 420 / 383 / 285,
+//    B11 N1000 H16/2 D64 263 / 281 / 217, B6 N900 H12/4 141 / 149 / 130, B4 N293 H16 D64 32 / 30 / 25. In a loop the next call
+//    fills such SMs too, and less or nothing is left of it: B2 N1511 H24/8 D64 158 / 160 / 139 one by one, 152 / 160 / 156 in a
+//    loop, B1 N1408 H24/8 D128 101 / 100 / 88, 97 / 99 / 103.
 template <int D, bool CAUSAL>
 int dq_ctas(const hk::BwdParams& p, int nbq, int nbk, int grid, int sm_count) {
   const long long items = 1ll * p.B * p.H * nbq;
@@ -474,8 +484,14 @@ int dq_ctas(const hk::BwdParams& p, int nbq, int nbk, int grid, int sm_count) {
   }
   const long long tiles = 1ll * p.B * p.H * nbq * nbk;
   const bool long_call = tiles > (D == 64 ? 300ll : CAUSAL ? 120ll : 40ll) * grid;
-  const bool long_blocks = CAUSAL && p.split == 1 && p.n_pairs == 0 && p.G >= 3 && grid < sm_count && 4 * grid > 3 * sm_count;
-  return long_call || long_blocks ? -all : all;
+  bool held_up = p.n_pairs > 0;  // the key blocks, by dQ beside them
+  if (p.split == 1 && p.n_pairs == 0) {
+    const double full = double(p.n_items) / sm_count, from = p.G >= 8 ? 3.0 / 8 : CAUSAL ? 3.0 / 4 : 5.0 / 8;
+    if (CAUSAL) held_up = p.G >= 3 && full > from && full <= 1.4 && nbk < 24;
+    else if (rounds == 1) held_up = p.G >= 2 && full > from;
+    else held_up = last > (p.G == 1 ? 0.6 : 0.25) * sm_count;
+  }
+  return long_call || held_up ? -all : all;
 }
 
 template <int D, bool CAUSAL>
@@ -1044,6 +1060,26 @@ int hk_selftest_dkdv_in_pairs(int B, int Nq, int Nk, int H, int H_KV, int D, int
   const int nbk = (Nk + hk::kBlockN - 1) / hk::kBlockN;
   if (static_cast<long long>(B) * H_KV * nbk > 0x3fffffffll) return HK_EINVAL;
   return deal_in_pairs(B * H_KV, H / H_KV, Nq, nbk, D, sm_count) ? 1 : 0;
+}
+
+int hk_selftest_bwd_dealing(int B, int Nq, int Nk, int H, int H_KV, int D, int causal, int sm_count, const int* clusters,
+                            int* dq_ctas_out) {
+  if (B <= 0 || Nq <= 0 || Nk <= 0 || H <= 0 || H_KV <= 0 || H % H_KV != 0 || sm_count <= 0 || !clusters || !dq_ctas_out)
+    return HK_EINVAL;
+  if (D != 64 && D != 128) return HK_EUNSUPPORTED;
+  const int nbq = (Nq + hk::kBlockM - 1) / hk::kBlockM, nbk = (Nk + hk::kBlockN - 1) / hk::kBlockN;
+  if (static_cast<long long>(B) * H * nbq > 0x3fffffffll || static_cast<long long>(B) * H_KV * nbk > 0x3fffffffll)
+    return HK_EINVAL;
+  hk::BwdParams p = {};
+  p.B = B, p.N = Nq, p.NK = Nk, p.H = H, p.H_KV = H_KV, p.G = H / H_KV;
+  p.group_units = 1;
+  auto deal = [&](auto dkdv, auto dq) {
+    const int grid = dkdv(p, nbk, sm_count, clusters);
+    *dq_ctas_out = dq(p, nbq, nbk, grid, sm_count);
+    return p.split;
+  };
+  if (D == 128) return causal ? deal(deal_dkdv<128, true>, dq_ctas<128, true>) : deal(deal_dkdv<128, false>, dq_ctas<128, false>);
+  return causal ? deal(deal_dkdv<64, true>, dq_ctas<64, true>) : deal(deal_dkdv<64, false>, dq_ctas<64, false>);
 }
 
 int hk_selftest_decode_shape(int S, int H_KV, int max_pages, int sm_count, const int* clusters, int clusters8, int* warps) {

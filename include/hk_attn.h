@@ -284,6 +284,12 @@ int hk_selftest_fastdiv(void);
  * of equal cost, 0 = singly, the longest first; a negative HK_E* code for what hk_attn_bwd_cross would refuse. */
 int hk_selftest_dkdv_in_pairs(int B, int Nq, int Nk, int H, int H_KV, int D, int sm_count);
 
+/* Host-only self-test: how the backward deals such a call to a GPU of sm_count SMs that holds clusters[n] clusters of n dK/dV
+ * CTAs (n from 2 to 8): how many CTAs share a key block, and in *dq_ctas the CTAs of the dQ kernel, negative if they wait for
+ * the dK/dV kernel. A negative HK_E* code for what hk_attn_bwd_cross would refuse. */
+int hk_selftest_bwd_dealing(int B, int Nq, int Nk, int H, int H_KV, int D, int causal, int sm_count, const int* clusters,
+                            int* dq_ctas);
+
 /* Host-only self-test: how hk_attn_paged_decode spreads the contexts of such a call on a GPU of sm_count SMs that holds
  * clusters[n] clusters of n CTAs of 4 warps (n from 2 to 16) and clusters8 clusters of 16 CTAs of 8 warps: the size of a
  * cluster (0: chunks and a combining kernel), and in *warps the warps of a CTA. */
