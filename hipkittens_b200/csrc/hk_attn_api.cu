@@ -365,9 +365,13 @@ bool deal_in_pairs(int units, int G, int N, int nbk, int D, int sm_count) {
 // longer than the best on average, never to split 20 %. us per backward, 1 / chosen: B1 N1024 H8/1 D128 causal 108 / 33 (8),
 // B1 N4096 H8/1 D128 488 / 214 (4), B1 N8192 H8/1 D128 causal 936 / 423 (3), B1 N2048 H8/1 D64 causal 164 / 38 (8),
 // B2 N384 H8/2 D128 causal 28 / 21 (4), B2 N1024 H16/4 D128 87 / 71 (2).
-// A block's sums are split in other places than those of a call that does not, so a batch element's gradients are not
-// those of the same element in a larger batch to the last bit. Clusters of several waves are therefore taken only for
-// half the time, and pairs of CTAs not for causal calls.
+// A block's sums are split in other places than those of a call that does not split it, so a batch element's dK and dV are not
+// those of the same element in a batch, or a shard, of another size to the last bit. Two limits keep that to the calls that
+// gain most, and cost the others what they would gain: causal calls take no pairs of CTAs, and clusters of several waves have
+// to take half the time. us per backward in a loop, 1 / 2 / 3 / 4 CTAs per block: causal B1 N2048 H16/4 D128 131 / 90 / 81 /
+// 84, B1 N2944 H16/4 D64 149 / 101 / 107 / 108, B1 N1536 H24/8 D128 87 / 68 / 90 / 93, B2 N2048 H16/4 D128 163 / 126 / 152 /
+// 163, B1 N3000 H32/8 D64 193 / 185 / 214 / 222 (all stay whole). Without a causal mask they cost nothing: B1 N2944 H16/4 D128
+// 244 / 257 / 244 / 235, B2 N2048 H16/4 D128 204 / 220 / 240 / 252, B1 N4096 H32/4 D128 825 / 844 / 856 / 873.
 int dkdv_split(int units, int G, int N, int NK, bool causal, int sm_count, const int* clusters) {
   const int nbq = (N + hk::kBlockM - 1) / hk::kBlockM, nbk = (NK + hk::kBlockN - 1) / hk::kBlockN;
   if (1ll * units * nbk > 2ll * sm_count) return 1;

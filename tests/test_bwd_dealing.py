@@ -1,4 +1,4 @@
-"""When the backward's dQ kernel runs beside the dK/dV kernel, by what either order was measured to take in a loop."""
+"""How many CTAs share a key block of the dK/dV kernel, and when the dQ kernel runs beside it, by what was measured."""
 import ctypes
 
 import pytest
@@ -14,6 +14,30 @@ def deal(B, N, H, H_KV, D, causal, NK=None):
     held, ctas = (ctypes.c_int * 9)(0, 0, *HELD), ctypes.c_int()
     split = hk.capi().hk_selftest_bwd_dealing(B, N, NK or N, H, H_KV, D, int(causal), 148, held, ctypes.byref(ctas))
     return split, ctas.value
+
+
+# us per backward, alone / shared
+@pytest.mark.parametrize("shape,split", [
+    ((1, 1024, 8, 1, 128, True), 8),    # 108 / 33
+    ((1, 4096, 8, 1, 128, False), 4),   # 488 / 214
+    ((1, 8192, 8, 1, 128, True), 3),    # 936 / 423
+    ((1, 2048, 8, 1, 64, True), 8),     # 164 / 38
+    ((2, 384, 8, 2, 128, True), 4),     # 28 / 21
+    ((2, 1024, 16, 4, 128, False), 2),  # 87 / 71
+    # not shared, so that a batch element's gradients are the same bits in a batch of any size: 131 / 81, 149 / 101, 163 / 126
+    ((1, 2048, 16, 4, 128, True), 1), ((1, 2944, 16, 4, 64, True), 1), ((2, 2048, 16, 4, 128, True), 1),
+    # nothing to gain: 204 / 220, 825 / 844, more than two blocks per SM
+    ((2, 2048, 16, 4, 128, False), 1), ((1, 4096, 32, 4, 128, False), 1), ((16, 2048, 64, 8, 128, False), 1),
+])
+def test_key_blocks_are_shared_where_they_are_few(native_built, shape, split):
+    assert deal(*shape)[0] == split
+
+
+def test_no_cluster_that_the_gpu_does_not_hold(native_built):
+    held, ctas = (ctypes.c_int * 9)(0, 0, 74, 45, 33), ctypes.c_int()
+    for n, want in ((8, 4), (3, 3), (2, 1), (0, 1)):  # causal calls take no pairs
+        sizes = (ctypes.c_int * 9)(*[held[i] if i <= n else 0 for i in range(9)])
+        assert hk.capi().hk_selftest_bwd_dealing(1, 1024, 1024, 8, 1, 128, 1, 148, sizes, ctypes.byref(ctas)) == want
 
 
 # us per backward in a loop: behind / beside
