@@ -449,12 +449,13 @@ int deal_dkdv(hk::BwdParams& p, int nbk, int sm_count, const int* clusters) {
 //    as long, while dQ comes to them: groups of heads on blocks for 5/8 of a round of the SMs and more (B5 N1408 H8/2 D64 101
 //    / 118, B4 N940 H16/8 D64 89 / 105, B3 N1405 H16/4 D64 116 / 129) or with a last round more than a quarter full (B6
 //    N1129 H16/4 D64 164 / 189), single heads with one more than 0.6 full (B8 N2176 H4 D64 166 / 182; 0.4 full: B9 N1100 H8
-//    D128 180 / 167); of causal blocks, whose lengths differ, groups of 3 heads and more on 3/4 to 1.4 rounds (B5 N300 H32/8
-//    53 / 61, B7 N457 H32/4 104 / 117, B2 N1280 H64/8 D128 233 / 259, B3 N2073 H16/4 D64 151 / 162) unless there are
-//    24 lengths of them (B5 N4218 H4/1 D64 254 / 241); either with groups of 8 from 3/8 of a round on (B4 N295 H64/8 D64 68 /
-//    81, B10 N256 H32/4 D64 causal 49 / 55); and pairs (B9 N2857 H8/4 D64 348 / 360; 0.98 to 1.11 of the time behind). Of
-//    2465 shapes of 20 to 600 us, 5 take more than 2.5 % longer than behind in a loop, 5 % at most (121 and 21 % without these
-//    lines); what the lines give up of calls waited for one by one is 0.1 % on average.
+//    D128 180 / 167) and no key lengths, which leave rounds that are not known here (B16 N512 H16 D64 97 / 86 when padded);
+//    of causal blocks, whose lengths differ, groups of 3 heads and more on 3/4 to 1.4 rounds (B5 N300 H32/8 53 / 61, B7
+//    N457 H32/4 104 / 117, B2 N1280 H64/8 D128 233 / 259, B3 N2073 H16/4 D64 151 / 162) unless there are 24 lengths of them
+//    (B5 N4218 H4/1 D64 254 / 241); either with groups of 8 from 3/8 of a round on (B4 N295 H64/8 D64 68 / 81, B10 N256
+//    H32/4 D64 causal 49 / 55); and pairs (B9 N2857 H8/4 D64 348 / 360; 0.98 to 1.11 of the time behind). Of 2465 shapes of
+//    20 to 600 us, 5 take more than 2.5 % longer than behind in a loop, 5 % at most (121 and 21 % without these lines);
+//    what the lines give up of calls waited for one by one is 0.1 % on average.
 //  * When the last round of key blocks leaves many SMs free, these are dealt all of dQ, if that is estimated to end sooner: in
 //    the pairs of dkdv_split, a dQ item costs 1 and 0.45 per pair alone, 1.5 and 0.65 beside dK/dV. us behind / all SMs /
 //    the free ones (D128 unless said), calls waited for one by one: B5 N512 H32/8 108 / 101 / 78, B1 N2500 H32/8 420 / 383 / 285,
@@ -493,7 +494,7 @@ int dq_ctas(const hk::BwdParams& p, int nbq, int nbk, int grid, int sm_count) {
     const double full = double(p.n_items) / sm_count, from = p.G >= 8 ? 3.0 / 8 : CAUSAL ? 3.0 / 4 : 5.0 / 8;
     if (CAUSAL) held_up = p.G >= 3 && full > from && full <= 1.4 && nbk < 24;
     else if (rounds == 1) held_up = p.G >= 2 && full > from;
-    else held_up = last > (p.G == 1 ? 0.6 : 0.25) * sm_count;
+    else held_up = p.G == 1 ? !p.kv_lens && last > 0.6 * sm_count : last > 0.25 * sm_count;
   }
   return long_call || held_up ? -all : all;
 }
