@@ -9,7 +9,8 @@
 // With P = exp(scale * Q K^T - L), dP = dO V^T and dS = P * (dP - delta):
 //     dV = P^T dO        dK = scale * dS^T Q        dQ = scale * dS K
 // The reference accumulates dQ with packed-bf16 atomic adds from the kernel that owns a K/V block. Here
-// nothing is accumulated across thread blocks: two kernels each own their outputs outright, which makes
+// nothing is accumulated with atomics: two kernels each own their outputs - dQ by query tile, dK and dV by key block, or by
+// the cluster of CTAs that shares a block and adds its partial sums up in a fixed order -, which makes
 // every gradient bit-reproducible from run to run, at the price of computing S and dP twice.
 //   attn_bwd_dkdv_kernel  one K/V block of 128 keys stays in shared memory; the query tiles of all heads
 //                         of the group stream past it. Everything is computed transposed (S^T = K Q^T,
@@ -17,7 +18,7 @@
 //                         already in the A-operand position of dV += P^T dO and dK += dS^T Q.
 //   attn_bwd_dq_kernel    one query tile of 128 rows stays in shared memory; the K/V tiles stream past it:
 //                         S = Q K^T, dP = dO V^T, dQ += dS K.
-// Both kernels are persistent (one CTA per SM, 384 threads): warps 0-7 do the element-wise work
+// Both kernels run one CTA per SM, of 384 threads, persistent but where CTAs share a key block: warps 0-7 do the element-wise work
 // (two threads per TMEM lane, 64 columns each), then one warp each for the TMA producer, the two UMMA-issuing
 // roles and, in the dK/dV kernel, the loader of the per-row statistics.
 // TMEM is laid out so that a score-shaped accumulator is free for the next product as soon as the element-wise
@@ -270,18 +271,6 @@ __device__ __forceinline__ void bwd_issue_ss(uint32_t d_tmem, uint32_t a_lo, uin
     const uint32_t off = (k / 4) * sub16 + (k % 4) * 2;  // 32 bytes per 16-element step inside a 128-byte row
     ptx::umma_ss_lohi(d_tmem, a_lo + off, b_lo + off, desc_hi, idesc, k > 0 ? 1u : 0u);
   }
-}
-// Gradient-shaped product: d[128 x D] (+)= a * b, a = bf16 [128 x 128] in TMEM (each of the kBwdParts thread
-// groups of a row keeps its packed columns inside the kBwdPC columns it owns, starting at `a_tmem`),
-// b = a 128 x D tile in shared memory read MN-major (its rows are the contraction index).
-template <int D>
-__device__ __forceinline__ void bwd_issue_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo_mn, bool acc) {
-  constexpr uint32_t idesc = ptx::make_idesc_bf16(kBlockM, D, true);
-  constexpr uint32_t desc_hi = ptx::smem_desc_hi(1024);
-#pragma unroll
-  for (int k = 0; k < kBlockN / 16; ++k)
-    ptx::umma_ts_lohi(d_tmem, a_tmem + ((16 * k) / kBwdPC) * kBwdPC + ((16 * k) % kBwdPC) / 2, b_lo_mn + k * 128,
-                      desc_hi, idesc, (acc || k > 0) ? 1u : 0u);
 }
 
 // Accumulator rows (this thread's TMEM lane, D / kBwdParts columns from `taddr`) -> bf16 -> global, scaled.

@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 1 : 2) paged_decode_split_ker
   const int g = lane >> 2, t = lane & 3;
   const int total_pages = (ctx + kPageTokens - 1) / kPageTokens;
   // This warp's pages: page_first, page_first + page_step, ... below page_end. A CTA of a cluster takes every n_used-th
-  // group of four, so that whatever the length the live CTAs of a cluster differ by a page per warp at most.
+  // group of W pages, so that whatever the length the live CTAs of a cluster differ by a page per warp at most.
   int n_used, page_first, page_step, page_end;
   if constexpr (CLUSTER) {
     if (ctx <= 0) {  // defined output for an empty context
@@ -349,11 +349,11 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 1 : 2) paged_decode_split_ker
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
 
-  // ---- merge the 4 warps through shared memory (the ring is idle now)
+  // ---- merge the W warps through shared memory (the ring is idle now)
   __syncthreads();
-  float* sm_o = reinterpret_cast<float*>(dsmem);                    // [4][8][128]
-  float* sm_m = sm_o + W * 8 * kDecodeD;                 // [4][8]
-  float* sm_l = sm_m + W * 8;                            // [4][8]
+  float* sm_o = reinterpret_cast<float*>(dsmem);  // [W][8][128]
+  float* sm_m = sm_o + W * 8 * kDecodeD;          // [W][8]
+  float* sm_l = sm_m + W * 8;                     // [W][8]
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     float2 v2 = make_float2(oacc[j][0], oacc[j][1]);
